@@ -26,19 +26,23 @@
 //                    into units of whole (u3,v3) iterations on a device queue,
 //                    storing each one's windows as an image;
 //   yz_first_kernel  persistent warps (28 per SM, 72 registers) drain the
-//                    queue with the first cut only: fit of the station-3 and
-//                    station-2 y hits, 2-sigma cut, scratch-entry scan; each
-//                    unit's survivors (about 6 %) go in order to a device pool;
-//                    with the combination scorer it walks only the listed
+//                    queue with the first cut (fit of the station-3 and
+//                    station-2 y hits, 2-sigma cut) and the prop-tube and
+//                    hodoscope gates; the survivors that pass, and those that
+//                    set station-3 signs for them, go in order to a device
+//                    pool; with the combination scorer it walks only the
 //                    kept (u3,v3) iterations;
-//   yz_second_kernel per unit, the survivors replayed in order with the sign
-//                    carry: left/right walk, prop and hodoscope gates, chi2
-//                    (28 warps per SM, 72 registers; a survivor's hits are
-//                    register offsets into the arena); a unit whose survivors
-//                    did not fit runs whole, first cut and survivors together
+//   yz_second_kernel per unit, those survivors replayed in order with the
+//                    sign carry: left/right walk and chi2 (28 warps per SM,
+//                    72 registers; a survivor's hits are register offsets
+//                    into the arena); a unit whose survivors did not fit runs
+//                    whole, first cut and survivors together
 //                    (yz_work_kernel's path, which also serves contexts
-//                    without a pool, such as the no-allocation entry);
-//   yz_apply_kernel  writes each heavy tracklet's best combination.
+//                    without a pool, such as the no-allocation entry); the
+//                    best combination of a tracklet of one unit is written
+//                    here;
+//   yz_apply_kernel  writes the best combination of tracklets of several
+//                    units.
 // Inside a range, lanes evaluate 32 combinations at a time in the reference
 // order; ballot/shuffle scans recover the sign state and the scratch entry.
 // A unit starts with the scratch entries left by everything before it, which
@@ -46,6 +50,8 @@
 // pass and each unit derive them without evaluating the earlier work.  The
 // best combination of a tracklet is the minimum of (chi2, combination index),
 // the reference's first-strictly-smaller rule.
+#include <type_traits>
+
 #include "window_pairs.cuh"
 
 namespace orgpu {
@@ -83,18 +89,18 @@ constexpr int YZ_MAXPAIR = 100;         // pairs per projection (the reference's
 #ifndef OR_YZ_POOL_PER_UNIT
 #define OR_YZ_POOL_PER_UNIT 48
 #endif
-// survivor entries in the pool (32 B each), per unit of queue capacity: a
+// survivor entries in the pool (16 B each), per unit of queue capacity: a
 // context sized for the 100,000-event uneven batch (4 Mi units) holds
-// 192 Mi, and that batch queues between 64 Mi and 128 Mi survivors; units
-// that do not fit run on the combined path
+// 192 Mi, several times what that batch passes on; units that do not fit run
+// on the combined path
 constexpr long long YZ_POOL_PER_UNIT = OR_YZ_POOL_PER_UNIT;
 #ifndef OR_YZ_IMG_PER_UNIT
-#define OR_YZ_IMG_PER_UNIT 36
+#define OR_YZ_IMG_PER_UNIT 80
 #endif
-// window images (16-byte words) per unit of queue capacity: 144 Mi words
-// (2.25 GiB) for 4 Mi units, and the 100,000-event uneven batch's queued
-// tracklets take 128 Mi words (1.9 GiB); tracklets whose image does not fit
-// are windowed again by each of their units
+// window images (16-byte words) per unit of queue capacity: 320 Mi words
+// (5 GiB) for 4 Mi units, and the 100,000-event uneven batch's queued
+// tracklets take 128 Mi words (1.9 GiB); the units of tracklets whose image
+// does not fit run on the combined path
 constexpr long long YZ_IMG_PER_UNIT = OR_YZ_IMG_PER_UNIT;
 constexpr int YZ_ARENA_HITS = OR_YZ_ARENA;      // windowed hits kept in shared memory per warp
 #ifndef OR_YZ_LIGHT
@@ -103,9 +109,10 @@ constexpr int YZ_ARENA_HITS = OR_YZ_ARENA;      // windowed hits kept in shared 
 constexpr long YZ_LIGHT = OR_YZ_LIGHT;         // combinations a planning warp evaluates itself per tracklet
 constexpr long YZ_CHUNK_INLINE = OR_YZ_LIGHT;  // ... and per planning unit
 #ifndef OR_YZ_PLAN_CHUNK
-#define OR_YZ_PLAN_CHUNK 8
+#define OR_YZ_PLAN_CHUNK 1
 #endif
 constexpr int YZ_PLAN_CHUNK = OR_YZ_PLAN_CHUNK;  // slots per planning unit
+constexpr int YZ_PLAN_CHUNK_SCORED = 8;          // ... with the combination scorer
 #ifndef OR_YZ_UNIT
 #define OR_YZ_UNIT 8192
 #endif
@@ -198,18 +205,19 @@ constexpr int YZ_CTR_FITTED = 16, YZ_CTR_HITSUM = 18, YZ_CTR_SURVIVORS = 20;
 
 struct YzScratch {
     const YzTab *tab;        // 2 x YZ_TAB_SETS entries: station-3 half 0 (D3p) then 1 (D3m)
+    unsigned *list;          // planning units with tracklets; nullptr: every unit is visited
     YzUnit *units;
     YzHeavy *heavy;
     YzBest *best;
     unsigned int *counters;  // [0] units reserved, [1] heavy reserved, [2] queue head, [3] survivor-kernel
-                             // head, [4..5] planning units, [8..9] pool entries, [10..11] image words,
+                             // head, [4..5] planning units taken, [6] planning units listed, [8..9] pool entries, [10..11] image words,
                              // [16..21] work counters
     YzHit *garena;           // per-warp overflow arenas
     struct PassEntryStore *qbuf;  // per-warp survivor queues (qcap entries each)
     int cap_units, cap_heavy, garena_warps, qcap;
     // split first-cut / survivor kernels: each unit's survivors in order in
     // pool[useg[u].x .. + useg[u].y); useg[u].x < 0: the unit runs combined
-    struct PassEntryStore *pool;
+    struct YzSurv *pool;
     int2 *useg;
     long long pool_cap;  // 0: no pool, the combined kernel runs
     // window images of the queued tracklets (YzImgHead, arena, pairs),
@@ -246,6 +254,20 @@ struct PassEntryStore {
     int stdet;
 };
 
+// A survivor as the first-cut kernel hands it to the survivor kernel:
+// combination index, first fit, and a code: bits 0-9 the arena offset of the
+// scratch entry past its hit count, bits 10-11 where that entry stands
+// (YZ_ENT_*), bits 12-13 the unit's starting entry (4..7) when it stands
+// there, bits 14-20 the plane set's table index, bit 31 whether the gates
+// passed (a survivor that fails them is only kept for the station-3 signs it
+// sets).
+struct __align__(16) YzSurv {
+    int c;
+    float y0, ty;
+    unsigned code;
+};
+constexpr unsigned YZ_ENT_HIT = 1u, YZ_ENT_UNIT = 2u;  // 0: no such entry
+
 struct YzEvent {
     HitPlane hc[8];
     HitPlane p1y1, p1y2, p2y1, p2y2;
@@ -253,29 +275,15 @@ struct YzEvent {
     short dl[8];
 };
 
-// the first cut's listed iterations at a time (yz_first_kept)
-constexpr int YZ_KEPT_BATCH = 32;
-// inner-pair records (yz_s2_record) the first cut keeps in shared memory
-constexpr int YZ_REC_SMEM = (8 * YZ_MAXWIN * 2 + 2 * YZ_MAXWIN) / 8;
-
 struct YzWarp {
-    union {
-        YzEvent ev;  // the event's plane views, the same for every lane
-        // first cut (the event's views are not read there): the scratch
-        // writes of the pruned iterations before each listed one
-        unsigned long long kgap[YZ_KEPT_BATCH];
-    };
+    YzEvent ev;  // the event's plane views, the same for every lane
     Stale st[4];  // scratch entries 4..7 as the next combination finds them, the same for every lane
     YzHit arena[YZ_ARENA_HITS];
     short2 pair[4][YZ_MAXPAIR];  // windowed indices (or -1) in sides 0, 1 of list q
-    union {
-        struct {
-            short widx[8][YZ_MAXWIN];  // plane hit index of each windowed hit
-            uint8_t wfl[2][YZ_MAXWIN];
-        } w;                           // while the windows are built
-        unsigned long long rec[YZ_REC_SMEM];  // first cut: the inner pairs' records
-    };
-    unsigned short kuv[YZ_KEPT_BATCH];  // first cut: the listed iterations, iu3 | iv3 << 8
+    struct {
+        short widx[8][YZ_MAXWIN];  // plane hit index of each windowed hit
+        uint8_t wfl[2][YZ_MAXWIN];
+    } w;                           // while the windows are built
     int np[4], nw[8], woff[8];
     float x0, tx, ex0, etx;
     int nhx;
@@ -906,17 +914,46 @@ struct Phase2Carry {
 // The full evaluation of n (<= 32) queued survivors Qc[0..n), in order: sign
 // state, left/right walk, prop and hodoscope gates, chi2, best key
 // (K:1613-1799).  Out of line: it runs once per 32 survivors, and inlined it
-// would sit in the middle of the first-cut loop's instructions.
+// would sit in the middle of the first-cut loop's instructions.  GATED: the
+// survivors come from the first-cut kernel (YzSurv), which has evaluated the
+// gates; `tab` is the station half's table, S.st the unit's starting entries.
+template <bool GATED>
 __device__ __noinline__ void yz_phase2(YzWarp &S, const YzEvent &E, const YzHit *base, int C2, const or_plane_t &P,
-                                       const PassEntryStore *Qc, int n, Phase2Carry &cs) {
+                                       const std::conditional_t<GATED, YzSurv, PassEntryStore> *Qc, int n,
+                                       const YzTab *__restrict__ tab, Phase2Carry &cs) {
     const int lane = lane_id();
     const float x0 = S.x0, tx = S.tx, ex0 = S.ex0, etx = S.etx;
     const int nhx = S.nhx;
-    if (lane == 0) S.nsurv += (unsigned long long)n;
+    if (!GATED && lane == 0) S.nsurv += (unsigned long long)n;
     // --- one chunk of survivors ------------------------------------------
     const bool valid = lane < n;
     PassEntry q;
-    if (valid) q = Qc[lane];
+    bool gated = false;
+    if constexpr (GATED) {
+        if (valid) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(Qc + lane);
+            q.c = (int)v.x;
+            q.y0 = __uint_as_float(v.y);
+            q.ty = __uint_as_float(v.z);
+            gated = (v.w >> 31) != 0u;
+            const float2 er = __ldg(reinterpret_cast<const float2 *>(&tab[(v.w >> 14) & 0x7Fu].ey0));
+            q.ey0 = er.x;
+            q.ety = er.y;
+            const unsigned src = (v.w >> 10) & 3u;
+            Stale e3{DET_SENTINEL, 0.f, 0.f};
+            if (src == YZ_ENT_HIT) {
+                const YzHit &r = base[v.w & 0x3FFu];
+                e3 = Stale{r.det, r.pos, r.drift};
+            } else if (src == YZ_ENT_UNIT) {
+                e3 = S.st[(v.w >> 12) & 3u];
+            }
+            q.stdet = e3.det;
+            q.stpos = e3.pos;
+            q.stdrift = e3.drift;
+        }
+    } else if (valid) {
+        q = Qc[lane];
+    }
     const int c = valid ? q.c : 0;
     const int g = valid ? c / C2 : -1 - lane;
     UvSet U{0ull, 0ull, 0u};
@@ -984,7 +1021,7 @@ __device__ __noinline__ void yz_phase2(YzWarp &S, const YzEvent &E, const YzHit 
         }
     }
     if (valid) {
-        pass = yz_gates(E, P, x0, y0, tx, ty, ex0, ey0, etx, ety);
+        pass = GATED ? gated : yz_gates(E, P, x0, y0, tx, ty, ex0, ey0, etx, ety);
         if (pass) chi2 = yz_chi2(S, U, base, nuv, nhx, P, x0, y0, tx, ty);
     }
     // carry of the sign state to the next survivor chunk
@@ -1449,72 +1486,6 @@ __device__ __forceinline__ int yz_scan_queue(const YzHit *base, Stale st[4], uns
     return qn;
 }
 
-// yz_scan_queue for the first-cut kernel, with the scratch state in a
-// register: field k (16 bits) of `stp` is the arena offset of the last write
-// of entry k before this chunk, 0xFFFF while entry k still holds st[k] (the
-// unit's starting state, which stays in shared memory unchanged).  Hits are
-// read only for the survivors' entries, and a chunk without survivors only
-// advances the state.
-__device__ __forceinline__ int yz_scan_queue_off(const YzHit *base, const Stale *st, unsigned long long &stp,
-                                                 unsigned long long own, unsigned wmask, int nuv, bool pass1, int c,
-                                                 float y0, float ty, float ey0, float ety, PassEntryStore *Q, int qn) {
-    const unsigned pm = __ballot_sync(0xffffffffu, pass1);
-    if (pm == 0u) {
-#pragma unroll 1
-        for (int k = 0; k < 4; ++k) {
-            const unsigned m = __ballot_sync(0xffffffffu, (wmask >> k) & 1u);
-            if (m) {
-                const int ok = (int)((own >> (16 * k)) & 0x3FFull);
-                const unsigned long long v = (unsigned)__shfl_sync(0xffffffffu, ok, last_lane(m));
-                stp = (stp & ~(0xFFFFull << (16 * k))) | (v << (16 * k));
-            }
-        }
-        return qn;
-    }
-    const unsigned lt = lanemask_lt();
-    int stj = -2;  // the entry past the hit count: -2 none, -1 st[kk], else an arena offset
-    int kk = 0;
-#pragma unroll 1
-    for (int k = 0; k < 4; ++k) {
-        const bool mine = (wmask >> k) & 1u;
-        const int ok = (int)((own >> (16 * k)) & 0x3FFull);
-        const unsigned m = __ballot_sync(0xffffffffu, mine);
-        const int src = last_lane(m & lt);
-        const int so = __shfl_sync(0xffffffffu, ok, src < 0 ? 0 : src);
-        if (nuv == k + 4) {
-            const int cur = (int)((stp >> (16 * k)) & 0xFFFFull);
-            stj = mine ? ok : (src >= 0 ? so : (cur == 0xFFFF ? -1 : cur));
-            kk = k;
-        }
-        if (m) {
-            const unsigned long long v = (unsigned)__shfl_sync(0xffffffffu, ok, last_lane(m));
-            stp = (stp & ~(0xFFFFull << (16 * k))) | (v << (16 * k));
-        }
-    }
-    if (pass1) {
-        Stale e3{DET_SENTINEL, 0.f, 0.f};
-        if (stj >= 0) {
-            const YzHit &r = base[stj];
-            e3 = Stale{r.det, r.pos, r.drift};
-        } else if (stj == -1) {
-            e3 = st[kk];
-        }
-        PassEntryStore e;
-        e.c = c;
-        e.y0 = y0;
-        e.ty = ty;
-        e.ey0 = ey0;
-        e.ety = ety;
-        e.stdet = e3.det;
-        e.stpos = e3.pos;
-        e.stdrift = e3.drift;
-        Q[qn + __popc(pm & lt)] = e;
-    }
-    qn += __popc(pm);
-    __syncwarp();
-    return qn;
-}
-
 template <bool PRUNE = false>
 __device__ unsigned long long yz_range_t(YzWarp &S, const YzEvent &E, const YzHit *base, long c0l, long c1l,
                                          Stale st[4], const or_plane_t &P, const YzTab *__restrict__ tab,
@@ -1654,7 +1625,7 @@ __device__ unsigned long long yz_range_t(YzWarp &S, const YzEvent &E, const YzHi
             // range: evaluate every waiting survivor, 32 at a time, in order
             while (qh < qn) {
                 const int n = min(qn - qh, 32);
-                yz_phase2(S, E, base, C2, P, Q + qh, n, cs);
+                yz_phase2<false>(S, E, base, C2, P, Q + qh, n, nullptr, cs);
                 qh += n;
                 __syncwarp();
             }
@@ -1665,192 +1636,478 @@ __device__ unsigned long long yz_range_t(YzWarp &S, const YzEvent &E, const YzHi
 }
 
 
-// The first cut of one unit over its live outer iterations, or with the
-// combination scorer (`osc`) over the kept ones only (first kernel).  The unit's live outer iterations
-// -- the scorer's rows [r0, r1) of its tracklet, in loop order -- are
-// classified 32 at a time; the kept ones go, 32 at a time, into a list in
-// the warp's shared memory, each with the scratch writes of
-// the pruned iterations right before it (its gap: for every entry 4..7 the
-// arena offset of the last pruned iteration's write there, from the load
-// pattern alone, as yz_skip_pruned finds it).  The list's combinations are
-// then walked densely, 32 a chunk, as yz_range_t walks a range; the first
-// combination of a kept iteration counts its gap's writes as its own, made
-// before its own loads, so every survivor reads the scratch entry of the
-// plain run.  A combination's station-2 part comes from the record of its
-// inner pair (R, yz_s2_record); its station-3 part is computed once per
-// listed iteration.  Survivors go to Q in order; *nsurv = their count, or -1
-// when the queue could overflow (the unit then runs on the combined path).
+// ---------------------------------------------------------------------------
+// First cut (split path)
+// ---------------------------------------------------------------------------
+//
+// A combination is an outer iteration (u3, v3) with an inner pair (u2, v2).
+// Everything the cut needs from either side is made once per unit:
+//   - per outer iteration, 32 listed at a time: the fit's right-hand side
+//     over its station-3 hits, its hit count and plane set, and the scratch
+//     entries 4..7 as the iteration finds them (a last-writer scan over the
+//     live iterations before it; which entries an iteration leaves depends
+//     on its hit count alone, the inner pairs being the same in every one);
+//   - per inner pair that reaches the fit, in order: the accepted hits, the
+//     plane set, and the scratch entry past the hit count where this pair or
+//     an earlier one of the same outer iteration has written it.
+// A combination then costs its additions, two dot products and two compares,
+// and its scratch entry is a lookup.  Combinations that pass wait in a ring
+// in shared memory; 32 at a time they go through the prop-tube and hodoscope
+// gates, all lanes in use.  Only those that pass reach the survivor kernel,
+// with the two kinds that set station-3 signs for them: the first survivor
+// of their outer iteration, and the survivors whose walk pairs the last
+// station-3 hit with the first station-2 hit (planes 19, 18).
+//
+// Bound: instruction issue.  Listing each inner pair's attempts per
+// combination, scanning the scratch entries over every chunk of 32 and
+// passing every survivor on took 22.9 ms of the 100,000-event uneven batch
+// with 19.5 ms in the survivor kernel; this takes 10.6 ms with 8.2 ms.
+constexpr int YZ_KEPT_BATCH = 32;     // outer iterations listed at a time
+constexpr int YZ_TT_SMEM = 256;       // hits whose fit terms are kept in shared memory
+constexpr int YZ_FIT_SMEM = 180;      // inner pairs' records kept in shared memory
+constexpr int YZ_PROP_SMEM = 40;      // hits per prop-tube y plane kept in shared memory
+// ... beyond them in the warp's overflow arena: the terms of every hit, then
+// the records, whose pair indices take the end of the warp's survivor queue
+constexpr int YZ_TT_ARENA_BYTES = YZ_GARENA_HITS * 8;
+constexpr int YZ_FIT_MAX = (int)(YZ_GARENA_HITS * sizeof(YzHit) - YZ_TT_ARENA_BYTES) / 8;
+constexpr int YZ_R2_ENTRIES = (YZ_FIT_MAX * 2 + (int)sizeof(YzSurv) - 1) / (int)sizeof(YzSurv);
 
-// inner-pair records (8 B) that fit the per-warp overflow arena, where the
-// first cut keeps them when the shared ones do not suffice
-constexpr int YZ_RECORDS_MAX = (int)(YZ_GARENA_HITS * sizeof(YzHit) / 8);
-static_assert(sizeof(YzEvent) >= sizeof(unsigned long long) * YZ_KEPT_BATCH, "the listed gaps fit the event's views");
+// hodoscope x planes of stations 2-4 and the prop-tube y planes
+struct YzGate {
+    float hz[6], ymin[6], ymax[6];
+    float pz[4];
+};
 
-__device__ void yz_first_kept(YzWarp &S, const YzHit *base, int r0, int r1, Stale st[4],
-                              const YzTab *__restrict__ tab, PassEntryStore *Q, int qcap, int *nsurv,
-                              const float *__restrict__ osc, float t_keep, const unsigned long long *R) {
+struct YzFirstWarp {
+    uint4 ring[64];  // survivors waiting for the gates: pair (g << 14 | r2), y0, ty, code
+    unsigned long long rec[YZ_FIT_SMEM];
+    unsigned long long kent[YZ_KEPT_BATCH];  // scratch entries 4..7, 16 bits each: arena offset, 0xFFFF = the unit's
+    float2 kb[YZ_KEPT_BATCH];
+    unsigned kt[YZ_KEPT_BATCH];  // g | table offset << 14 | n3 << 21 | only v3' << 24
+    float2 tt[YZ_TT_SMEM];       // (eY * Y, eY * Y * z) of each windowed hit
+    uint4 pend;                  // the current outer iteration's first survivor, not passed on yet
+    float prop[4][YZ_PROP_SMEM];
+    uchar2 pair[4][YZ_MAXPAIR];  // 255 = none
+    unsigned acc[(8 * YZ_MAXWIN + 31) / 32];
+    int np[4], woff[8];
+    HitPlane pp[4];
+    unsigned short r2[YZ_FIT_SMEM];
+};
+
+__device__ __forceinline__ bool yz_acc(const YzFirstWarp &S, int off) { return (S.acc[off >> 5] >> (off & 31)) & 1u; }
+// which of a pair's two hits are accepted (bit 0: the first plane's)
+__device__ __forceinline__ int yz_group(const YzFirstWarp &S, int q, uchar2 p) {
+    return (p.x != 255 && yz_acc(S, S.woff[2 * q] + p.x) ? 1 : 0) |
+           (p.y != 255 && yz_acc(S, S.woff[2 * q + 1] + p.y) ? 2 : 0);
+}
+
+// A tracklet's windows from its image, as the first cut needs them.
+__device__ __forceinline__ void yz_first_load(YzFirstWarp &S, const uint4 *__restrict__ img, float2 *tt, int total) {
+    const int lane = lane_id();
+    const YzImgHead &h = *reinterpret_cast<const YzImgHead *>(img);
+    if (lane < 4) S.np[lane] = h.np[lane];
+    if (lane < 8) S.woff[lane] = h.woff[lane];
+    const uint4 *ia = img + YZ_IMG_HEAD_WORDS;
+#pragma unroll 1
+    for (int b0 = 0; b0 < total; b0 += 32) {
+        const int i = b0 + lane;
+        bool a = false;
+        if (i < total) {
+            const float2 ye = *reinterpret_cast<const float2 *>(ia + 2 * i);
+            const uint4 v = ia[2 * i + 1];
+            const float t = ye.y * ye.x;
+            tt[i] = make_float2(t, t * __uint_as_float(v.y));
+            a = v.w != 0u;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, a);
+        if (lane == 0) S.acc[b0 >> 5] = m;
+    }
+    const short2 *ip = reinterpret_cast<const short2 *>(ia + 2 * total);
+    int off = 0;
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+        const int n = h.np[q];
+#pragma unroll 1
+        for (int i = lane; i < n; i += 32) {
+            const short2 p = ip[off + i];
+            S.pair[q][i] = make_uchar2((unsigned char)(p.x < 0 ? 255 : p.x), (unsigned char)(p.y < 0 ? 255 : p.y));
+        }
+        off += n;
+    }
+}
+
+// The event's prop-tube y planes and, for the tracklet's x fit, which of the
+// six hodoscope x planes (bit 2q + c) hold a hit in its x window: that part
+// of match_tracklet_to_hodo (H:1002-1087) does not depend on the y fit, and
+// its y window is the same for every hit of a plane.
+__device__ __forceinline__ unsigned yz_first_event(YzFirstWarp &S, const or_hits_view_t &hv, long e,
+                                                   const YzGate &G, const or_plane_t *__restrict__ P, float x0,
+                                                   float tx, float ex0, float etx) {
+    const int lane = lane_id();
+    bool has = false;
+    if (lane < 4) {
+        S.pp[lane] = hits_of(hv, e, lane == 0 ? DET_P1Y1 : lane == 1 ? DET_P1Y2 : lane == 2 ? DET_P2Y1 : DET_P2Y2);
+    } else if (lane < 10) {
+        const int i = lane - 4;
+        int stid = (i >> 1) + 1;
+        const int det = c_hodoplanesx[stid][i & 1];
+        const HitPlane h = hits_of(hv, e, det);
+        if (det > 40) stid = 3;
+        const float fudgefac = c_hodofudgefac[stid];
+        const float cellwidth = __ldg(&P->cellwidth[det]);
+        const float xhodo = G.hz[i] * tx + x0;
+        float err_x = 3.f * (fabsf(G.hz[i] * etx) + ex0);
+#pragma unroll 4
+        for (int k = 0; k < h.n; ++k) {
+            const float p = h.pos(k);
+            float xmin = p - cellwidth * 0.5f;
+            float xmax = p + cellwidth * 0.5f;
+            xmin -= (xmax - xmin) * fudgefac;
+            xmax += (xmax - xmin) * fudgefac;
+            err_x += (xmax - xmin) * 0.15f;
+            xmin -= err_x;
+            xmax += err_x;
+            has |= xmin <= xhodo && xhodo <= xmax;
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int n = min(S.pp[q].n, YZ_PROP_SMEM);
+#pragma unroll 1
+        for (int i = lane; i < n; i += 32) S.prop[q][i] = S.pp[q].pos(i);
+    }
+    return __ballot_sync(0xffffffffu, has) >> 4;
+}
+
+// a hit of prop-tube plane q within tol of e (prop_hits, K:1640-1701), for
+// the lanes with `want`
+__device__ __forceinline__ bool yz_prop_plane(const YzFirstWarp &S, int q, float e, float tol, bool want) {
+    const int n = S.pp[q].n;
+    bool ok = false;
+    const int m = min(n, YZ_PROP_SMEM);
+#pragma unroll 4
+    for (int i = 0; i < m; ++i) ok |= fabsf(S.prop[q][i] - e) < tol;
+#pragma unroll 1
+    for (int i = m; i < n && __any_sync(0xffffffffu, want && !ok); ++i) ok |= fabsf(S.pp[q].pos(i) - e) < tol;
+    return ok && want;
+}
+
+// the gates of a survivor (yz_gates), every lane of the warp
+__device__ __forceinline__ bool yz_first_gates(const YzFirstWarp &S, const YzGate &G, unsigned hasx, bool valid, float y0,
+                                               float ty, float ey0, float ety) {
+    bool ok = valid && !(fabsf(y0) > Y0_MAX || fabsf(ty) > TY_MAX);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        bool m = false;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int i = 2 * q + c;
+            const float yhodo = G.hz[i] * ty + y0;
+            const float err_y = 3.f * (fabsf(G.hz[i] * ety) + ey0);
+            m |= ((hasx >> i) & 1u) && G.ymin[i] - err_y <= yhodo && yhodo <= G.ymax[i] + err_y;
+        }
+        ok = ok && m;
+    }
+#pragma unroll 1
+    for (int s = 0; s < 2; ++s) {
+        if (!__any_sync(0xffffffffu, ok)) return false;
+        const float tol = s ? 10.16f : 5.08f;
+        const bool a = yz_prop_plane(S, 2 * s, ty * G.pz[2 * s] + y0, tol, ok);
+        bool b = false;
+        if (__any_sync(0xffffffffu, ok && !a)) b = yz_prop_plane(S, 2 * s + 1, ty * G.pz[2 * s + 1] + y0, tol, ok && !a);
+        ok = a || b;
+    }
+    return ok;
+}
+
+// State of the survivors' order from one ring chunk to the next.
+struct YzOrder {
+    int g = -1;         // outer iteration of the last survivor
+    bool pend = false;  // its first survivor waits in S.pend
+};
+
+// Up to 32 survivors from the ring, in order: the gates, then those the
+// survivor kernel needs go to Q; returns the new queue length.
+__device__ __forceinline__ int yz_first_pass(YzFirstWarp &S, const YzGate &G, unsigned hasx, int head, int n, int C2,
+                                             const YzTab *__restrict__ tab, YzOrder &od, YzSurv *Q, int qn) {
     const int lane = lane_id();
     const unsigned lt = lanemask_lt();
-    const int nu2 = S.np[0], nv2 = S.np[1], nu3 = S.np[2];
-    const int C2 = nu2 * nv2;
-    const YzAlive alive = yz_alive(S, base);
-    const int Au = bits128(alive.u);
-    const unsigned long long lasto = osc ? yz_last_writes(S, base) : ~0ull;
-    const int sg = 32 / C2, sr = 32 - sg * C2;
-    const int s0 = sr % nu2, s1 = sr / nu2;  // a chunk's step in the inner digits ...
-    int qn = 0;
-    unsigned long long stp = ~0ull;  // scratch entries' last writes (yz_scan_queue_off)
-    unsigned long long gapc = ~0ull;  // writes of the pruned iterations since the last kept one
-    int r = r0;
-    while (r < r1) {
-        // --- the next kept iterations and their gaps ---------------------
-        int nk = 0;
-        __syncwarp();  // every lane is done with the previous list
-        while (r < r1 && nk <= YZ_KEPT_BATCH - 32) {
-            const int j = r + lane;
-            const bool in = j < r1;
-            bool kept = false;
-            int iu = 0, iv = 0;
-            unsigned long long w = ~0ull;  // this pruned iteration's writes
-            if (in) {
-                kept = !osc || osc[j] >= t_keep;
-                iu = nth_bit128(alive.u, j % Au);
-                iv = nth_bit128(alive.v, j / Au);
-                if (!kept) {
-                    bool v;
-                    const int n3 = s3_count(S, base, iu, iv, v);
+    const bool valid = lane < n;
+    const uint4 v = S.ring[(head + lane) & 63];
+    const float y0 = __uint_as_float(v.y), ty = __uint_as_float(v.z);
+    float2 er = make_float2(0.f, 0.f);
+    if (valid) er = __ldg(reinterpret_cast<const float2 *>(&tab[(v.w >> 14) & 0x7Fu].ey0));
+    const bool pass = yz_first_gates(S, G, hasx, valid, y0, ty, er.x, er.y);
+    const int g = valid ? (int)(v.x >> 14) : -2 - lane;
+    const int gp = __shfl_up_sync(0xffffffffu, g, 1);
+    const bool first = valid && g != (lane == 0 ? od.g : gp);
+    const bool keep = valid && (pass || ((v.w >> 21) & 1u));  // bit 21: may pair planes 19 and 18
+    const unsigned seg = __match_any_sync(0xffffffffu, g);
+    const unsigned km = __ballot_sync(0xffffffffu, keep);
+    const bool emit = keep || (first && (km & seg) != 0u);
+    const unsigned em = __ballot_sync(0xffffffffu, emit);
+    auto put = [&](int at, uint4 w, bool gate) {
+        const int gg = (int)(w.x >> 14), rr = (int)(w.x & 0x3FFFu);
+        const uint4 o = make_uint4((unsigned)(gg * C2 + rr), w.y, w.z, (w.w & 0x1FFFFFu) | (gate ? 0x80000000u : 0u));
+        *reinterpret_cast<uint4 *>(Q + at) = o;
+    };
+    // the iteration carried from the last chunk: its first survivor goes
+    // before the first one kept here
+    const unsigned cont = __ballot_sync(0xffffffffu, valid && g == od.g);
+    if (od.pend && (km & cont)) {
+        if (lane == 0) put(qn, S.pend, false);
+        ++qn;
+        od.pend = false;
+    }
+    if (emit) put(qn + __popc(em & lt), v, pass);
+    qn += __popc(em);
+    // the chunk's last iteration may go on
+    const int last = n - 1;
+    const int gl = __shfl_sync(0xffffffffu, g, last);
+    if (gl != od.g) {
+        const unsigned segl = __shfl_sync(0xffffffffu, seg, last);
+        od.pend = (km & segl) == 0u;
+        od.g = gl;
+        __syncwarp();
+        if (od.pend && lane == __ffs(segl) - 1) S.pend = v;
+    }
+    __syncwarp();
+    return qn;
+}
+
+// The first cut of one unit.  `tt` and `R` / `R2` (nf records) are in shared
+// memory or in the warp's overflow arena.  Returns the survivors passed on in
+// Q, or -1 when the queue could overflow (the unit then runs on the combined
+// path); *count = the combinations that passed the cut.
+template <bool PRUNE>
+__device__ __forceinline__ int yz_first_walk(YzFirstWarp &S, const YzGate &G, unsigned hasx, const float2 *tt,
+                                             unsigned long long *R, unsigned short *R2, int nf, int r0, int r1,
+                                             bool half_p, const YzTab *__restrict__ tab, YzSurv *Q, int qcap,
+                                             const float *__restrict__ osc, float t_keep, int *count) {
+    const int lane = lane_id();
+    const unsigned lt = lanemask_lt();
+    const int nu2 = S.np[0], nu3 = S.np[2];
+    const int C2 = nu2 * S.np[1];
+    // --- the inner pairs' records ------------------------------------------
+    // the last write of offset m past the station-3 hits over the pairs so
+    // far, 16 bits each (yz_last_writes)
+    unsigned long long lasto = ~0ull;
+    {
+        int at = 0;
+#pragma unroll 1
+        for (int b0 = 0; b0 < C2; b0 += 32) {
+            const int r = b0 + lane;
+            unsigned long long off = 0ull;  // hit e of the pair's accepted ones, or the failed attempt after them
+            unsigned pm = 0u;
+            int nacc = 0, gu = 0, gv = 0;
+            if (r < C2) {
+                const uchar2 pu = S.pair[0][r % nu2], pv = S.pair[1][r / nu2];
+                const int o[4] = {pu.x != 255 ? S.woff[0] + pu.x : -1, pu.y != 255 ? S.woff[1] + pu.y : -1,
+                                  pv.x != 255 ? S.woff[2] + pv.x : -1, pv.y != 255 ? S.woff[3] + pv.y : -1};
+                int g = 0;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const int mm = k + 4 - n3;
-                        if (mm >= 0 && mm < 4)
-                            w = (w & ~(0xFFFFull << (16 * k))) | (((lasto >> (16 * mm)) & 0xFFFFull) << (16 * k));
+                for (int a = 0; a < 4; ++a) {
+                    if (a == 2 && nacc == 0) break;  // no u2 hit: v2 is not loaded
+                    if (o[a] < 0) continue;
+                    const int sh = 16 * nacc;
+                    off = (off & ~(0xFFFFull << sh)) | ((unsigned long long)o[a] << sh);
+                    pm |= 1u << nacc;
+                    if (yz_acc(S, o[a])) {
+                        g |= 1 << a;
+                        ++nacc;
                     }
                 }
+                gu = g & 3;
+                gv = g >> 2;
             }
-            const unsigned km = __ballot_sync(0xffffffffu, kept);
-            const int lk = last_lane(km & lt);  // the last kept lane before this one
-            const unsigned after = lk >= 0 ? ~((2u << lk) - 1u) : 0xffffffffu;
-            const int lka = last_lane(km);  // ... and of the chunk
-            const unsigned aftera = lka >= 0 ? ~((2u << lka) - 1u) : 0xffffffffu;
-            unsigned long long gap = 0ull, carry = 0ull;
+            const bool fit = gu != 0 && gv != 0;
+            // the entry past the hit count as this pair leaves it or finds it
+            unsigned stale = 0xFFFFu;
+            unsigned long long nl = lasto;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                const unsigned mine = (unsigned)(off >> (16 * m)) & 0xFFFFu;
+                const unsigned wm = __ballot_sync(0xffffffffu, (pm >> m) & 1u);
+                if (m >= 2) {
+                    const int src = last_lane(wm & lt);
+                    const unsigned before = __shfl_sync(0xffffffffu, mine, src < 0 ? 0 : src);
+                    if (nacc == m) {
+                        if ((pm >> m) & 1u) stale = mine;
+                        else stale = src >= 0 ? before : (unsigned)((lasto >> (16 * m)) & 0xFFFFull);
+                    }
+                }
+                if (wm) {
+                    const unsigned long long w = __shfl_sync(0xffffffffu, mine, last_lane(wm));
+                    nl = (nl & ~(0xFFFFull << (16 * m))) | (w << (16 * m));
+                }
+            }
+            lasto = nl;
+            const unsigned fm = __ballot_sync(0xffffffffu, fit);
+            if (fit) {
+                const int k = at + __popc(fm & lt);
+                unsigned long long rec = 0ull;
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (e < nacc) rec |= ((off >> (16 * e)) & 0x3FFull) << (10 * e);
+                rec |= (unsigned long long)nacc << 40;
+                rec |= (unsigned long long)(gu * 3 - 4 + gv) << 43;
+                if (stale != 0xFFFFu) rec |= ((unsigned long long)stale << 47) | (1ull << 57);
+                if (gu & 1) rec |= 1ull << 58;  // starts with a hit of plane 18
+                R[k] = rec;
+                R2[k] = (unsigned short)r;
+            }
+            at += __popc(fm);
+        }
+    }
+    // --- pairs with an accepted hit ------------------------------------------
+    YzAlive alive;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        const int i = w * 32 + lane;
+        alive.u[w] = __ballot_sync(0xffffffffu, i < S.np[2] && yz_group(S, 2, S.pair[2][i < S.np[2] ? i : 0]) != 0);
+        alive.v[w] = __ballot_sync(0xffffffffu, i < S.np[3] && yz_group(S, 3, S.pair[3][i < S.np[3] ? i : 0]) != 0);
+    }
+    const int Au = bits128(alive.u);
+    const int sg = 32 / nf, sr = 32 - sg * nf;
+    int qn = 0, nsurv = 0;
+    int head = 0, waiting = 0;
+    YzOrder od;
+    unsigned long long carry = ~0ull;  // scratch entries as the next iteration finds them
+#pragma unroll 1
+    for (int b = r0; b < r1; b += 32) {
+        // --- list the outer iterations of ranks b .. b+31 ------------------
+        const int j = b + lane;
+        const bool in = j < r1;
+        bool kept = false;
+        unsigned long long w = ~0ull;  // the entries this iteration writes
+        float b0 = 0.f, b1 = 0.f;
+        unsigned kt = 0u;
+        if (in) {
+            kept = !(PRUNE && osc) || osc[j] >= t_keep;
+            const int iu = nth_bit128(alive.u, j % Au), iv = nth_bit128(alive.v, j / Au);
+            const uchar2 pu = S.pair[2][iu], pv = S.pair[3][iv];
+            const int gu = yz_group(S, 2, pu), gv = yz_group(S, 3, pv);
+            const int n3 = __popc(gu) + __popc(gv);
+            auto term = [&](int off) {
+                const float2 t = tt[off];
+                b0 += t.x;
+                b1 += t.y;
+            };
+            if (gu & 1) term(S.woff[4] + pu.x);
+            if (gu & 2) term(S.woff[5] + pu.y);
+            if (gv & 1) term(S.woff[6] + pv.x);
+            if (gv & 2) term(S.woff[7] + pv.y);
+            kt = (unsigned)(iu + iv * nu3) | ((unsigned)yz_tab_index(gu, gv, 1, 1) << 14) | ((unsigned)n3 << 21) |
+                 ((half_p && gv == 2) ? 1u << 24 : 0u);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const unsigned wk = (unsigned)((w >> (16 * k)) & 0xFFFFull);
-                const unsigned ck = (unsigned)((gapc >> (16 * k)) & 0xFFFFull);
-                const unsigned pm = __ballot_sync(0xffffffffu, wk != 0xFFFFu);
-                const int src = last_lane(pm & lt & after);
-                const unsigned v = __shfl_sync(0xffffffffu, wk, src < 0 ? 0 : src);
-                const unsigned g = src >= 0 ? v : (lk >= 0 ? 0xFFFFu : ck);
-                gap |= (unsigned long long)g << (16 * k);
-                const int srca = last_lane(pm & aftera);
-                const unsigned va = __shfl_sync(0xffffffffu, wk, srca < 0 ? 0 : srca);
-                const unsigned ga = srca >= 0 ? va : (lka >= 0 ? 0xFFFFu : ck);
-                carry |= (unsigned long long)ga << (16 * k);
+                const int mm = k + 4 - n3;
+                if (mm < 4) w = (w & ~(0xFFFFull << (16 * k))) | (((lasto >> (16 * mm)) & 0xFFFFull) << (16 * k));
             }
-            gapc = carry;
-            if (kept) {
-                const int pos = nk + __popc(km & lt);
-                S.kuv[pos] = (unsigned short)(iu | (iv << 8));
-                S.kgap[pos] = gap;
+        }
+        unsigned long long ent = 0ull;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const unsigned wk = (unsigned)(w >> (16 * k)) & 0xFFFFu;
+            const unsigned wm = __ballot_sync(0xffffffffu, wk != 0xFFFFu);
+            const int src = last_lane(wm & lt);
+            const unsigned v = __shfl_sync(0xffffffffu, wk, src < 0 ? 0 : src);
+            const unsigned c = (unsigned)(carry >> (16 * k)) & 0xFFFFu;
+            ent |= (unsigned long long)(src >= 0 ? v : c) << (16 * k);
+            if (wm) {
+                const unsigned long long l = __shfl_sync(0xffffffffu, wk, last_lane(wm));
+                carry = (carry & ~(0xFFFFull << (16 * k))) | (l << (16 * k));
             }
-            nk += __popc(km);
-            r += 32;
         }
-        __syncwarp();  // the list is written
-        // --- their combinations, 32 a chunk ------------------------------
-        const int ctot = nk * C2;
-        int k = lane / C2, d0, d1;
-        {
-            const int rr = lane - k * C2;
-            d0 = rr % nu2;
-            d1 = rr / nu2;
+        const unsigned km = __ballot_sync(0xffffffffu, kept);
+        __syncwarp();  // every lane is done with the previous list; the records are written
+        if (kept) {
+            const int pos = __popc(km & lt);
+            S.kb[pos] = make_float2(b0, b1);
+            S.kt[pos] = kt;
+            S.kent[pos] = ent;
         }
-        int kl = -1;  // list index whose station-3 part the lane holds
-        Yz3 t3{0.f, 0.f, 0, 0};
-        bool alive3 = false;
+        __syncwarp();
+        // --- their combinations, 32 a chunk ----------------------------------
+        const int ctot = __popc(km) * nf;
+        int k = lane / nf, r = lane - k * nf;
 #pragma unroll 1
         for (int cb = 0; cb < ctot; cb += 32) {
-            const bool valid = cb + lane < ctot;
-            int nuv = 0, c = 0;
-            unsigned long long own = 0ull;
-            unsigned wmask = 0u;
-            float y0 = 0.f, ty = 0.f, ey0 = 0.f, ety = 0.f;
-            bool pass1 = false;
-            if (valid) {
-                const unsigned uv = S.kuv[k];
-                const int iu3 = (int)(uv & 0xFFu), iv3 = (int)(uv >> 8);
-                if (k != kl) {
-                    alive3 = yz_station3(S, base, iu3, iv3, t3);
-                    kl = k;
+            bool pass = false;
+            float y0 = 0.f, ty = 0.f;
+            unsigned t3 = 0u;
+            unsigned long long rec = 0ull;
+            if (cb + lane < ctot) {
+                t3 = S.kt[k];
+                const float2 s = S.kb[k];
+                rec = R[r];
+                const int nacc = (int)(rec >> 40) & 7;
+                float2 t = tt[(int)rec & 0x3FF];
+                float f0 = s.x + t.x, f1 = s.y + t.y;
+                t = tt[(int)(rec >> 10) & 0x3FF];
+                f0 += t.x;
+                f1 += t.y;
+                if (nacc > 2) {
+                    t = tt[(int)(rec >> 20) & 0x3FF];
+                    f0 += t.x;
+                    f1 += t.y;
                 }
-                const int r2 = d1 * nu2 + d0;
-                c = (iu3 + iv3 * nu3) * C2 + r2;
-                if (r2 == 0) {
-                    // the gap's writes come before the iteration's own
-                    own = S.kgap[k];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (((own >> (16 * e)) & 0xFFFFull) != 0xFFFFull) wmask |= 1u << e;
+                if (nacc > 3) {
+                    t = tt[(int)(rec >> 30) & 0x3FF];
+                    f0 += t.x;
+                    f1 += t.y;
                 }
-                if (alive3) {
-                    // the inner pair's attempts: scratch writes shifted by the
-                    // station-3 count (n3 = 2..4), accepted hits in order
-                    const unsigned long long rec = R[r2];
-                    const int sh = 4 - t3.n3;
-                    const int nacc = (int)((rec >> 26) & 7u);
-                    const unsigned wr = ((unsigned)(rec >> 10) & 0xFu) >> sh;
-                    const unsigned long long mine = rec >> (16 * sh);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if ((wr >> e) & 1u) own = (own & ~(0xFFFFull << (16 * e))) | (mine & (0xFFFFull << (16 * e)));
-                    wmask |= wr;
-                    nuv = t3.n3 + nacc;
-                    if ((rec >> 58) & 1u) {
-                        // Fit2::solve with the plane set's tabulated inverse
-                        float b0 = t3.b0, b1 = t3.b1;
-#pragma unroll 1
-                        for (int e = 0; e < nacc; ++e) {
-                            const YzHit &h = base[(int)((rec >> (16 * e)) & 0x3FFull)];
-                            const float t = h.eY * h.Y;
-                            b0 += t;
-                            b1 += t * h.z;
-                        }
-                        const unsigned g2 = (unsigned)(rec >> 42) & 0xFu;
-                        const YzTab *te = tab + t3.tab3 + (g2 & 3u) * 3 - 4 + (g2 >> 2);
-                        const float4 ai = __ldg(reinterpret_cast<const float4 *>(te));
-                        const float2 thr = __ldg(reinterpret_cast<const float2 *>(&te->thr_y0));
-                        y0 = 0.0f;
-                        y0 += ai.x * b0;
-                        y0 += ai.y * b1;
-                        ty = 0.0f;
-                        ty += ai.z * b0;
-                        ty += ai.w * b1;
-                        pass1 = !(fabsf(y0) > thr.x || fabsf(ty) > thr.y);
-                        if (pass1) {
-                            const float2 er = __ldg(reinterpret_cast<const float2 *>(&te->ey0));
-                            ey0 = er.x;
-                            ety = er.y;
-                        }
+                // Fit2::solve with the plane set's tabulated inverse
+                const YzTab *te = tab + ((t3 >> 14) & 0x7Fu) + ((unsigned)(rec >> 43) & 0xFu);
+                const float4 ai = __ldg(reinterpret_cast<const float4 *>(te));
+                const float2 thr = __ldg(reinterpret_cast<const float2 *>(&te->thr_y0));
+                y0 = 0.0f;
+                y0 += ai.x * f0;
+                y0 += ai.y * f1;
+                ty = 0.0f;
+                ty += ai.z * f0;
+                ty += ai.w * f1;
+                pass = !(fabsf(y0) > thr.x || fabsf(ty) > thr.y);
+            }
+            const unsigned pm = __ballot_sync(0xffffffffu, pass);
+            if (pm) {
+                if (pass) {
+                    const int n3 = (int)(t3 >> 21) & 7, nacc = (int)(rec >> 40) & 7;
+                    // the scratch entry past the hit count
+                    unsigned code = ((t3 >> 14) & 0x7Fu) + ((unsigned)(rec >> 43) & 0xFu);
+                    code <<= 14;
+                    const int e = n3 + nacc - 4;  // entry 4 + e
+                    if ((rec >> 57) & 1u) {
+                        code |= ((unsigned)(rec >> 47) & 0x3FFu) | (YZ_ENT_HIT << 10);
+                    } else if (e < 4) {
+                        const unsigned o = (unsigned)(S.kent[k] >> (16 * e)) & 0xFFFFu;
+                        code |= o == 0xFFFFu ? (YZ_ENT_UNIT << 10) | ((unsigned)e << 12) : o | (YZ_ENT_HIT << 10);
                     }
+                    if (((t3 >> 24) & 1u) && ((rec >> 58) & 1u)) code |= 1u << 21;
+                    S.ring[(head + waiting + __popc(pm & lt)) & 63] =
+                        make_uint4(((t3 & 0x3FFFu) << 14) | R2[r], __float_as_uint(y0), __float_as_uint(ty), code);
+                }
+                waiting += __popc(pm);
+                nsurv += __popc(pm);
+                __syncwarp();
+                if (waiting >= 32) {
+                    qn = yz_first_pass(S, G, hasx, head, 32, C2, tab, od, Q, qn);
+                    head = (head + 32) & 63;
+                    waiting -= 32;
+                    if (qn > qcap - 34) return -1;
                 }
             }
-            qn = yz_scan_queue_off(base, st, stp, own, wmask, nuv, pass1, c, y0, ty, ey0, ety, Q, qn);
-            if (qn > qcap - 32) {
-                *nsurv = -1;
-                return;
-            }
-            d0 += s0;
-            int cy = d0 >= nu2;
-            d0 -= cy ? nu2 : 0;
-            d1 += s1 + cy;
-            cy = d1 >= nv2;
-            d1 -= cy ? nv2 : 0;
+            r += sr;
+            const int cy = r >= nf;
+            r -= cy ? nf : 0;
             k += sg + cy;
         }
     }
-    *nsurv = qn;
+    if (waiting) qn = yz_first_pass(S, G, hasx, head, waiting, C2, tab, od, Q, qn);
+    *count = nsurv;
+    return qn;
 }
-
 
 // The combined evaluation of a range, out of line: the survivor kernel runs
 // it only for units whose survivors did not fit the pool, the planning
@@ -1887,6 +2144,15 @@ __device__ __forceinline__ void yz_store(float *T, const YzBest &b, int nhx) {
         if (n < nhx) T[OR_TRK_HIT_RESID + n] = b.res[n];
         T[OR_TRK_HIT_RESID + nhx + n] = b.res[nhx + n];
     }
+}
+
+// the result of a heavy tracklet: its best combination (K:1804-1825) and,
+// for the scorer's labels, that combination's outer index
+__device__ __forceinline__ void yz_finish(const YzScratch &sc, int heavy, int c2, float *T, unsigned long long key,
+                                          const YzBest &b, int nhx) {
+    if (key == ~0ull) return;  // best_g stays -1
+    if (lane_id() == 0) sc.heavy[heavy].best_g = (int)((unsigned)key / (unsigned)max(c2, 1));
+    yz_store(T, b, nhx);
 }
 
 __device__ __forceinline__ YzHit *yz_garena(const YzScratch &sc, int gwarp) {
@@ -1932,8 +2198,8 @@ __device__ __forceinline__ void yz_flush_counts(const YzScratch &sc, unsigned lo
 template <int W>
 __global__ void __launch_bounds__(W * 32, (OR_YZ_PLAN_WARPS_SM / W > 0 ? OR_YZ_PLAN_WARPS_SM / W : 1))
     yz_plan_kernel(const or_plane_t *__restrict__ gplane, or_hits_view_t hv, or_tracks_view_t tv,
-                   const uint8_t *__restrict__ toomany, int n_events, YzScratch sc, uint32_t *__restrict__ errw,
-                   YzPrune prune) {
+                   const uint8_t *__restrict__ toomany, int n_events, int chunk, YzScratch sc,
+                   uint32_t *__restrict__ errw, YzPrune prune) {
     extern __shared__ __align__(16) unsigned char yz_smem[];
     or_plane_t &P = *reinterpret_cast<or_plane_t *>(yz_smem);
     YzWarp *warps = reinterpret_cast<YzWarp *>(yz_smem + ((sizeof(or_plane_t) + 15) & ~size_t(15)));
@@ -1947,17 +2213,20 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_PLAN_WARPS_SM / W > 0 ? OR_YZ_P
     if (lane == 0) S.nsurv = 0ull;
     unsigned long long n_fitted = 0ull, n_hitsum = 0ull;  // lane 0's work counters
 
-    // planning units (event, YZ_PLAN_CHUNK slots) from a device counter: slots
-    // are independent (one reference thread each), events very uneven
-    const unsigned long long nplan = (unsigned long long)n_events * (OR_NSLOTS / YZ_PLAN_CHUNK);
+    // planning units (event, `chunk` slots) from a device counter: slots are
+    // independent (one reference thread each), events very uneven
+    const int per_event = OR_NSLOTS / chunk;
+    const unsigned long long nplan =
+        sc.list ? (unsigned long long)sc.counters[6] : (unsigned long long)n_events * per_event;
     unsigned long long *plan_ctr = reinterpret_cast<unsigned long long *>(sc.counters + 4);
     for (;;) {
         unsigned long long pu = 0;
         if (lane == 0) pu = atomicAdd(plan_ctr, 1ull);
         pu = __shfl_sync(0xffffffffu, pu, 0);
         if (pu >= nplan) break;
-        const long e = (long)(pu / (OR_NSLOTS / YZ_PLAN_CHUNK));
-        const int slot0 = (int)(pu % (OR_NSLOTS / YZ_PLAN_CHUNK)) * YZ_PLAN_CHUNK;
+        if (sc.list) pu = sc.list[pu];
+        const long e = (long)(pu / per_event);
+        const int slot0 = (int)(pu % per_event) * chunk;
         if (toomany[e]) continue;  // K:873-878
         long budget = YZ_CHUNK_INLINE;
         long row = 0;  // scorer row of the next tracklet (slots in order, tracklets in slot order)
@@ -1967,7 +2236,7 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_PLAN_WARPS_SM / W > 0 ? OR_YZ_P
             for (int s = 0; s < slot0; ++s) row += min((int)tv.ntracks[e * OR_NSLOTS + s], OR_SLOTCAP);
         }
 #pragma unroll 1
-        for (int slot = slot0; slot < slot0 + YZ_PLAN_CHUNK; ++slot) {
+        for (int slot = slot0; slot < slot0 + chunk; ++slot) {
             const int ntr = min((int)tv.ntracks[e * OR_NSLOTS + slot], OR_SLOTCAP);
             const long slot_row = row;
             row += ntr;
@@ -2129,7 +2398,7 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_WARPS_SM / W > 0 ? OR_YZ_WARPS_
         const YzUnit un = sc.units[u];
         if (un.heavy < 0) continue;
         const YzHeavy hv2 = sc.heavy[un.heavy];
-        const float *T = trk_rec(tv, hv2.e, hv2.slot, hv2.k);
+        float *T = trk_rec(tv, hv2.e, hv2.slot, hv2.k);
         const int st3 = 3 + (hv2.slot & 1);
         YzEvent &E = S.ev;
         __syncwarp();  // every lane is done with the previous unit's views
@@ -2151,7 +2420,9 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_WARPS_SM / W > 0 ? OR_YZ_WARPS_
                               sc.tab + YZ_TAB_SETS * (st3 - 3), Q, sc.qcap, osc, prune.t_keep);
         __syncwarp();
         YzBest *dst = sc.best + u;
-        if (bk == ~0ull) {
+        if (hv2.nunits == 1) {  // the tracklet's only unit
+            yz_finish(sc, un.heavy, hv2.c2, T, bk, S.b, S.nhx);
+        } else if (bk == ~0ull) {
             if (lane == 0) dst->key = ~0ull;
         } else {
             const unsigned *src = reinterpret_cast<const unsigned *>(&S.b);
@@ -2165,84 +2436,105 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_WARPS_SM / W > 0 ? OR_YZ_WARPS_
 }
 
 
-// Split path, first kernel: the first cut of every queued unit (no survivor
-// evaluation, so it needs far fewer registers and no per-lane hit arrays);
-// a unit's survivors go, in order, to one contiguous piece of the pool.
-
+// Split path, first kernel: the first cut and the gates of every queued unit
+// (no left/right walk, so it needs far fewer registers); what the survivor
+// kernel needs of a unit goes, in order, to one contiguous piece of the pool.
 template <int W, bool PRUNE>
 __global__ void __launch_bounds__(W * 32, (OR_YZ_FIRST_WARPS_SM / W > 0 ? OR_YZ_FIRST_WARPS_SM / W : 1))
     yz_first_kernel(const or_plane_t *__restrict__ gplane, or_hits_view_t hv, or_tracks_view_t tv, YzScratch sc,
                     YzPrune prune) {
     extern __shared__ __align__(16) unsigned char yz_smem[];
-    or_plane_t &P = *reinterpret_cast<or_plane_t *>(yz_smem);
-    YzWarp *warps = reinterpret_cast<YzWarp *>(yz_smem + ((sizeof(or_plane_t) + 15) & ~size_t(15)));
-    load_plane_smem(&P, gplane);
-    __syncthreads();
+    YzGate &G = *reinterpret_cast<YzGate *>(yz_smem);
+    YzFirstWarp *warps = reinterpret_cast<YzFirstWarp *>(yz_smem + ((sizeof(YzGate) + 15) & ~size_t(15)));
     const int w = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    YzWarp &S = warps[w];
+    if (threadIdx.x < 6) {
+        const int i = threadIdx.x;
+        int stid = (i >> 1) + 1;
+        const int det = c_hodoplanesx[stid][i & 1];
+        if (det > 40) stid = 3;
+        const float fudgefac = c_hodofudgefac[stid];
+        float ymin = gplane->y1[det], ymax = gplane->y2[det];
+        ymin -= (ymax - ymin) * fudgefac;
+        ymax += (ymax - ymin) * fudgefac;
+        G.hz[i] = gplane->z[det];
+        G.ymin[i] = ymin;
+        G.ymax[i] = ymax;
+    } else if (threadIdx.x < 10) {
+        const int q = threadIdx.x - 6;
+        G.pz[q] = gplane->z[q == 0 ? DET_P1Y1 : q == 1 ? DET_P1Y2 : q == 2 ? DET_P2Y1 : DET_P2Y2];
+    }
+    __syncthreads();
+    YzFirstWarp &S = warps[w];
     const int gw = blockIdx.x * W + w;
     if (gw >= sc.garena_warps) return;  // queues and arenas exist for garena_warps warps
-    YzHit *garena = yz_garena(sc, gw);
-    PassEntryStore *Q = sc.qbuf + (long)gw * sc.qcap;
+    unsigned char *garena = reinterpret_cast<unsigned char *>(yz_garena(sc, gw));
+    YzSurv *Q = reinterpret_cast<YzSurv *>(sc.qbuf + (long)gw * sc.qcap);
+    const int qcap = sc.qcap * (int)(sizeof(PassEntryStore) / sizeof(YzSurv));
     unsigned long long *pool_ctr = reinterpret_cast<unsigned long long *>(sc.counters + 8);
     const int nunits = min((int)sc.counters[0], sc.cap_units);
+    unsigned long long n_surv = 0ull;
     for (;;) {
         int u = 0;
         if (lane == 0) u = (int)atomicAdd(&sc.counters[2], 1u);
         u = __shfl_sync(0xffffffffu, u, 0);
         if (u >= nunits) break;
-        const YzUnit un = sc.units[u];
-        if (un.heavy < 0) continue;
-        const YzHeavy hv2 = sc.heavy[un.heavy];
-        const float *T = trk_rec(tv, hv2.e, hv2.slot, hv2.k);
+        const int heavy = sc.units[u].heavy;
+        if (heavy < 0) continue;
+        const YzHeavy hv2 = sc.heavy[heavy];
+        const int r0 = sc.units[u].r0, r1 = sc.units[u].r1;
         const int st3 = 3 + (hv2.slot & 1);
-        YzEvent &E = S.ev;
-        const YzHit *base;
-        __syncwarp();  // every lane is done with the previous unit's state
+        const YzTab *tab = sc.tab + YZ_TAB_SETS * (st3 - 3);
+        int ns = -1, count = 0;  // -1: the unit runs on the combined path (survivor kernel)
+        __syncwarp();            // every lane is done with the previous unit's state
         if (hv2.img >= 0) {
-            base = yz_load_image(S, sc.img + hv2.img);
-        } else {
-            yz_event_planes(E, hv, hv2.e, st3);
+            const uint4 *img = sc.img + hv2.img;
+            const YzImgHead &h = *reinterpret_cast<const YzImgHead *>(img);
+            const int total = h.total;
+            float2 *tt = total <= YZ_TT_SMEM ? S.tt : reinterpret_cast<float2 *>(garena);
+            yz_first_load(S, img, tt, total);
+            const unsigned hasx = yz_first_event(S, hv, hv2.e, G, gplane, h.x0, h.tx, h.ex0, h.etx);
             __syncwarp();
-            yz_build(S, E, T, P, st3, base, garena);
-        }
-        Stale *st = S.st;
-        __syncwarp();
+            // inner pairs that reach the fit
+            int nu = 0, nv = 0;
 #pragma unroll 1
-        for (int k = 0; k < 4; ++k) st[k] = un.entry[k];
-        __syncwarp();
-        const int C2 = S.np[0] * S.np[1];
-        int ns = -1;  // -1: the unit runs on the combined path (survivor kernel)
-        if (C2 <= YZ_REC_SMEM || (hv2.img >= 0 && C2 <= YZ_RECORDS_MAX)) {
-            // the inner pairs' records: in shared memory (the window indices
-            // are not needed once the windows exist), else in the per-warp
-            // overflow arena, free when the windows came from an image
-            unsigned long long *R = C2 <= YZ_REC_SMEM ? S.rec : reinterpret_cast<unsigned long long *>(garena);
-            const int nu2 = S.np[0];
+            for (int i = lane; i < S.np[0]; i += 32) nu += yz_group(S, 0, S.pair[0][i]) != 0;
 #pragma unroll 1
-            for (int r = lane; r < C2; r += 32) R[r] = yz_s2_record(S, base, r % nu2, r / nu2);
-            __syncwarp();
+            for (int i = lane; i < S.np[1]; i += 32) nv += yz_group(S, 1, S.pair[1][i]) != 0;
+            const int nf = __reduce_add_sync(0xffffffffu, nu) * __reduce_add_sync(0xffffffffu, nv);
             const float *osc = PRUNE ? yz_tracklet_scores(prune, hv2) : nullptr;
-            yz_first_kept(S, base, un.r0, un.r1, st, sc.tab + YZ_TAB_SETS * (st3 - 3), Q, sc.qcap, &ns, osc,
-                          prune.t_keep, R);
+            // a station without a hodoscope hit in the x window closes the
+            // gates for every combination
+            if (nf == 0 || !(hasx & 3u) || !(hasx & 12u) || !(hasx & 48u)) {
+                ns = sc.count_work && nf ? -1 : 0;
+            } else if (nf <= YZ_FIT_SMEM && total <= YZ_TT_SMEM) {
+                ns = yz_first_walk<PRUNE>(S, G, hasx, S.tt, S.rec, S.r2, nf, r0, r1, st3 == 3, tab, Q, qcap, osc,
+                                          prune.t_keep, &count);
+            } else if (nf <= YZ_FIT_MAX) {
+                ns = yz_first_walk<PRUNE>(S, G, hasx, tt,
+                                          reinterpret_cast<unsigned long long *>(garena + YZ_TT_ARENA_BYTES),
+                                          reinterpret_cast<unsigned short *>(Q + qcap - YZ_R2_ENTRIES), nf, r0, r1,
+                                          st3 == 3, tab, Q, qcap - YZ_R2_ENTRIES, osc, prune.t_keep, &count);
+            }
         }
         __syncwarp();
         long long off = -1;
         if (lane == 0 && ns >= 0) {
-            const unsigned long long o = atomicAdd(pool_ctr, (unsigned long long)ns);
+            const unsigned long long o = ns ? atomicAdd(pool_ctr, (unsigned long long)ns) : 0ull;
             if (o + (unsigned long long)ns <= (unsigned long long)sc.pool_cap) off = (long long)o;
         }
         off = __shfl_sync(0xffffffffu, off, 0);
         if (off >= 0) {
+            n_surv += (unsigned long long)count;
             const uint4 *src = reinterpret_cast<const uint4 *>(Q);
             uint4 *dst = reinterpret_cast<uint4 *>(sc.pool + off);
 #pragma unroll 1
-            for (int i = lane; i < ns * 2; i += 32) dst[i] = src[i];
+            for (int i = lane; i < ns; i += 32) dst[i] = src[i];
         }
         if (lane == 0) sc.useg[u] = make_int2(off >= 0 ? (int)off : -1, off >= 0 ? ns : 0);
         __syncwarp();
     }
+    if (lane == 0 && sc.count_work) yz_flush_counts(sc, 0ull, 0ull, n_surv);
 }
 
 // Split path, second kernel: per unit, the windows again and then its
@@ -2283,39 +2575,39 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_SECOND_WARPS_SM / W > 0 ? OR_YZ
             continue;
         }
         const YzHeavy hv2 = sc.heavy[un.heavy];
-        const float *T = trk_rec(tv, hv2.e, hv2.slot, hv2.k);
+        float *T = trk_rec(tv, hv2.e, hv2.slot, hv2.k);
         const int st3 = 3 + (hv2.slot & 1);
         YzEvent &E = S.ev;
+        Stale *st = S.st;
         __syncwarp();
-        yz_event_planes(E, hv, hv2.e, st3);
+        if (seg.x < 0) yz_event_planes(E, hv, hv2.e, st3);  // the gates and the windows are evaluated here
+        if (lane < 4) st[lane] = sc.units[u].entry[lane];
         __syncwarp();
         const YzHit *base;
         if (hv2.img >= 0) base = yz_load_image(S, sc.img + hv2.img);
         else yz_build(S, E, T, P, st3, base, garena);
         yz_xhits(S, T, P);
         const long C2 = (long)S.np[0] * S.np[1];
+        const YzTab *tab = sc.tab + YZ_TAB_SETS * (st3 - 3);
         unsigned long long bk;
         if (seg.x < 0) {
-            Stale *st = S.st;
-            __syncwarp();
-#pragma unroll 1
-            for (int k = 0; k < 4; ++k) st[k] = un.entry[k];
-            __syncwarp();
             const float *osc = PRUNE ? yz_tracklet_scores(prune, hv2) : nullptr;
-            bk = yz_range_ool<PRUNE>(S, E, base, (long)un.g0 * C2, (long)un.g1 * C2, st, P,
-                                     sc.tab + YZ_TAB_SETS * (st3 - 3), Q, sc.qcap, osc, prune.t_keep);
+            bk = yz_range_ool<PRUNE>(S, E, base, (long)un.g0 * C2, (long)un.g1 * C2, st, P, tab, Q, sc.qcap, osc,
+                                     prune.t_keep);
         } else {
             Phase2Carry cs;
 #pragma unroll 1
             for (int i = 0; i < seg.y; i += 32) {
-                yz_phase2(S, E, base, (int)C2, P, sc.pool + seg.x + i, min(seg.y - i, 32), cs);
+                yz_phase2<true>(S, E, base, (int)C2, P, sc.pool + seg.x + i, min(seg.y - i, 32), tab, cs);
                 __syncwarp();
             }
             bk = cs.best;
         }
         __syncwarp();
         YzBest *dst = sc.best + u;
-        if (bk == ~0ull) {
+        if (hv2.nunits == 1) {  // the tracklet's only unit
+            yz_finish(sc, un.heavy, hv2.c2, T, bk, S.b, S.nhx);
+        } else if (bk == ~0ull) {
             if (lane == 0) dst->key = ~0ull;
         } else {
             const unsigned *src = reinterpret_cast<const unsigned *>(&S.b);
@@ -2329,46 +2621,96 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_SECOND_WARPS_SM / W > 0 ? OR_YZ
 }
 
 
-// one warp per heavy tracklet: its units' minimum key wins
+// Heavy tracklets of several units: the units' minimum key wins (those of
+// one unit are written by the kernel that evaluates it).  A warp reads the
+// unit counts of 32 tracklets at a time: few have more than one.  One warp
+// per tracklet, whatever its units, took 1.18 ms of the 100,000-event batch.
 __global__ void __launch_bounds__(128) yz_apply_kernel(or_tracks_view_t tv, YzScratch sc) {
     const int lane = threadIdx.x & 31;
     const int nheavy = min((int)sc.counters[1], sc.cap_heavy);
 #pragma unroll 1
-    for (int h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; h < nheavy; h += (gridDim.x * blockDim.x) >> 5) {
-        const YzHeavy hv2 = sc.heavy[h];
-        if (hv2.nunits <= 0 || (long)hv2.unit0 + hv2.nunits > sc.cap_units) continue;
-        unsigned long long best = ~0ull;
-        int bu = -1;
+    for (int h0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; h0 < nheavy; h0 += gridDim.x * blockDim.x) {
+        const int mine = h0 + lane < nheavy ? sc.heavy[h0 + lane].nunits : 0;
+        for (unsigned m = __ballot_sync(0xffffffffu, mine > 1); m; m &= m - 1) {
+            const int h = h0 + __ffs(m) - 1;
+            const YzHeavy hv2 = sc.heavy[h];
+            if ((long)hv2.unit0 + hv2.nunits > sc.cap_units) continue;
+            unsigned long long best = ~0ull;
+            int bu = -1;
 #pragma unroll 1
-        for (int u = lane; u < hv2.nunits; u += 32) {
-            const unsigned long long k = sc.best[hv2.unit0 + u].key;
-            if (k < best) {
-                best = k;
-                bu = hv2.unit0 + u;
+            for (int u = lane; u < hv2.nunits; u += 32) {
+                const unsigned long long k = sc.best[hv2.unit0 + u].key;
+                if (k < best) {
+                    best = k;
+                    bu = hv2.unit0 + u;
+                }
             }
-        }
 #pragma unroll 1
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long ok = __shfl_xor_sync(0xffffffffu, best, o);
-            const int ou = __shfl_xor_sync(0xffffffffu, bu, o);
-            if (ok < best) {
-                best = ok;
-                bu = ou;
+            for (int o = 16; o > 0; o >>= 1) {
+                const unsigned long long ok = __shfl_xor_sync(0xffffffffu, best, o);
+                const int ou = __shfl_xor_sync(0xffffffffu, bu, o);
+                if (ok < best) {
+                    best = ok;
+                    bu = ou;
+                }
             }
+            if (best == ~0ull) continue;
+            float *T = trk_rec(tv, hv2.e, hv2.slot, hv2.k);
+            const int nhx = min((int)T[OR_TRK_NHITS], 4);
+            __syncwarp();  // every lane has read the count that yz_finish replaces
+            yz_finish(sc, h, hv2.c2, T, best, sc.best[bu], nhx);
         }
-        if (lane == 0) sc.heavy[h].best_g = best == ~0ull ? -1 : (int)((unsigned)best / (unsigned)max(hv2.c2, 1));
-        if (best == ~0ull) continue;
-        float *T = trk_rec(tv, hv2.e, hv2.slot, hv2.k);
-        const int nhx = min((int)T[OR_TRK_NHITS], 4);
-        yz_store(T, sc.best[bu], nhx);
     }
+}
+
+// Planning units (event, chunk of `chunk` slots) that hold tracklets, in
+// event order within a block; counters[6] = their number.  The planning
+// warps take them one by one from a counter, so units without tracklets (all
+// of a rejected event's) would cost an atomic each: 0.4 ms for 20,000
+// rejected events at one slot per unit.
+constexpr int YZ_LIST_THREADS = 1024;
+__device__ __forceinline__ void yz_list_units(const or_tracks_view_t &tv, const uint8_t *__restrict__ toomany,
+                                              int n_events, int chunk, const YzScratch &sc, int block) {
+    __shared__ int warp_n[YZ_LIST_THREADS / 32];
+    __shared__ unsigned base;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long e = (long)block * (YZ_LIST_THREADS / 32) + w;
+    const bool have = e < n_events && !toomany[e] && tv.ntracks[e * OR_NSLOTS + lane] > 0;
+    const unsigned hm = __ballot_sync(0xffffffffu, have);
+    // the first lane of each chunk with tracklets stands for it
+    const int c0 = lane / chunk * chunk;
+    const unsigned cm = (chunk == 32 ? ~0u : (1u << chunk) - 1u) << c0;
+    const bool take = lane == c0 && (hm & cm) != 0u;
+    const unsigned tm = __ballot_sync(0xffffffffu, take);
+    if (lane == 0) warp_n[w] = __popc(tm);
+    __syncthreads();
+    if (w == 0) {
+        const int v = warp_n[lane];
+        int incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += x;
+        }
+        warp_n[lane] = incl - v;
+        if (lane == 31) base = incl ? atomicAdd(&sc.counters[6], (unsigned)incl) : 0u;
+    }
+    __syncthreads();
+    if (take) sc.list[base + warp_n[w] + __popc(tm & lanemask_lt())] = (unsigned)(e * (OR_NSLOTS / chunk) + lane / chunk);
 }
 
 // The 2 x 81 plane-set entries of the first y fit (see YzTab): for every
 // set, Fit2's normal matrix accumulated over the set's planes in the order
 // u3 u3' v3 v3' u2 u2' v2 v2' with the plane's weight and z, then
 // matinv_2x2 and the errors as in Fit2::solve, and the first cut's bounds.
-__global__ void __launch_bounds__(256) yz_tab_kernel(const or_plane_t *__restrict__ gplane, YzTab *__restrict__ tab) {
+// The blocks after the first list the planning units.
+__global__ void __launch_bounds__(YZ_LIST_THREADS)
+    yz_tab_kernel(const or_plane_t *__restrict__ gplane, YzTab *__restrict__ tab, or_tracks_view_t tv,
+                  const uint8_t *__restrict__ toomany, int n_events, int chunk, YzScratch sc) {
+    if (blockIdx.x > 0) {
+        yz_list_units(tv, toomany, n_events, chunk, sc, (int)blockIdx.x - 1);
+        return;
+    }
     const int t = threadIdx.x;
     if (t >= 2 * YZ_TAB_SETS) return;
     const or_plane_t &P = *gplane;
@@ -2466,6 +2808,9 @@ __global__ void __launch_bounds__(128) yz_outer_labels_kernel(YzScratch sc, or_t
     }
 }
 
+size_t yz_first_smem_bytes(int warps) {
+    return ((sizeof(YzGate) + 15) & ~size_t(15)) + sizeof(YzFirstWarp) * (size_t)warps;
+}
 size_t yz_smem_bytes(int warps) {
     return ((sizeof(or_plane_t) + 15) & ~size_t(15)) + sizeof(YzWarp) * (size_t)warps;
 }
@@ -2489,7 +2834,7 @@ size_t yz_scratch_bytes_q(int cap_units, int cap_heavy, int garena_warps, int qc
         b = (b + 255) & ~size_t(255);
         b += sizeof(int2) * (size_t)cap_units;
         b = (b + 255) & ~size_t(255);
-        b += sizeof(PassEntryStore) * (size_t)yz_pool_cap(qcap, cap_units);
+        b += sizeof(YzSurv) * (size_t)yz_pool_cap(qcap, cap_units);
     }
     if (yz_img_cap(qcap, cap_units) > 0) {
         b = (b + 255) & ~size_t(255);
@@ -2548,7 +2893,7 @@ static YzScratch yz_scratch_layout(void *scratch, int cap_units, int cap_heavy, 
         sc.useg = reinterpret_cast<int2 *>(p);
         p += sizeof(int2) * (size_t)cap_units;
         p = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) + 255) & ~uintptr_t(255));
-        sc.pool = reinterpret_cast<PassEntryStore *>(p);
+        sc.pool = reinterpret_cast<YzSurv *>(p);
     }
     // the images follow the whole pool (pool_limit only narrows its use)
     p = reinterpret_cast<char *>(scratch) + yz_scratch_bytes_q(cap_units, cap_heavy, garena_warps, qcap) -
@@ -2560,6 +2905,7 @@ static YzScratch yz_scratch_layout(void *scratch, int cap_units, int cap_heavy, 
     sc.garena_warps = garena_warps;
     sc.qcap = qcap;
     sc.count_work = 0;
+    sc.list = nullptr;
     return sc;
 }
 
@@ -2586,12 +2932,24 @@ static cudaError_t launch_yz_impl(const or_plane_t *d_plane, or_hits_view_t hv, 
     YzTab *tab = const_cast<YzTab *>(sc.tab);
     sc.count_work = count_work;
     if ((err = cudaMemsetAsync(sc.counters, 0, 256, stream))) return err;
-    yz_tab_kernel<<<1, 256, 0, stream>>>(d_plane, tab);
+    // One slot per planning unit: a heavy event's tracklets spread over 32
+    // warps (a single uneven event's planning pass 442 -> 59 us, 333 of them
+    // 619 -> 107 us, 100,000 12.6 -> 11.8 ms).  With the combination scorer
+    // the unit stays at 8 slots: which light tracklets it evaluates itself,
+    // and so which ones have score rows, depends on the unit's budget.
+    const int chunk = prune.ofeat ? YZ_PLAN_CHUNK_SCORED : YZ_PLAN_CHUNK;
+    const long nplan = (long)n_events * (OR_NSLOTS / chunk);
+    // the list stands in the best records' area, which no kernel before the
+    // survivor kernel uses
+    const bool listed = nplan <= (long)(sizeof(YzBest) / 4) * cap_units;
+    sc.list = listed ? reinterpret_cast<unsigned *>(sc.best) : nullptr;
+    const unsigned list_blocks = listed ? (unsigned)(((long)n_events * 32 + YZ_LIST_THREADS - 1) / YZ_LIST_THREADS) : 0u;
+    yz_tab_kernel<<<1 + list_blocks, YZ_LIST_THREADS, 0, stream>>>(d_plane, tab, tv, toomany, n_events, chunk, sc);
     if ((err = cudaGetLastError())) return err;
     const long blocks = garena_warps / W;
-    const long blocks_plan = min(((long)n_events * (OR_NSLOTS / YZ_PLAN_CHUNK) + W - 1) / W, blocks);
-    yz_plan_kernel<W><<<(unsigned)blocks_plan, W * 32, smem, stream>>>(d_plane, hv, tv, toomany, n_events, sc, errw,
-                                                                       prune);
+    const long blocks_plan = min((nplan + W - 1) / W, blocks);
+    yz_plan_kernel<W><<<(unsigned)blocks_plan, W * 32, smem, stream>>>(d_plane, hv, tv, toomany, n_events, chunk, sc,
+                                                                       errw, prune);
     if ((err = cudaGetLastError())) return err;
     if (prune.model) {
         // score the rows on the tensor cores (the row count stays on the
@@ -2606,17 +2964,19 @@ static cudaError_t launch_yz_impl(const or_plane_t *d_plane, or_hits_view_t hv, 
         if ((err = cudaGetLastError())) return err;
     }
     if (sc.pool_cap > 0) {
+        const size_t smem1 = yz_first_smem_bytes(W);
+        const long res1 = (long)sm_count * (OR_YZ_FIRST_WARPS_SM / W > 0 ? OR_YZ_FIRST_WARPS_SM / W : 1);
         const long res = (long)sm_count * (OR_YZ_SECOND_WARPS_SM / W > 0 ? OR_YZ_SECOND_WARPS_SM / W : 1);
         if (prune.model) {
-            if ((err = smem_attr_once((const void *)yz_first_kernel<W, true>, (int)smem))) return err;
+            if ((err = smem_attr_once((const void *)yz_first_kernel<W, true>, (int)smem1))) return err;
             if ((err = smem_attr_once((const void *)yz_second_kernel<W, true>, (int)smem))) return err;
-            yz_first_kernel<W, true><<<(unsigned)blocks, W * 32, smem, stream>>>(d_plane, hv, tv, sc, prune);
+            yz_first_kernel<W, true><<<(unsigned)min(blocks, res1), W * 32, smem1, stream>>>(d_plane, hv, tv, sc, prune);
             if ((err = cudaGetLastError())) return err;
             yz_second_kernel<W, true><<<(unsigned)min(blocks, res), W * 32, smem, stream>>>(d_plane, hv, tv, sc, prune);
         } else {
-            if ((err = smem_attr_once((const void *)yz_first_kernel<W, false>, (int)smem))) return err;
+            if ((err = smem_attr_once((const void *)yz_first_kernel<W, false>, (int)smem1))) return err;
             if ((err = smem_attr_once((const void *)yz_second_kernel<W, false>, (int)smem))) return err;
-            yz_first_kernel<W, false><<<(unsigned)blocks, W * 32, smem, stream>>>(d_plane, hv, tv, sc, prune);
+            yz_first_kernel<W, false><<<(unsigned)min(blocks, res1), W * 32, smem1, stream>>>(d_plane, hv, tv, sc, prune);
             if ((err = cudaGetLastError())) return err;
             yz_second_kernel<W, false><<<(unsigned)min(blocks, res), W * 32, smem, stream>>>(d_plane, hv, tv, sc,
                                                                                           prune);
