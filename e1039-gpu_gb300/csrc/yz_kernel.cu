@@ -118,6 +118,7 @@ constexpr int YZ_PLAN_CHUNK_SCORED = 8;          // ... with the combination sco
 #endif
 constexpr long YZ_UNIT = OR_YZ_UNIT;    // live combinations per queued unit (whole (u3,v3) iterations)
 constexpr int YZ_GARENA_HITS = 8 * YZ_MAXWIN;  // per-warp global overflow arena
+static_assert(OR_MAXHITS_CHAM <= 256, "a chamber plane's hit index fits a byte");
 // survivors of the first cut wait in a per-warp queue in global memory and
 // are evaluated in a batch when it fills or the range ends, so that the two
 // phases do not alternate every 32 survivors (each switch refetches the
@@ -254,18 +255,20 @@ struct PassEntryStore {
     int stdet;
 };
 
-// A survivor as the first-cut kernel hands it to the survivor kernel:
-// combination index, first fit, and a code: bits 0-9 the arena offset of the
-// scratch entry past its hit count, bits 10-11 where that entry stands
-// (YZ_ENT_*), bits 12-13 the unit's starting entry (4..7) when it stands
-// there, bits 14-20 the plane set's table index, bit 31 whether the gates
-// passed (a survivor that fails them is only kept for the station-3 signs it
-// sets).
+// A survivor as the first-cut kernel hands it to the survivor kernel: its
+// four pairs (7 bits each: u3, v3, u2, v2), its first fit, and a code: bits
+// 0-9 the arena offset of the scratch entry past its hit count, bits 10-11
+// where that entry stands (YZ_ENT_*), bits 12-13 the unit's starting entry
+// (4..7) when it stands there, bits 14-20 the plane set's table index, bits
+// 22-29 the planes that give a hit (u3 u3' v3 v3' u2 u2' v2 v2'), bit 31
+// whether the gates passed (a survivor that fails them is only kept for the
+// station-3 signs it sets).
 struct __align__(16) YzSurv {
-    int c;
+    unsigned pairs;
     float y0, ty;
     unsigned code;
 };
+static_assert(YZ_MAXPAIR <= 128, "a pair index fits 7 bits");
 constexpr unsigned YZ_ENT_HIT = 1u, YZ_ENT_UNIT = 2u;  // 0: no such entry
 
 struct YzEvent {
@@ -281,9 +284,11 @@ struct YzWarp {
     YzHit arena[YZ_ARENA_HITS];
     short2 pair[4][YZ_MAXPAIR];  // windowed indices (or -1) in sides 0, 1 of list q
     struct {
-        short widx[8][YZ_MAXWIN];  // plane hit index of each windowed hit
-        uint8_t wfl[2][YZ_MAXWIN];
-    } w;                           // while the windows are built
+        int start[8];
+        float xmin[4], xmax[4];
+        unsigned fl[(8 * YZ_MAXWIN + 31) / 32];  // windowed hits that are in a pair
+        unsigned char widx[8 * YZ_MAXWIN];       // plane hit index of each windowed hit
+    } w;                                         // while the windows are built
     int np[4], nw[8], woff[8];
     float x0, tx, ex0, etx;
     int nhx;
@@ -297,7 +302,9 @@ struct YzWarp {
 // The event's plane views for a tracklet of station half st3, one plane per
 // lane (every lane calls): u2 u2' v2 v2' u3 u3' v3 v3' (K:910-984), the
 // prop-tube y planes and the x hodoscopes of stations 2-4.
-__device__ __forceinline__ void yz_event_planes(YzEvent &E, const or_hits_view_t &hv, long e, int st3) {
+// chambers: only the u and v planes.
+__device__ __forceinline__ void yz_event_planes(YzEvent &E, const or_hits_view_t &hv, long e, int st3,
+                                                bool chambers = false) {
     const int lane = lane_id();
     int det = 0;
     HitPlane *dst = nullptr;
@@ -307,6 +314,7 @@ __device__ __forceinline__ void yz_event_planes(YzEvent &E, const or_hits_view_t
             : lane == 4 ? u3 : lane == 5 ? u3 - 1 : lane == 6 ? v3 : v3 - 1;
         E.dl[lane] = (short)det;
         dst = &E.hc[lane];
+    } else if (chambers) {
     } else if (lane < 12) {
         det = lane == 8 ? DET_P1Y1 : lane == 9 ? DET_P1Y2 : lane == 10 ? DET_P2Y1 : DET_P2Y2;
         dst = lane == 8 ? &E.p1y1 : lane == 9 ? &E.p1y2 : lane == 10 ? &E.p2y1 : &E.p2y2;
@@ -321,116 +329,156 @@ __device__ __forceinline__ void yz_event_planes(YzEvent &E, const or_hits_view_t
 // Build the tracklet's windows (make_hitpairs_in_station, H:464-549) with the
 // per-hit y of this tracklet (calculate_y_uvhit, H:75-100).  Returns false
 // when a window or a pair list exceeds the reference's 100-entry arrays.
+//
+// The hits of the eight planes are one index space in list order, and so are
+// the hits in the windows, the candidate pairs of the four projections and
+// the hits left unpaired: 32 entries of each at a time, whatever plane they
+// belong to.  A plane holds some ten hits and a window some five, so plane
+// by plane most lanes were idle and the loops' instructions were fetched
+// eight times over (planning pass of 100,000 uneven events, with the changes
+// to the unit states below: 12.1 -> 5.2 ms).
 __device__ bool yz_build(YzWarp &S, const YzEvent &E, const float *T, const or_plane_t &P, int st3,
                          const YzHit *&base, YzHit *garena) {
     const int lane = lane_id();
+    const unsigned lt = lanemask_lt();
     const float x0 = T[OR_TRK_X0], tx = T[OR_TRK_TX], ex0 = T[OR_TRK_ERR_X0], etx = T[OR_TRK_ERR_TX];
-    const int stid_of[4] = {2, 2, st3, st3}, proj_of[4] = {1, 2, 1, 2};
-    bool ok = true;
-    int total = 0;
-    // windowed hit lists, in plane order (H:480-511)
-#pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
-        const int a = 2 * q;
-        const float za = P.z[E.dl[a]], zb = P.z[E.dl[a + 1]];
-        const float sp = P.spacing[E.dl[a]];
-        const float xmin = fminf((tx - etx) * za, (tx - etx) * zb) + x0 - ex0 - sp;
-        const float xmax = fmaxf((tx + etx) * za, (tx + etx) * zb) + x0 + ex0 + sp;
-#pragma unroll 1
-        for (int side = 0; side < 2; ++side) {
-            const HitPlane &h = E.hc[a + side];
-            const int det = E.dl[a + side];
-            int c = 0;
-#pragma unroll 1
-            for (int b0 = 0; b0 < h.n; b0 += 32) {
-                const int i = b0 + lane;
-                const bool in = i < h.n && wp_in_window(det, h.chan(i), xmin, xmax, P);
-                const unsigned m = __ballot_sync(0xffffffffu, in);
-                if (in) {
-                    const int k = c + __popc(m & lanemask_lt());
-                    if (k < YZ_MAXWIN) S.w.widx[a + side][k] = (short)i;
-                }
-                c += __popc(m);
-            }
-            if (c > YZ_MAXWIN) ok = false;
-            c = min(c, YZ_MAXWIN);
-            if (lane == 0) {
-                S.nw[a + side] = c;
-                S.woff[a + side] = total;
-            }
-            total += c;
+    // hits of the planes before plane `lane`, and the window of each projection
+    int start, total;
+    {
+        const int n = lane < 8 ? E.hc[lane].n : 0;
+        start = n;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, start, o);
+            if (lane >= o) start += v;
+        }
+        total = __shfl_sync(0xffffffffu, start, 7);
+        start -= n;
+        if (lane < 8) S.w.start[lane] = start;
+        if (lane < 4) {
+            const float za = P.z[E.dl[2 * lane]], zb = P.z[E.dl[2 * lane + 1]];
+            const float sp = P.spacing[E.dl[2 * lane]];
+            S.w.xmin[lane] = fminf((tx - etx) * za, (tx - etx) * zb) + x0 - ex0 - sp;
+            S.w.xmax[lane] = fmaxf((tx + etx) * za, (tx + etx) * zb) + x0 + ex0 + sp;
+            S.np[lane] = 0;
         }
     }
+    __syncwarp();
+    // list of entry i of an index space whose lists start at s[0..7]
+    auto list_of = [](const int *s, int i) {
+        int l = 0;
+#pragma unroll
+        for (int k = 1; k < 8; ++k) l += i >= s[k];
+        return l;
+    };
+    // windowed hits, in list order (H:480-511)
+    int nwin = 0, wo = -1;
+#pragma unroll 1
+    for (int b0 = 0; b0 < total; b0 += 32) {
+        const int f = b0 + lane;
+        bool in = false;
+        int i = 0;
+        if (f < total) {
+            const int l = list_of(S.w.start, f);
+            i = f - S.w.start[l];
+            in = wp_in_window(E.dl[l], E.hc[l].chan(i), S.w.xmin[l >> 1], S.w.xmax[l >> 1], P);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        const int k = nwin + __popc(m & lt);
+        if (in && k < 8 * YZ_MAXWIN) S.w.widx[k] = (unsigned char)i;
+        if (lane < 8 && start >= b0 && start < b0 + 32) wo = nwin + __popc(m & ((1u << (start - b0)) - 1u));
+        nwin += __popc(m);
+    }
+    if (wo < 0) wo = nwin;
+    const int next = __shfl_down_sync(0xffffffffu, wo, 1);
+    const int nw = (lane == 7 ? nwin : next) - wo;
+    if (__any_sync(0xffffffffu, lane < 8 && nw > YZ_MAXWIN)) return false;
+    if (lane < 8) {
+        S.nw[lane] = nw;
+        S.woff[lane] = wo;
+    }
+    if (lane < (8 * YZ_MAXWIN + 31) / 32) S.w.fl[lane] = 0u;
     __syncwarp();
     // windowed hit records (K:1326-1355 computes these per combination)
-    YzHit *dst = (total <= YZ_ARENA_HITS) ? S.arena : garena;
+    YzHit *dst = (nwin <= YZ_ARENA_HITS) ? S.arena : garena;
 #pragma unroll 1
-    for (int l = 0; l < 8; ++l) {
+    for (int k = lane; k < nwin; k += 32) {
+        const int l = list_of(S.woff, k);
         const HitPlane &h = E.hc[l];
         const int det = E.dl[l];
-#pragma unroll 1
-        for (int i = lane; i < S.nw[l]; i += 32) {
-            const int hi = S.w.widx[l][i];
-            YzHit r;
-            r.det = (short)det;
-            r.el = (short)h.chan(hi);
-            r.tdc = h.tdc(hi);
-            r.drift = h.drift(hi);
-            r.pos = h.pos(hi);
-            float yy = 0.f, ey = 0.f;
-            r.acc = calculate_y_uvhit(det, r.el, r.drift, 0, x0, tx, P, yy, ey) ? 1 : 0;
-            r.Y = yy;
-            r.eY = ey;
-            r.z = P.z[det];
-            dst[S.woff[l] + i] = r;
-        }
+        const int hi = S.w.widx[k];
+        YzHit r;
+        r.det = (short)det;
+        r.el = (short)h.chan(hi);
+        r.tdc = h.tdc(hi);
+        r.drift = h.drift(hi);
+        r.pos = h.pos(hi);
+        float yy = 0.f, ey = 0.f;
+        r.acc = calculate_y_uvhit(det, r.el, r.drift, 0, x0, tx, P, yy, ey) ? 1 : 0;
+        r.Y = yy;
+        r.eY = ey;
+        r.z = P.z[det];
+        dst[k] = r;
     }
     __syncwarp();
-    // pairs over each projection's two windowed lists (H:513-546)
-#pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
-        const int a = 2 * q;
-        const int c1 = S.nw[a], c2 = S.nw[a + 1];
-#pragma unroll 1
-        for (int i = lane; i < c1; i += 32) S.w.wfl[0][i] = 0;
-#pragma unroll 1
-        for (int i = lane; i < c2; i += 32) S.w.wfl[1][i] = 0;
+    // append to projection q's pair list, in lane order
+    auto append = [&](bool take, int q, short2 v) {
+        const unsigned peers = __match_any_sync(0xffffffffu, take ? q : 4 + lane);
+        int at = 0;
+        if (take) {
+            at = S.np[q];
+            const int k = at + __popc(peers & lt);
+            if (k < YZ_MAXPAIR) S.pair[q][k] = v;
+        }
         __syncwarp();
-        const float spacing = c_spacingplane[c_detsuperid[stid_of[q]][proj_of[q]]];
-        int np = 0;
+        if (take && (peers & lt) == 0u) S.np[q] = at + __popc(peers);
+        __syncwarp();
+    };
+    // pairs over each projection's two windowed lists (H:513-546)
+    {
+        const int n2 = __shfl_down_sync(0xffffffffu, nw, 1);
+        const int c12 = lane < 8 && (lane & 1) == 0 ? nw * n2 : 0;  // lane 2q: projection q
+        int incl = c12;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        const int npair = __shfl_sync(0xffffffffu, incl, 7);
+        if (lane < 8 && (lane & 1) == 0) S.w.start[lane >> 1] = incl - c12;
+        __syncwarp();
 #pragma unroll 1
-        for (int b0 = 0; b0 < c1 * c2; b0 += 32) {
-            const int c = b0 + lane;
+        for (int b0 = 0; b0 < npair; b0 += 32) {
+            const int f = b0 + lane;
             bool take = false;
+            int q = 0;
             short2 v = make_short2(0, 0);
-            if (c < c1 * c2) {
-                const int ia = c / c2, ib = c - ia * c2;
-                if (!(fabsf(dst[S.woff[a] + ia].pos - dst[S.woff[a + 1] + ib].pos) > spacing)) {
+            if (f < npair) {
+                q = (f >= S.w.start[1]) + (f >= S.w.start[2]) + (f >= S.w.start[3]);
+                const int n2 = S.nw[2 * q + 1], c = f - S.w.start[q];
+                const int ia = c / n2, ib = c - ia * n2;
+                const float spacing = c_spacingplane[c_detsuperid[q < 2 ? 2 : st3][1 + (q & 1)]];
+                const int oa = S.woff[2 * q] + ia, ob = S.woff[2 * q + 1] + ib;
+                if (!(fabsf(dst[oa].pos - dst[ob].pos) > spacing)) {
                     take = true;
                     v = make_short2((short)ia, (short)ib);
-                    S.w.wfl[0][ia] = 1;
-                    S.w.wfl[1][ib] = 1;
+                    atomicOr(&S.w.fl[oa >> 5], 1u << (oa & 31));
+                    atomicOr(&S.w.fl[ob >> 5], 1u << (ob & 31));
                 }
             }
-            wp_append(take, v, S.pair[q], YZ_MAXPAIR, np);
+            append(take, q, v);
         }
-        __syncwarp();
-#pragma unroll 1
-        for (int b0 = 0; b0 < c1; b0 += 32) {
-            const int ia = b0 + lane;
-            const bool take = ia < c1 && !S.w.wfl[0][ia];
-            wp_append(take, make_short2((short)ia, -1), S.pair[q], YZ_MAXPAIR, np);
-        }
-#pragma unroll 1
-        for (int b0 = 0; b0 < c2; b0 += 32) {
-            const int ib = b0 + lane;
-            const bool take = ib < c2 && !S.w.wfl[1][ib];
-            wp_append(take, make_short2(-1, (short)ib), S.pair[q], YZ_MAXPAIR, np);
-        }
-        if (np > YZ_MAXPAIR) ok = false;
-        if (lane == 0) S.np[q] = min(np, YZ_MAXPAIR);
-        __syncwarp();
     }
+    // then the hits without a partner, first plane's before second plane's
+#pragma unroll 1
+    for (int b0 = 0; b0 < nwin; b0 += 32) {
+        const int k = b0 + lane;
+        const bool take = k < nwin && !((S.w.fl[b0 >> 5] >> lane) & 1u);
+        const int l = take ? list_of(S.woff, k) : 0;
+        const short i = (short)(k - S.woff[l]);
+        append(take, l >> 1, (l & 1) ? make_short2(-1, i) : make_short2(i, -1));
+    }
+    const bool ok = !__any_sync(0xffffffffu, lane < 4 && S.np[lane & 3] > YZ_MAXPAIR);
     base = dst;
     if (lane == 0) {
         S.x0 = x0;
@@ -819,6 +867,97 @@ __device__ void yz_unit_states(const YzWarp &S, const YzHit *base, int G, int gp
     __syncwarp();
 }
 
+// Accepted hits of a pair of projection q (bit 0: first plane, bit 1: second).
+__device__ __forceinline__ int yz_pair_group(const YzWarp &S, const YzHit *base, int q, int i) {
+    const short2 p = S.pair[q][i];
+    return (p.x >= 0 && base[S.woff[2 * q] + p.x].acc ? 1 : 0) | (p.y >= 0 && base[S.woff[2 * q + 1] + p.y].acc ? 2 : 0);
+}
+
+// Which pairs of a projection come last, by their accepted hits.
+struct YzLast {
+    int one, two, r1;  // one hit; two hits; a second attempt after an accepted first one; -1: no such pair
+};
+__device__ __forceinline__ YzLast yz_last_pairs(const YzWarp &S, const YzHit *base, int q) {
+    YzLast o{-1, -1, -1};
+#pragma unroll 1
+    for (int b0 = 0; b0 < S.np[q]; b0 += 32) {
+        const int i = b0 + lane_id();
+        int g = 0;
+        bool r1 = false;
+        if (i < S.np[q]) {
+            g = yz_pair_group(S, base, q, i);
+            r1 = (g & 1) && S.pair[q][i].y >= 0;
+        }
+        const unsigned m1 = __ballot_sync(0xffffffffu, g == 1 || g == 2);
+        const unsigned m2 = __ballot_sync(0xffffffffu, g == 3);
+        const unsigned mr = __ballot_sync(0xffffffffu, r1);
+        if (m1) o.one = b0 + last_lane(m1);
+        if (m2) o.two = b0 + last_lane(m2);
+        if (mr) o.r1 = b0 + last_lane(mr);
+    }
+    return o;
+}
+
+// The last write of offset m = 0..3 past the station-3 hits over the inner
+// pairs of an outer iteration (what yz_last_writes finds by walking them),
+// from which u2 and v2 pairs come last: a combination tries its u2 pair, and
+// after an accepted u2 hit its v2 pair, each hit at the count so far.  `first`
+// / `second` give a pair's hits as arena offsets (-1: none) and the offset its
+// first attempt's place ends with.
+template <class First, class Rel0>
+__device__ __forceinline__ unsigned long long yz_lasto(int nu2, int nv2, const YzLast &u, const YzLast &v, First second,
+                                                       Rel0 rel0) {
+    unsigned o1 = 0xFFFFu, o2 = 0xFFFFu, o3 = 0xFFFFu;
+    const unsigned o0 = rel0(0, nu2 - 1);
+    if (u.one > u.two) o1 = rel0(1, nv2 - 1);
+    else if (u.two >= 0) o1 = second(0, u.two);
+    if (u.two >= 0) o2 = u.one > u.two && v.r1 == nv2 - 1 ? second(1, v.r1) : rel0(1, nv2 - 1);
+    else if (u.one >= 0 && v.r1 >= 0) o2 = second(1, v.r1);
+    if (u.two >= 0 && v.r1 >= 0) o3 = second(1, v.r1);
+    return (unsigned long long)o0 | ((unsigned long long)o1 << 16) | ((unsigned long long)o2 << 32) |
+           ((unsigned long long)o3 << 48);
+}
+
+// The scratch entries 4..7 after a whole tracklet: for each entry, the last
+// live outer iteration whose station-3 hit count puts one of the inner pairs'
+// writes there.  The last iteration of n3 hits is the last v3 pair of one
+// kind with the last u3 pair of another.
+__device__ void yz_final_state(const YzWarp &S, const YzHit *base, Stale st[4]) {
+    const YzLast u2 = yz_last_pairs(S, base, 0), v2 = yz_last_pairs(S, base, 1);
+    const YzLast u3 = yz_last_pairs(S, base, 2), v3 = yz_last_pairs(S, base, 3);
+    auto second = [&](int q, int i) { return (unsigned)(S.woff[2 * q + 1] + S.pair[q][i].y); };
+    auto rel0 = [&](int q, int i) {
+        const short2 p = S.pair[q][i];
+        const bool sec = p.x < 0 || (!base[S.woff[2 * q] + p.x].acc && p.y >= 0);
+        return (unsigned)(sec ? S.woff[2 * q + 1] + p.y : S.woff[2 * q] + p.x);
+    };
+    const unsigned long long lasto = yz_lasto(S.np[0], S.np[1], u2, v2, second, rel0);
+    const int nu3 = S.np[2];
+    auto g_of = [&](int iu, int iv) { return iu >= 0 && iv >= 0 ? iv * nu3 + iu : -1; };
+    const int lastg[3] = {g_of(u3.one, v3.one), max(g_of(u3.one, v3.two), g_of(u3.two, v3.one)), g_of(u3.two, v3.two)};
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        int best = -1;
+        unsigned off = 0xFFFFu;
+#pragma unroll
+        for (int n3 = 2; n3 <= 4; ++n3) {
+            const int mm = k + 4 - n3;
+            if (mm > 3) continue;
+            const unsigned o = (unsigned)(lasto >> (16 * mm)) & 0xFFFFu;
+            if (o != 0xFFFFu && lastg[n3 - 2] > best) {
+                best = lastg[n3 - 2];
+                off = o;
+            }
+        }
+        if (off != 0xFFFFu && lane_id() == 0) {
+            const YzHit &r = base[off];
+            st[k] = Stale{r.det, r.pos, r.drift};
+        }
+    }
+    __syncwarp();
+}
+
 // A combination that passed the first y cut, queued for the full evaluation:
 // index inside the tracklet, first fit, scratch entry past its hit count.
 using PassEntry = PassEntryStore;
@@ -843,6 +982,26 @@ __device__ __forceinline__ int yz_gather(const YzWarp &S, const YzHit *base, int
         const int off = S.woff[l] + wi;
         if (!base[off].acc) continue;
         const unsigned long long f = (unsigned long long)off << (16 * (nuv & 3));
+        if (nuv < 4) U.lo |= f;
+        else U.hi |= f;
+        ++nuv;
+    }
+    return nuv;
+}
+
+// The same from the pairs and the planes that give a hit (bits u3 u3' v3 v3'
+// u2 u2' v2 v2').
+__device__ __forceinline__ int yz_gather_planes(const YzWarp &S, int iu3, int iv3, int iu2, int iv2, unsigned planes,
+                                                UvSet &U, int &n3) {
+    const short2 p3u = S.pair[2][iu3], p3v = S.pair[3][iv3], p2u = S.pair[0][iu2], p2v = S.pair[1][iv2];
+    int nuv = 0;
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+        if (a == 4) n3 = nuv;
+        if (!((planes >> a) & 1u)) continue;
+        const short2 p = a < 2 ? p3u : a < 4 ? p3v : a < 6 ? p2u : p2v;
+        const unsigned long long f = (unsigned long long)(S.woff[(a + 4) & 7] + ((a & 1) ? p.y : p.x))
+                                     << (16 * (nuv & 3));
         if (nuv < 4) U.lo |= f;
         else U.hi |= f;
         ++nuv;
@@ -929,10 +1088,16 @@ __device__ __noinline__ void yz_phase2(YzWarp &S, const YzEvent &E, const YzHit 
     const bool valid = lane < n;
     PassEntry q;
     bool gated = false;
+    UvSet U{0ull, 0ull, 0u};
+    int n3 = 0, nuv = 0, g = -1 - lane;
     if constexpr (GATED) {
         if (valid) {
             const uint4 v = *reinterpret_cast<const uint4 *>(Qc + lane);
-            q.c = (int)v.x;
+            const int iu3 = (int)(v.x & 127u), iv3 = (int)(v.x >> 7) & 127;
+            const int iu2 = (int)(v.x >> 14) & 127, iv2 = (int)(v.x >> 21) & 127;
+            g = iu3 + iv3 * S.np[2];
+            q.c = g * C2 + iu2 + iv2 * S.np[0];
+            nuv = yz_gather_planes(S, iu3, iv3, iu2, iv2, v.w >> 22, U, n3);
             q.y0 = __uint_as_float(v.y);
             q.ty = __uint_as_float(v.z);
             gated = (v.w >> 31) != 0u;
@@ -955,10 +1120,10 @@ __device__ __noinline__ void yz_phase2(YzWarp &S, const YzEvent &E, const YzHit 
         q = Qc[lane];
     }
     const int c = valid ? q.c : 0;
-    const int g = valid ? c / C2 : -1 - lane;
-    UvSet U{0ull, 0ull, 0u};
-    int n3 = 0, nuv = 0;
-    if (valid) nuv = yz_gather(S, base, c, C2, U, n3);
+    if constexpr (!GATED) g = valid ? c / C2 : -1 - lane;
+    if constexpr (!GATED) {
+        if (valid) nuv = yz_gather(S, base, c, C2, U, n3);
+    }
     const Stale stj{(short)(valid ? q.stdet : DET_SENTINEL), valid ? q.stpos : 0.f, valid ? q.stdrift : 0.f};
     const float y0 = valid ? q.y0 : 0.f, ty = valid ? q.ty : 0.f;
     const float ey0 = valid ? q.ey0 : 0.f, ety = valid ? q.ety : 0.f;
@@ -1104,7 +1269,7 @@ __device__ __noinline__ void yz_phase2(YzWarp &S, const YzEvent &E, const YzHit 
 // and hodoscope gates, chi2 (K:1613-1799).  This combined walk serves the
 // planning kernel's light tracklets and the units whose survivors do not fit
 // the pool; the first-cut kernel walks listed outer iterations with the
-// inner pairs' records instead (yz_first_kept).
+// inner pairs' lists instead (yz_first_walk).
 //
 // Outer iterations (iu3, iv3) whose u3 pair or v3 pair gives no accepted hit
 // are skipped whole: the reference leaves such an iteration before any
@@ -1641,36 +1806,35 @@ __device__ unsigned long long yz_range_t(YzWarp &S, const YzEvent &E, const YzHi
 // ---------------------------------------------------------------------------
 //
 // A combination is an outer iteration (u3, v3) with an inner pair (u2, v2).
-// Everything the cut needs from either side is made once per unit:
-//   - per outer iteration, 32 listed at a time: the fit's right-hand side
-//     over its station-3 hits, its hit count and plane set, and the scratch
-//     entries 4..7 as the iteration finds them (a last-writer scan over the
-//     live iterations before it; which entries an iteration leaves depends
-//     on its hit count alone, the inner pairs being the same in every one);
-//   - per inner pair that reaches the fit, in order: the accepted hits, the
-//     plane set, and the scratch entry past the hit count where this pair or
-//     an earlier one of the same outer iteration has written it.
-// A combination then costs its additions, two dot products and two compares,
-// and its scratch entry is a lookup.  Combinations that pass wait in a ring
-// in shared memory; 32 at a time they go through the prop-tube and hodoscope
-// gates, all lanes in use.  Only those that pass reach the survivor kernel,
-// with the two kinds that set station-3 signs for them: the first survivor
-// of their outer iteration, and the survivors whose walk pairs the last
-// station-3 hit with the first station-2 hit (planes 19, 18).
+// Of each projection only the pairs with an accepted hit matter; they are
+// listed once per unit with their terms of the fit's right-hand side, and the
+// combinations are walked over those lists, so each costs its additions, two
+// dot products and two compares.
+//   - Per outer iteration, 32 at a time: the sums over its station-3 hits,
+//     its hit count and plane set, and the scratch entries 4..7 as the
+//     iteration finds them (a last-writer scan over the live iterations
+//     before it; which entries an iteration leaves depends on its hit count
+//     alone, the inner pairs being the same in every one).
+//   - The scratch entry past a combination's hit count is only read by the
+//     left/right walk when its last hit is a v2 hit without its partner
+//     plane's, and only pairs with a hit of that plane; the last writer of
+//     that entry follows from the lists (yz_stale_code).
+// Combinations that pass wait in a ring in shared memory; 32 at a time they
+// go through the prop-tube and hodoscope gates, all lanes in use.  Only those
+// that pass reach the survivor kernel, with the two kinds that set station-3
+// signs for them: the first survivor of their outer iteration, and the
+// survivors whose walk pairs the last station-3 hit with the first station-2
+// hit (planes 19, 18).
 //
-// Bound: instruction issue.  Listing each inner pair's attempts per
-// combination, scanning the scratch entries over every chunk of 32 and
-// passing every survivor on took 22.9 ms of the 100,000-event uneven batch
-// with 19.5 ms in the survivor kernel; this takes 10.6 ms with 8.2 ms.
-constexpr int YZ_KEPT_BATCH = 32;     // outer iterations listed at a time
-constexpr int YZ_TT_SMEM = 256;       // hits whose fit terms are kept in shared memory
-constexpr int YZ_FIT_SMEM = 180;      // inner pairs' records kept in shared memory
-constexpr int YZ_PROP_SMEM = 40;      // hits per prop-tube y plane kept in shared memory
-// ... beyond them in the warp's overflow arena: the terms of every hit, then
-// the records, whose pair indices take the end of the warp's survivor queue
-constexpr int YZ_TT_ARENA_BYTES = YZ_GARENA_HITS * 8;
-constexpr int YZ_FIT_MAX = (int)(YZ_GARENA_HITS * sizeof(YzHit) - YZ_TT_ARENA_BYTES) / 8;
-constexpr int YZ_R2_ENTRIES = (YZ_FIT_MAX * 2 + (int)sizeof(YzSurv) - 1) / (int)sizeof(YzSurv);
+// Bound: instruction issue.  Rebuilding each combination's station-3 part and
+// attempts, scanning the scratch entries over every chunk of 32 and passing
+// every survivor on took 22.9 ms of the 100,000-event uneven batch with 19.5
+// ms in the survivor kernel; this takes 9.2 ms with 8.3 ms.
+constexpr int YZ_KEPT_BATCH = 32;  // outer iterations listed at a time
+constexpr int YZ_LIST_SMEM = 48;   // pairs per projection listed in shared memory; a unit with more uses the
+                                   // warp's overflow arena
+constexpr int YZ_PROP_SMEM = 40;   // hits per prop-tube y plane kept in shared memory
+static_assert(4 * YZ_MAXPAIR * (sizeof(float4) + 4) <= YZ_GARENA_HITS * sizeof(YzHit), "the lists fit the arena");
 
 // hodoscope x planes of stations 2-4 and the prop-tube y planes
 struct YzGate {
@@ -1679,61 +1843,124 @@ struct YzGate {
 };
 
 struct YzFirstWarp {
-    uint4 ring[64];  // survivors waiting for the gates: pair (g << 14 | r2), y0, ty, code
-    unsigned long long rec[YZ_FIT_SMEM];
+    uint4 ring[64];  // survivors waiting for the gates (YzSurv; code bit 21: may pair planes 19 and 18)
+    float4 term[4][YZ_LIST_SMEM];   // u2 v2 u3 v3 pairs with an accepted hit: (eY Y, eY Y z) of each hit, 0 if refused
+    unsigned info[4][YZ_LIST_SMEM]; // pair | planes << 7; v2: | latest earlier pair with two attempts << 16
     unsigned long long kent[YZ_KEPT_BATCH];  // scratch entries 4..7, 16 bits each: arena offset, 0xFFFF = the unit's
     float2 kb[YZ_KEPT_BATCH];
-    unsigned kt[YZ_KEPT_BATCH];  // g | table offset << 14 | n3 << 21 | only v3' << 24
-    float2 tt[YZ_TT_SMEM];       // (eY * Y, eY * Y * z) of each windowed hit
+    unsigned kt[YZ_KEPT_BATCH];  // pairs u3, v3 | table offset << 14 | planes << 21 | n3 << 25
     uint4 pend;                  // the current outer iteration's first survivor, not passed on yet
     float prop[4][YZ_PROP_SMEM];
-    uchar2 pair[4][YZ_MAXPAIR];  // 255 = none
-    unsigned acc[(8 * YZ_MAXWIN + 31) / 32];
-    int np[4], woff[8];
     HitPlane pp[4];
-    unsigned short r2[YZ_FIT_SMEM];
+    int np[4], woff[8];
 };
 
-__device__ __forceinline__ bool yz_acc(const YzFirstWarp &S, int off) { return (S.acc[off >> 5] >> (off & 31)) & 1u; }
-// which of a pair's two hits are accepted (bit 0: the first plane's)
-__device__ __forceinline__ int yz_group(const YzFirstWarp &S, int q, uchar2 p) {
-    return (p.x != 255 && yz_acc(S, S.woff[2 * q] + p.x) ? 1 : 0) |
-           (p.y != 255 && yz_acc(S, S.woff[2 * q + 1] + p.y) ? 2 : 0);
+// What the scratch entries need to know of a unit's u2 and v2 pairs.
+struct YzInner {
+    const uint4 *hits;    // the image's arena
+    const short2 *pu, *pv;
+    int ou, ov, ova;      // arena offsets of the lists u2', v2' and v2
+    YzLast u, v;
+    int first_two;        // first u2 pair with two accepted hits
+};
+
+__device__ __forceinline__ bool yz_img_acc(const uint4 *hits, int off) { return hits[2 * off + 1].w != 0u; }
+
+// List the pairs of projection q with an accepted hit, in order; returns
+// their number.
+__device__ __forceinline__ int yz_first_list(const YzFirstWarp &S, int q, const short2 *__restrict__ pair,
+                                             const uint4 *__restrict__ hits, float4 *term, unsigned *info, YzLast &last,
+                                             int &first_two) {
+    const int lane = lane_id();
+    const unsigned lt = lanemask_lt();
+    const int n = S.np[q], oa = S.woff[2 * q], ob = S.woff[2 * q + 1];
+    last = YzLast{-1, -1, -1};
+    first_two = 1 << 20;
+    int count = 0;
+#pragma unroll 1
+    for (int b0 = 0; b0 < n; b0 += 32) {
+        const int i = b0 + lane;
+        int g = 0;
+        bool r1 = false;
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < n) {
+            const short2 p = pair[i];
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                const int k = a == 0 ? p.x : p.y;
+                if (k < 0) continue;
+                const int off = (a == 0 ? oa : ob) + k;
+                const uint4 v = hits[2 * off + 1];  // tdc, z, det | el, acc
+                if (v.w == 0u) continue;
+                const float2 ye = *reinterpret_cast<const float2 *>(hits + 2 * off);
+                const float s = ye.y * ye.x, sz = s * __uint_as_float(v.y);
+                g |= 1 << a;
+                if (a == 0) {
+                    t.x = s;
+                    t.y = sz;
+                } else {
+                    t.z = s;
+                    t.w = sz;
+                }
+            }
+            r1 = (g & 1) && p.y >= 0;
+        }
+        const unsigned m1 = __ballot_sync(0xffffffffu, g == 1 || g == 2);
+        const unsigned m2 = __ballot_sync(0xffffffffu, g == 3);
+        const unsigned mr = __ballot_sync(0xffffffffu, r1);
+        if (g) {
+            const int k = count + __popc((m1 | m2) & lt);
+            const int pr = last_lane(mr & lt);
+            term[k] = t;
+            info[k] = (unsigned)(i | g << 7) | (unsigned)(pr >= 0 ? b0 + pr : (last.r1 >= 0 ? last.r1 : 255)) << 16;
+        }
+        count += __popc(m1 | m2);
+        if (m2 && last.two < 0) first_two = b0 + __ffs(m2) - 1;
+        if (m1) last.one = b0 + last_lane(m1);
+        if (m2) last.two = b0 + last_lane(m2);
+        if (mr) last.r1 = b0 + last_lane(mr);
+    }
+    return count;
 }
 
-// A tracklet's windows from its image, as the first cut needs them.
-__device__ __forceinline__ void yz_first_load(YzFirstWarp &S, const uint4 *__restrict__ img, float2 *tt, int total) {
-    const int lane = lane_id();
-    const YzImgHead &h = *reinterpret_cast<const YzImgHead *>(img);
-    if (lane < 4) S.np[lane] = h.np[lane];
-    if (lane < 8) S.woff[lane] = h.woff[lane];
-    const uint4 *ia = img + YZ_IMG_HEAD_WORDS;
-#pragma unroll 1
-    for (int b0 = 0; b0 < total; b0 += 32) {
-        const int i = b0 + lane;
-        bool a = false;
-        if (i < total) {
-            const float2 ye = *reinterpret_cast<const float2 *>(ia + 2 * i);
-            const uint4 v = ia[2 * i + 1];
-            const float t = ye.y * ye.x;
-            tt[i] = make_float2(t, t * __uint_as_float(v.y));
-            a = v.w != 0u;
+// Code of the scratch entry past the hits of the combination of u2 pair ui
+// and v2 pair vi (info words), in an outer iteration of n3 hits that finds
+// the entries `ent`: the latest attempt at that offset, by this combination,
+// an earlier one of the iteration, or before the iteration.
+__device__ __forceinline__ unsigned yz_stale_code(const YzInner &I, unsigned ui, unsigned vi, int n3,
+                                                  unsigned long long ent) {
+    const int iu = (int)(ui & 127u), gu = (int)(ui >> 7) & 3, iv = (int)(vi & 127u), gv = (int)(vi >> 7) & 3;
+    const int prev = (int)(vi >> 16);
+    if (gv == 3) return 0u;  // v2 and v2' pair with each other
+    const int cu = gu == 3 ? 2 : 1;
+    int off = -1;
+    bool before = false;
+    if (gv == 1 && I.pv[iv].y >= 0) {
+        off = I.ov + I.pv[iv].y;  // its own refused v2' hit
+    } else if (cu == 1 && I.first_two < iu) {
+        return 0u;  // this v2 pair's own hit, tried after two u2 hits
+    } else if (cu == 1 && I.u.two >= 0) {
+        if (iv == 0) {
+            before = true;
+        } else if (I.u.one > I.u.two && prev == iv - 1) {
+            off = I.ov + I.pv[prev].y;
+        } else {
+            const short2 p = I.pv[iv - 1];
+            const bool sec = p.x < 0 || (!yz_img_acc(I.hits, I.ova + p.x) && p.y >= 0);
+            off = sec ? I.ov + p.y : I.ova + p.x;
         }
-        const unsigned m = __ballot_sync(0xffffffffu, a);
-        if (lane == 0) S.acc[b0 >> 5] = m;
+    } else if (prev != 255) {
+        off = I.ov + I.pv[prev].y;
+    } else {
+        before = true;
     }
-    const short2 *ip = reinterpret_cast<const short2 *>(ia + 2 * total);
-    int off = 0;
-#pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
-        const int n = h.np[q];
-#pragma unroll 1
-        for (int i = lane; i < n; i += 32) {
-            const short2 p = ip[off + i];
-            S.pair[q][i] = make_uchar2((unsigned char)(p.x < 0 ? 255 : p.x), (unsigned char)(p.y < 0 ? 255 : p.y));
-        }
-        off += n;
+    if (before) {
+        const int e = n3 + cu + 1 - 4;  // entry 4 + e
+        if (e > 3) return 0u;
+        const unsigned o = (unsigned)(ent >> (16 * e)) & 0xFFFFu;
+        return o == 0xFFFFu ? (YZ_ENT_UNIT << 10) | ((unsigned)e << 12) : o | (YZ_ENT_HIT << 10);
     }
+    return (unsigned)off | (YZ_ENT_HIT << 10);
 }
 
 // The event's prop-tube y planes and, for the tracklet's x fit, which of the
@@ -1797,7 +2024,7 @@ __device__ __forceinline__ bool yz_prop_plane(const YzFirstWarp &S, int q, float
 __device__ __forceinline__ bool yz_first_gates(const YzFirstWarp &S, const YzGate &G, unsigned hasx, bool valid, float y0,
                                                float ty, float ey0, float ety) {
     bool ok = valid && !(fabsf(y0) > Y0_MAX || fabsf(ty) > TY_MAX);
-#pragma unroll
+#pragma unroll 1
     for (int q = 0; q < 3; ++q) {
         bool m = false;
 #pragma unroll
@@ -1812,25 +2039,26 @@ __device__ __forceinline__ bool yz_first_gates(const YzFirstWarp &S, const YzGat
 #pragma unroll 1
     for (int s = 0; s < 2; ++s) {
         if (!__any_sync(0xffffffffu, ok)) return false;
-        const float tol = s ? 10.16f : 5.08f;
-        const bool a = yz_prop_plane(S, 2 * s, ty * G.pz[2 * s] + y0, tol, ok);
-        bool b = false;
-        if (__any_sync(0xffffffffu, ok && !a)) b = yz_prop_plane(S, 2 * s + 1, ty * G.pz[2 * s + 1] + y0, tol, ok && !a);
-        ok = a || b;
+        bool found = false;
+#pragma unroll 1
+        for (int q = 2 * s; q < 2 * s + 2 && __any_sync(0xffffffffu, ok && !found); ++q)
+            found |= yz_prop_plane(S, q, ty * G.pz[q] + y0, s ? 10.16f : 5.08f, ok && !found);
+        ok = found;
     }
     return ok;
 }
 
 // State of the survivors' order from one ring chunk to the next.
 struct YzOrder {
-    int g = -1;         // outer iteration of the last survivor
+    unsigned g = ~0u;   // outer iteration (its pairs) of the last survivor
     bool pend = false;  // its first survivor waits in S.pend
 };
 
 // Up to 32 survivors from the ring, in order: the gates, then those the
-// survivor kernel needs go to Q; returns the new queue length.
-__device__ __forceinline__ int yz_first_pass(YzFirstWarp &S, const YzGate &G, unsigned hasx, int head, int n, int C2,
-                                             const YzTab *__restrict__ tab, YzOrder &od, YzSurv *Q, int qn) {
+// survivor kernel needs go to Q; returns the new queue length.  Out of line:
+// it runs once per 32 survivors.
+__device__ __noinline__ int yz_first_pass(YzFirstWarp &S, const YzGate &G, unsigned hasx, int head, int n,
+                                          const YzTab *__restrict__ tab, YzOrder &od, YzSurv *Q, int qn) {
     const int lane = lane_id();
     const unsigned lt = lanemask_lt();
     const bool valid = lane < n;
@@ -1839,18 +2067,17 @@ __device__ __forceinline__ int yz_first_pass(YzFirstWarp &S, const YzGate &G, un
     float2 er = make_float2(0.f, 0.f);
     if (valid) er = __ldg(reinterpret_cast<const float2 *>(&tab[(v.w >> 14) & 0x7Fu].ey0));
     const bool pass = yz_first_gates(S, G, hasx, valid, y0, ty, er.x, er.y);
-    const int g = valid ? (int)(v.x >> 14) : -2 - lane;
-    const int gp = __shfl_up_sync(0xffffffffu, g, 1);
+    const unsigned g = valid ? v.x & 0x3FFFu : 0x10000u + lane;
+    const unsigned gp = __shfl_up_sync(0xffffffffu, g, 1);
     const bool first = valid && g != (lane == 0 ? od.g : gp);
-    const bool keep = valid && (pass || ((v.w >> 21) & 1u));  // bit 21: may pair planes 19 and 18
+    const bool keep = valid && (pass || ((v.w >> 21) & 1u));
     const unsigned seg = __match_any_sync(0xffffffffu, g);
     const unsigned km = __ballot_sync(0xffffffffu, keep);
     const bool emit = keep || (first && (km & seg) != 0u);
     const unsigned em = __ballot_sync(0xffffffffu, emit);
     auto put = [&](int at, uint4 w, bool gate) {
-        const int gg = (int)(w.x >> 14), rr = (int)(w.x & 0x3FFFu);
-        const uint4 o = make_uint4((unsigned)(gg * C2 + rr), w.y, w.z, (w.w & 0x1FFFFFu) | (gate ? 0x80000000u : 0u));
-        *reinterpret_cast<uint4 *>(Q + at) = o;
+        w.w = (w.w & 0x3FDFFFFFu) | (gate ? 0x80000000u : 0u);
+        *reinterpret_cast<uint4 *>(Q + at) = w;
     };
     // the iteration carried from the last chunk: its first survivor goes
     // before the first one kept here
@@ -1864,7 +2091,7 @@ __device__ __forceinline__ int yz_first_pass(YzFirstWarp &S, const YzGate &G, un
     qn += __popc(em);
     // the chunk's last iteration may go on
     const int last = n - 1;
-    const int gl = __shfl_sync(0xffffffffu, g, last);
+    const unsigned gl = __shfl_sync(0xffffffffu, g, last);
     if (gl != od.g) {
         const unsigned segl = __shfl_sync(0xffffffffu, seg, last);
         od.pend = (km & segl) == 0u;
@@ -1876,100 +2103,25 @@ __device__ __forceinline__ int yz_first_pass(YzFirstWarp &S, const YzGate &G, un
     return qn;
 }
 
-// The first cut of one unit.  `tt` and `R` / `R2` (nf records) are in shared
-// memory or in the warp's overflow arena.  Returns the survivors passed on in
-// Q, or -1 when the queue could overflow (the unit then runs on the combined
-// path); *count = the combinations that passed the cut.
+// The first cut of one unit, ranks [r0, r1) of the tracklet's live outer
+// iterations.  `term` / `info`: the four lists (stride `cap`), of na[q]
+// entries.  Returns the survivors passed on in Q, or -1 when the queue could
+// overflow (the unit then runs on the combined path); *count = the
+// combinations that passed the cut.
 template <bool PRUNE>
-__device__ __forceinline__ int yz_first_walk(YzFirstWarp &S, const YzGate &G, unsigned hasx, const float2 *tt,
-                                             unsigned long long *R, unsigned short *R2, int nf, int r0, int r1,
-                                             bool half_p, const YzTab *__restrict__ tab, YzSurv *Q, int qcap,
+__device__ __forceinline__ int yz_first_walk(YzFirstWarp &S, const YzGate &G, unsigned hasx, const float4 *term,
+                                             const unsigned *info, int cap, const int na[4], const YzInner &I,
+                                             unsigned long long lasto, int r0, int r1, bool half_p,
+                                             const YzTab *__restrict__ tab, YzSurv *Q, int qcap,
                                              const float *__restrict__ osc, float t_keep, int *count) {
     const int lane = lane_id();
     const unsigned lt = lanemask_lt();
-    const int nu2 = S.np[0], nu3 = S.np[2];
-    const int C2 = nu2 * S.np[1];
-    // --- the inner pairs' records ------------------------------------------
-    // the last write of offset m past the station-3 hits over the pairs so
-    // far, 16 bits each (yz_last_writes)
-    unsigned long long lasto = ~0ull;
-    {
-        int at = 0;
-#pragma unroll 1
-        for (int b0 = 0; b0 < C2; b0 += 32) {
-            const int r = b0 + lane;
-            unsigned long long off = 0ull;  // hit e of the pair's accepted ones, or the failed attempt after them
-            unsigned pm = 0u;
-            int nacc = 0, gu = 0, gv = 0;
-            if (r < C2) {
-                const uchar2 pu = S.pair[0][r % nu2], pv = S.pair[1][r / nu2];
-                const int o[4] = {pu.x != 255 ? S.woff[0] + pu.x : -1, pu.y != 255 ? S.woff[1] + pu.y : -1,
-                                  pv.x != 255 ? S.woff[2] + pv.x : -1, pv.y != 255 ? S.woff[3] + pv.y : -1};
-                int g = 0;
-#pragma unroll
-                for (int a = 0; a < 4; ++a) {
-                    if (a == 2 && nacc == 0) break;  // no u2 hit: v2 is not loaded
-                    if (o[a] < 0) continue;
-                    const int sh = 16 * nacc;
-                    off = (off & ~(0xFFFFull << sh)) | ((unsigned long long)o[a] << sh);
-                    pm |= 1u << nacc;
-                    if (yz_acc(S, o[a])) {
-                        g |= 1 << a;
-                        ++nacc;
-                    }
-                }
-                gu = g & 3;
-                gv = g >> 2;
-            }
-            const bool fit = gu != 0 && gv != 0;
-            // the entry past the hit count as this pair leaves it or finds it
-            unsigned stale = 0xFFFFu;
-            unsigned long long nl = lasto;
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const unsigned mine = (unsigned)(off >> (16 * m)) & 0xFFFFu;
-                const unsigned wm = __ballot_sync(0xffffffffu, (pm >> m) & 1u);
-                if (m >= 2) {
-                    const int src = last_lane(wm & lt);
-                    const unsigned before = __shfl_sync(0xffffffffu, mine, src < 0 ? 0 : src);
-                    if (nacc == m) {
-                        if ((pm >> m) & 1u) stale = mine;
-                        else stale = src >= 0 ? before : (unsigned)((lasto >> (16 * m)) & 0xFFFFull);
-                    }
-                }
-                if (wm) {
-                    const unsigned long long w = __shfl_sync(0xffffffffu, mine, last_lane(wm));
-                    nl = (nl & ~(0xFFFFull << (16 * m))) | (w << (16 * m));
-                }
-            }
-            lasto = nl;
-            const unsigned fm = __ballot_sync(0xffffffffu, fit);
-            if (fit) {
-                const int k = at + __popc(fm & lt);
-                unsigned long long rec = 0ull;
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (e < nacc) rec |= ((off >> (16 * e)) & 0x3FFull) << (10 * e);
-                rec |= (unsigned long long)nacc << 40;
-                rec |= (unsigned long long)(gu * 3 - 4 + gv) << 43;
-                if (stale != 0xFFFFu) rec |= ((unsigned long long)stale << 47) | (1ull << 57);
-                if (gu & 1) rec |= 1ull << 58;  // starts with a hit of plane 18
-                R[k] = rec;
-                R2[k] = (unsigned short)r;
-            }
-            at += __popc(fm);
-        }
-    }
-    // --- pairs with an accepted hit ------------------------------------------
-    YzAlive alive;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-        const int i = w * 32 + lane;
-        alive.u[w] = __ballot_sync(0xffffffffu, i < S.np[2] && yz_group(S, 2, S.pair[2][i < S.np[2] ? i : 0]) != 0);
-        alive.v[w] = __ballot_sync(0xffffffffu, i < S.np[3] && yz_group(S, 3, S.pair[3][i < S.np[3] ? i : 0]) != 0);
-    }
-    const int Au = bits128(alive.u);
-    const int sg = 32 / nf, sr = 32 - sg * nf;
+    const int nu2 = na[0], nf = na[0] * na[1], nu3 = na[2];
+    const float4 *tu = term, *tv = term + cap, *tu3 = term + 2 * cap, *tv3 = term + 3 * cap;
+    const unsigned *iu = info, *iv = info + cap, *iu3 = info + 2 * cap, *iv3 = info + 3 * cap;
+    // a chunk's step in the digits (u2, v2, outer)
+    const int s2 = 32 / nf, sr = 32 - s2 * nf, s1 = sr / nu2, s0 = sr - s1 * nu2;
+    const int l2 = lane / nf, lr = lane - l2 * nf, l1 = lr / nu2, l0 = lr - l1 * nu2;
     int qn = 0, nsurv = 0;
     int head = 0, waiting = 0;
     YzOrder od;
@@ -1985,21 +2137,22 @@ __device__ __forceinline__ int yz_first_walk(YzFirstWarp &S, const YzGate &G, un
         unsigned kt = 0u;
         if (in) {
             kept = !(PRUNE && osc) || osc[j] >= t_keep;
-            const int iu = nth_bit128(alive.u, j % Au), iv = nth_bit128(alive.v, j / Au);
-            const uchar2 pu = S.pair[2][iu], pv = S.pair[3][iv];
-            const int gu = yz_group(S, 2, pu), gv = yz_group(S, 3, pv);
+            const int jv = j / nu3, ju = j - jv * nu3;
+            const float4 a = tu3[ju], c = tv3[jv];
+            const unsigned ia = iu3[ju], ic = iv3[jv];
+            const int gu = (int)(ia >> 7) & 3, gv = (int)(ic >> 7) & 3;
+            // the hits in order; a refused one adds 0
+            b0 = a.x;
+            b1 = a.y;
+            b0 += a.z;
+            b1 += a.w;
+            b0 += c.x;
+            b1 += c.y;
+            b0 += c.z;
+            b1 += c.w;
             const int n3 = __popc(gu) + __popc(gv);
-            auto term = [&](int off) {
-                const float2 t = tt[off];
-                b0 += t.x;
-                b1 += t.y;
-            };
-            if (gu & 1) term(S.woff[4] + pu.x);
-            if (gu & 2) term(S.woff[5] + pu.y);
-            if (gv & 1) term(S.woff[6] + pv.x);
-            if (gv & 2) term(S.woff[7] + pv.y);
-            kt = (unsigned)(iu + iv * nu3) | ((unsigned)yz_tab_index(gu, gv, 1, 1) << 14) | ((unsigned)n3 << 21) |
-                 ((half_p && gv == 2) ? 1u << 24 : 0u);
+            kt = (ia & 127u) | (ic & 127u) << 7 | (unsigned)yz_tab_index(gu, gv, 1, 1) << 14 |
+                 (unsigned)(gu | gv << 2) << 21 | (unsigned)n3 << 25;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int mm = k + 4 - n3;
@@ -2021,7 +2174,7 @@ __device__ __forceinline__ int yz_first_walk(YzFirstWarp &S, const YzGate &G, un
             }
         }
         const unsigned km = __ballot_sync(0xffffffffu, kept);
-        __syncwarp();  // every lane is done with the previous list; the records are written
+        __syncwarp();  // every lane is done with the previous list
         if (kept) {
             const int pos = __popc(km & lt);
             S.kb[pos] = make_float2(b0, b1);
@@ -2031,35 +2184,29 @@ __device__ __forceinline__ int yz_first_walk(YzFirstWarp &S, const YzGate &G, un
         __syncwarp();
         // --- their combinations, 32 a chunk ----------------------------------
         const int ctot = __popc(km) * nf;
-        int k = lane / nf, r = lane - k * nf;
+        int d0 = l0, d1 = l1, d2 = l2;
 #pragma unroll 1
         for (int cb = 0; cb < ctot; cb += 32) {
             bool pass = false;
             float y0 = 0.f, ty = 0.f;
-            unsigned t3 = 0u;
-            unsigned long long rec = 0ull;
+            unsigned t3 = 0u, ui = 0u, vi = 0u, ti = 0u;
             if (cb + lane < ctot) {
-                t3 = S.kt[k];
-                const float2 s = S.kb[k];
-                rec = R[r];
-                const int nacc = (int)(rec >> 40) & 7;
-                float2 t = tt[(int)rec & 0x3FF];
-                float f0 = s.x + t.x, f1 = s.y + t.y;
-                t = tt[(int)(rec >> 10) & 0x3FF];
-                f0 += t.x;
-                f1 += t.y;
-                if (nacc > 2) {
-                    t = tt[(int)(rec >> 20) & 0x3FF];
-                    f0 += t.x;
-                    f1 += t.y;
-                }
-                if (nacc > 3) {
-                    t = tt[(int)(rec >> 30) & 0x3FF];
-                    f0 += t.x;
-                    f1 += t.y;
-                }
+                t3 = S.kt[d2];
+                const float2 s = S.kb[d2];
+                ui = iu[d0];
+                vi = iv[d1];
+                const float4 a = tu[d0], c = tv[d1];
+                // the station-2 hits in order; a refused one adds 0
+                float f0 = s.x + a.x, f1 = s.y + a.y;
+                f0 += a.z;
+                f1 += a.w;
+                f0 += c.x;
+                f1 += c.y;
+                f0 += c.z;
+                f1 += c.w;
                 // Fit2::solve with the plane set's tabulated inverse
-                const YzTab *te = tab + ((t3 >> 14) & 0x7Fu) + ((unsigned)(rec >> 43) & 0xFu);
+                ti = ((t3 >> 14) & 0x7Fu) + ((ui >> 7) & 3u) * 3u - 4u + ((vi >> 7) & 3u);
+                const YzTab *te = tab + ti;
                 const float4 ai = __ldg(reinterpret_cast<const float4 *>(te));
                 const float2 thr = __ldg(reinterpret_cast<const float2 *>(&te->thr_y0));
                 y0 = 0.0f;
@@ -2073,38 +2220,34 @@ __device__ __forceinline__ int yz_first_walk(YzFirstWarp &S, const YzGate &G, un
             const unsigned pm = __ballot_sync(0xffffffffu, pass);
             if (pm) {
                 if (pass) {
-                    const int n3 = (int)(t3 >> 21) & 7, nacc = (int)(rec >> 40) & 7;
-                    // the scratch entry past the hit count
-                    unsigned code = ((t3 >> 14) & 0x7Fu) + ((unsigned)(rec >> 43) & 0xFu);
-                    code <<= 14;
-                    const int e = n3 + nacc - 4;  // entry 4 + e
-                    if ((rec >> 57) & 1u) {
-                        code |= ((unsigned)(rec >> 47) & 0x3FFu) | (YZ_ENT_HIT << 10);
-                    } else if (e < 4) {
-                        const unsigned o = (unsigned)(S.kent[k] >> (16 * e)) & 0xFFFFu;
-                        code |= o == 0xFFFFu ? (YZ_ENT_UNIT << 10) | ((unsigned)e << 12) : o | (YZ_ENT_HIT << 10);
-                    }
-                    if (((t3 >> 24) & 1u) && ((rec >> 58) & 1u)) code |= 1u << 21;
+                    const unsigned g3 = (t3 >> 21) & 15u, g2 = ((ui >> 7) & 3u) | ((vi >> 7) & 3u) << 2;
+                    unsigned code = yz_stale_code(I, ui, vi, (int)(t3 >> 25), S.kent[d2]) | ti << 14 | (g3 | g2 << 4) << 22;
+                    // only v3' of the v3 pair, and a hit of plane 18
+                    if (half_p && (g3 >> 2) == 2u && (g2 & 1u)) code |= 1u << 21;
                     S.ring[(head + waiting + __popc(pm & lt)) & 63] =
-                        make_uint4(((t3 & 0x3FFFu) << 14) | R2[r], __float_as_uint(y0), __float_as_uint(ty), code);
+                        make_uint4((t3 & 0x3FFFu) | (ui & 127u) << 14 | (vi & 127u) << 21, __float_as_uint(y0),
+                                   __float_as_uint(ty), code);
                 }
                 waiting += __popc(pm);
                 nsurv += __popc(pm);
                 __syncwarp();
                 if (waiting >= 32) {
-                    qn = yz_first_pass(S, G, hasx, head, 32, C2, tab, od, Q, qn);
+                    qn = yz_first_pass(S, G, hasx, head, 32, tab, od, Q, qn);
                     head = (head + 32) & 63;
                     waiting -= 32;
                     if (qn > qcap - 34) return -1;
                 }
             }
-            r += sr;
-            const int cy = r >= nf;
-            r -= cy ? nf : 0;
-            k += sg + cy;
+            d0 += s0;
+            int cy = d0 >= nu2;
+            d0 -= cy ? nu2 : 0;
+            d1 += s1 + cy;
+            cy = d1 >= na[1];
+            d1 -= cy ? na[1] : 0;
+            d2 += s2 + cy;
         }
     }
-    if (waiting) qn = yz_first_pass(S, G, hasx, head, waiting, C2, tab, od, Q, qn);
+    if (waiting) qn = yz_first_pass(S, G, hasx, head, waiting, tab, od, Q, qn);
     *count = nsurv;
     return qn;
 }
@@ -2219,12 +2362,14 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_PLAN_WARPS_SM / W > 0 ? OR_YZ_P
     const unsigned long long nplan =
         sc.list ? (unsigned long long)sc.counters[6] : (unsigned long long)n_events * per_event;
     unsigned long long *plan_ctr = reinterpret_cast<unsigned long long *>(sc.counters + 4);
+    // the next unit is taken while the current one is worked on
+    unsigned long long nxt = 0;
+    if (lane == 0) nxt = atomicAdd(plan_ctr, 1ull);
     for (;;) {
-        unsigned long long pu = 0;
-        if (lane == 0) pu = atomicAdd(plan_ctr, 1ull);
-        pu = __shfl_sync(0xffffffffu, pu, 0);
-        if (pu >= nplan) break;
-        if (sc.list) pu = sc.list[pu];
+        const unsigned long long pt = __shfl_sync(0xffffffffu, nxt, 0);
+        if (pt >= nplan) break;
+        if (lane == 0) nxt = atomicAdd(plan_ctr, 1ull);
+        const unsigned long long pu = sc.list ? (unsigned long long)sc.list[pt] : pt;
         const long e = (long)(pu / per_event);
         const int slot0 = (int)(pu % per_event) * chunk;
         if (toomany[e]) continue;  // K:873-878
@@ -2244,12 +2389,9 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_PLAN_WARPS_SM / W > 0 ? OR_YZ_P
             const int st3 = 3 + (slot & 1);  // K:884
             YzEvent &E = S.ev;
             __syncwarp();  // every lane is done with the previous slot's views
-            yz_event_planes(E, hv, e, st3);
-            __syncwarp();
+            yz_event_planes(E, hv, e, st3, prune.ofeat == nullptr);
             Stale *st = S.st;
-            __syncwarp();  // every lane is done with the previous slot's states
-#pragma unroll 1
-            for (int k = 0; k < 4; ++k) st[k] = Stale{DET_SENTINEL, 0.f, 0.f};
+            if (lane < 4) st[lane] = Stale{DET_SENTINEL, 0.f, 0.f};
             __syncwarp();
 #pragma unroll 1
             for (int it = 0; it < ntr; ++it) {
@@ -2286,10 +2428,13 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_PLAN_WARPS_SM / W > 0 ? OR_YZ_P
                     n_fitted += f;
                     n_hitsum += h;
                 }
-                yz_xhits(S, T, P);
                 const long C = G * C2;
                 const long Cl = Ga * C2 + G;  // live combinations, plus one step per outer iteration
-                bool inline_it = Cl <= YZ_LIGHT && Cl <= budget;
+                // Light tracklets are evaluated here only with score rows
+                // (which ones have rows follows from it); without, queueing
+                // them too is faster (planning pass of 10,000 one-dimuon
+                // events 729 -> 548 us, both unit kernels 543 -> 580 us).
+                bool inline_it = prune.ofeat && Cl <= YZ_LIGHT && Cl <= budget;
                 if (!inline_it) {
                     // whole outer iterations per unit, about YZ_UNIT live combinations each
                     const long gper = max(1L, min(G, (YZ_UNIT * G) / (Ga * C2)));
@@ -2312,6 +2457,7 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_PLAN_WARPS_SM / W > 0 ? OR_YZ_P
                         // the combination scorer's rows: one per live outer iteration
                         int orow0 = -1;
                         if (prune.ofeat) {
+                            yz_xhits(S, T, P);
                             unsigned r0 = 0u;
                             if (lane == 0) r0 = atomicAdd(prune.orows, (unsigned)Ga);
                             r0 = __shfl_sync(0xffffffffu, r0, 0);
@@ -2346,11 +2492,32 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_PLAN_WARPS_SM / W > 0 ? OR_YZ_P
                             hv2.best_g = -1;
                             sc.heavy[hid] = hv2;
                         }
-                        yz_unit_states(S, base, (int)G, (int)gper, st, sc.units + u0, hid, al.u, al.v);
+                        if (nunits == 1) {
+                            if (lane < 4) sc.units[u0].entry[lane] = st[lane];
+                            if (lane == 4) {
+                                YzUnit &un = sc.units[u0];
+                                un.heavy = hid;
+                                un.g0 = 0;
+                                un.g1 = (int)G;
+                                un.pad = 0;
+                                un.r0 = 0;
+                                un.r1 = (int)Ga;
+                            }
+                            __syncwarp();
+                            // the entries the slot's next tracklet finds
+                            if (it + 1 < ntr) yz_final_state(S, base, st);
+                        } else {
+                            yz_unit_states(S, base, (int)G, (int)gper, st, sc.units + u0, hid, al.u, al.v);
+                        }
                     }
                 }
                 if (inline_it) {
                     budget -= Cl;
+                    yz_xhits(S, T, P);
+                    if (!prune.ofeat) {  // the gates' planes were not loaded
+                        yz_event_planes(E, hv, e, st3);
+                        __syncwarp();
+                    }
                     const unsigned long long bk =
                         yz_range_ool<false>(S, E, base, 0, C, st, P, sc.tab + YZ_TAB_SETS * (st3 - 3), Q, sc.qcap,
                                             nullptr, 0.f);
@@ -2468,21 +2635,23 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_FIRST_WARPS_SM / W > 0 ? OR_YZ_
     YzFirstWarp &S = warps[w];
     const int gw = blockIdx.x * W + w;
     if (gw >= sc.garena_warps) return;  // queues and arenas exist for garena_warps warps
-    unsigned char *garena = reinterpret_cast<unsigned char *>(yz_garena(sc, gw));
+    float4 *garena = reinterpret_cast<float4 *>(yz_garena(sc, gw));
     YzSurv *Q = reinterpret_cast<YzSurv *>(sc.qbuf + (long)gw * sc.qcap);
     const int qcap = sc.qcap * (int)(sizeof(PassEntryStore) / sizeof(YzSurv));
     unsigned long long *pool_ctr = reinterpret_cast<unsigned long long *>(sc.counters + 8);
     const int nunits = min((int)sc.counters[0], sc.cap_units);
     unsigned long long n_surv = 0ull;
+    // the next unit is taken while the current one is worked on
+    int nxt = 0;
+    if (lane == 0) nxt = (int)atomicAdd(&sc.counters[2], 1u);
     for (;;) {
-        int u = 0;
-        if (lane == 0) u = (int)atomicAdd(&sc.counters[2], 1u);
-        u = __shfl_sync(0xffffffffu, u, 0);
+        const int u = __shfl_sync(0xffffffffu, nxt, 0);
         if (u >= nunits) break;
+        if (lane == 0) nxt = (int)atomicAdd(&sc.counters[2], 1u);
         const int heavy = sc.units[u].heavy;
+        const int r0 = sc.units[u].r0, r1 = sc.units[u].r1;
         if (heavy < 0) continue;
         const YzHeavy hv2 = sc.heavy[heavy];
-        const int r0 = sc.units[u].r0, r1 = sc.units[u].r1;
         const int st3 = 3 + (hv2.slot & 1);
         const YzTab *tab = sc.tab + YZ_TAB_SETS * (st3 - 3);
         int ns = -1, count = 0;  // -1: the unit runs on the combined path (survivor kernel)
@@ -2491,30 +2660,70 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_FIRST_WARPS_SM / W > 0 ? OR_YZ_
             const uint4 *img = sc.img + hv2.img;
             const YzImgHead &h = *reinterpret_cast<const YzImgHead *>(img);
             const int total = h.total;
-            float2 *tt = total <= YZ_TT_SMEM ? S.tt : reinterpret_cast<float2 *>(garena);
-            yz_first_load(S, img, tt, total);
+            if (lane < 4) S.np[lane] = h.np[lane];
+            if (lane < 8) S.woff[lane] = h.woff[lane];
             const unsigned hasx = yz_first_event(S, hv, hv2.e, G, gplane, h.x0, h.tx, h.ex0, h.etx);
             __syncwarp();
-            // inner pairs that reach the fit
-            int nu = 0, nv = 0;
-#pragma unroll 1
-            for (int i = lane; i < S.np[0]; i += 32) nu += yz_group(S, 0, S.pair[0][i]) != 0;
-#pragma unroll 1
-            for (int i = lane; i < S.np[1]; i += 32) nv += yz_group(S, 1, S.pair[1][i]) != 0;
-            const int nf = __reduce_add_sync(0xffffffffu, nu) * __reduce_add_sync(0xffffffffu, nv);
-            const float *osc = PRUNE ? yz_tracklet_scores(prune, hv2) : nullptr;
             // a station without a hodoscope hit in the x window closes the
             // gates for every combination
-            if (nf == 0 || !(hasx & 3u) || !(hasx & 12u) || !(hasx & 48u)) {
-                ns = sc.count_work && nf ? -1 : 0;
-            } else if (nf <= YZ_FIT_SMEM && total <= YZ_TT_SMEM) {
-                ns = yz_first_walk<PRUNE>(S, G, hasx, S.tt, S.rec, S.r2, nf, r0, r1, st3 == 3, tab, Q, qcap, osc,
-                                          prune.t_keep, &count);
-            } else if (nf <= YZ_FIT_MAX) {
-                ns = yz_first_walk<PRUNE>(S, G, hasx, tt,
-                                          reinterpret_cast<unsigned long long *>(garena + YZ_TT_ARENA_BYTES),
-                                          reinterpret_cast<unsigned short *>(Q + qcap - YZ_R2_ENTRIES), nf, r0, r1,
-                                          st3 == 3, tab, Q, qcap - YZ_R2_ENTRIES, osc, prune.t_keep, &count);
+            const bool closed = !(hasx & 3u) || !(hasx & 12u) || !(hasx & 48u);
+            if (closed && !sc.count_work) {
+                ns = 0;
+            } else if (!closed) {
+                YzInner I;
+                I.hits = img + YZ_IMG_HEAD_WORDS;
+                const short2 *pair = reinterpret_cast<const short2 *>(I.hits + 2 * total);
+                int most = 0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) most = max(most, S.np[q]);
+                const bool small = most <= YZ_LIST_SMEM;
+                const int cap = small ? YZ_LIST_SMEM : YZ_MAXPAIR;
+                float4 *term = small ? &S.term[0][0] : garena;
+                unsigned *info = small ? &S.info[0][0] : reinterpret_cast<unsigned *>(garena + 4 * YZ_MAXPAIR);
+                int na[4];
+                YzLast last;
+                int first_two;
+                const short2 *pq = pair;
+#pragma unroll 1
+                for (int q = 0; q < 4; ++q) {
+                    const int n = yz_first_list(S, q, pq, I.hits, term + q * cap, info + q * cap, last, first_two);
+                    if (q == 0) {
+                        na[0] = n;
+                        I.pu = pq;
+                        I.u = last;
+                        I.first_two = first_two;
+                    } else if (q == 1) {
+                        na[1] = n;
+                        I.pv = pq;
+                        I.v = last;
+                    } else if (q == 2) {
+                        na[2] = n;
+                    } else {
+                        na[3] = n;
+                    }
+                    pq += S.np[q];
+                }
+                I.ou = S.woff[1];
+                I.ov = S.woff[3];
+                I.ova = S.woff[2];
+                __syncwarp();
+                auto second = [&](int q, int i) {
+                    return (unsigned)(q == 0 ? I.ou + I.pu[i].y : I.ov + I.pv[i].y);
+                };
+                auto rel0 = [&](int q, int i) {
+                    const short2 p = q == 0 ? I.pu[i] : I.pv[i];
+                    const int oa = q == 0 ? S.woff[0] : I.ova, ob = q == 0 ? I.ou : I.ov;
+                    const bool sec = p.x < 0 || (!yz_img_acc(I.hits, oa + p.x) && p.y >= 0);
+                    return (unsigned)(sec ? ob + p.y : oa + p.x);
+                };
+                if (na[0] * na[1] == 0) {
+                    ns = 0;
+                } else {
+                    const unsigned long long lasto = yz_lasto(S.np[0], S.np[1], I.u, I.v, second, rel0);
+                    const float *osc = PRUNE ? yz_tracklet_scores(prune, hv2) : nullptr;
+                    ns = yz_first_walk<PRUNE>(S, G, hasx, term, info, cap, na, I, lasto, r0, r1, st3 == 3, tab, Q, qcap,
+                                              osc, prune.t_keep, &count);
+                }
             }
         }
         __syncwarp();
