@@ -30,7 +30,8 @@ cudaError_t launch_histograms(or_tracks_view_t, or_dimuons_view_t, const int32_t
                               int, cudaStream_t, int);
 cudaError_t launch_back_clean(or_tracks_view_t, const uint8_t *, int, cudaStream_t, int, int);
 cudaError_t launch_global(const or_plane_t *, or_hits_view_t, or_tracks_view_t, const uint8_t *, int, uint32_t *,
-                          unsigned long long *, cudaStream_t, int, int);
+                          unsigned long long *, int, cudaStream_t, int, int);
+size_t global_sched_bytes(int);
 cudaError_t launch_pack(const or_hit_record_t *, const int64_t *, int, const float *, const or_rt_table_t *,
                         or_hits_view_t, uint32_t *, cudaStream_t, int);
 cudaError_t launch_wait_selftest(uint32_t *, uint32_t, cudaStream_t);
@@ -72,7 +73,8 @@ struct or_ctx {
     or_plane_t *d_plane;
     bool has_geom;
     uint32_t *d_errw;
-    unsigned long long *d_sched;  // work-unit counters of the dynamically scheduled kernels
+    unsigned long long *d_sched;  // global tracking's work-unit counters and slot list
+    int sched_slots;              // ... and how many slots the list holds
     // YZ work queue: units of heavy tracklets, their best records, overflow arenas
     void *yz_scratch;
     int yz_cap_units, yz_cap_heavy, yz_garena_warps;
@@ -164,6 +166,11 @@ static void yz_caps(int max_events, int &units, int &heavy) {
     }
 }
 
+// slots of the largest batch, for global tracking's list
+static int sched_slots(int max_events) {
+    return OR_NSLOTS * (max_events <= 0 || max_events >= 100000 ? 100000 : max_events);
+}
+
 // per-warp arenas and queues for the most warps a YZ kernel launches
 static int yz_arena_warps(int sm_count) { return sm_count * (OR_YZ_SPLIT ? OR_YZ_FIRST_WARPS_SM : OR_YZ_WARPS_SM); }
 
@@ -171,7 +178,7 @@ size_t or_context_bytes(int max_events, int sm_count) {
     if (max_events < 0 || sm_count <= 0) return 0;
     int units, heavy;
     yz_caps(max_events, units, heavy);
-    return sizeof(or_plane_t) + sizeof(uint32_t) + 256 +
+    return sizeof(or_plane_t) + sizeof(uint32_t) + orgpu::global_sched_bytes(sched_slots(max_events)) +
            orgpu::yz_scratch_bytes_ctx(units, heavy, yz_arena_warps(sm_count));
 }
 
@@ -204,7 +211,8 @@ int or_create_sized(int device, int max_events, or_ctx_t **out) {
         delete c;
         return fail(OR_ERR_NOMEM, "cudaMalloc error word");
     }
-    if ((e = cudaMalloc(&c->d_sched, 256)) != cudaSuccess) {
+    c->sched_slots = sched_slots(max_events);
+    if ((e = cudaMalloc(&c->d_sched, orgpu::global_sched_bytes(c->sched_slots))) != cudaSuccess) {
         cudaFree(c->d_plane);
         cudaFree(c->d_errw);
         delete c;
@@ -438,8 +446,8 @@ int or_global(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, const
     if (n_events < 0 || !toomany) return fail(OR_ERR_ARG, "bad event count or flag array");
     if ((rc = check_hits(hits)) || (rc = check_tracks(tracks))) return rc;
     cudaError_t e =
-        orgpu::launch_global(ctx->d_plane, hits, tracks, toomany, n_events, ctx->d_errw, ctx->d_sched, S(stream),
-                             ctx->sm_count, ctx->warps[OR_K_GLOBAL]);
+        orgpu::launch_global(ctx->d_plane, hits, tracks, toomany, n_events, ctx->d_errw, ctx->d_sched,
+                             ctx->sched_slots, S(stream), ctx->sm_count, ctx->warps[OR_K_GLOBAL]);
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "global tracking launch");
 }
 
@@ -900,7 +908,7 @@ extern "C" int or_gKernel_Global_tracking(gEventHitCollections *hitcolls, gEvent
                                                or_hits_view_from_collection(hitcolls),
                                                or_tracks_view_from_collection(tklcoll),
                                                reinterpret_cast<const uint8_t *>(hastoomanyhits), OR_REF_EVTMAX,
-                                               ctx->d_errw, ctx->d_sched, nullptr, ctx->sm_count,
+                                               ctx->d_errw, ctx->d_sched, ctx->sched_slots, nullptr, ctx->sm_count,
                                                ctx->warps[OR_K_GLOBAL]);
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "or_gKernel_Global_tracking launch");
 }
