@@ -10,17 +10,40 @@
 // slot) into shared memory with 1-D TMA bulk copies completing on an
 // mbarrier; planes are taken in batches that fit the warp's buffer (a warp
 // prefix sum over the planes' sizes), each lane issuing the copies of its
-// planes.  Each lane then runs the reference's per-plane state machine on one
-// plane out of shared memory and writes that plane's survivors back, with the
-// new SoA stride, into the same slot.  Bytes beyond the survivors are left as
-// they were, as the reference leaves them.
+// planes.  The hits of a batch are then one index space, 32 at a time,
+// whatever planes they belong to:
+//   - the reference's cluster state after an in-time hit is "closed" when
+//     the hit lies more than one channel from the one before and the run of
+//     such hits has an odd length (a hit that closes a cluster does not start
+//     the next one, so in a run every second hit opens one), else "open":
+//     the run's length is a ballot and a carry;
+//   - a hit that closes a cluster, or ends its plane inside one, walks back
+//     to the cluster's first hit and applies the 2-hit or the n-hit rule;
+//   - the first survivor of a channel is the first lane of its
+//     __match_any_sync group whose bit in the plane's map is not set yet.
+// Survivors are written back with the new SoA stride into the same slot,
+// consecutive lanes to consecutive words; a plane that keeps all its hits is
+// not written.  Bytes beyond the survivors are left as they were, as the
+// reference leaves them.
+//
+// Bound: instruction issue and shared-memory latency.  One lane per plane
+// running the state machine hit by hit, and writing its plane alone, left
+// most lanes idle, above all in events of many hits, whose batches hold few
+// planes: 2.82 ms for 100,000 uneven events, 972 us for 20,000 of high
+// occupancy, 245 us for 333 uneven ones; this takes 1.60 ms, 566 us and
+// 144 us.
 #include "or_device.cuh"
 
 namespace orgpu {
 
-constexpr int ER_BUF_FLOATS = 2048;                 // 8 KB staging buffer per warp
+// Staging buffer per warp: the smallest that holds a full chamber plane.  More
+// batches per event, but more warps per SM (100,000 uneven events 1.60 ms; 1.88
+// at 6 KB, 2.01 at 8 KB).
+constexpr int ER_BUF_FLOATS = 1024;
 constexpr int ER_MAX_STAGED_HITS = ER_BUF_FLOATS / 5 + 8;
-constexpr int ER_NPLANES = 48;
+constexpr int ER_FIRST_WORDS = (ER_MAX_STAGED_HITS + 31) / 32;
+constexpr int ER_NPLANES = 48, ER_NCHAMBERS = 24;
+static_assert(ER_BUF_FLOATS >= 5 * OR_MAXHITS_CHAM + 3, "a full plane fits the buffer");
 constexpr uint32_t ER_WAIT_LIMIT = 1u << 26;        // bounded mbarrier wait
 constexpr uint32_t ER_DRAIN_LIMIT = 1u << 28;       // ... and the wait for copies in flight after it gave up
 
@@ -35,12 +58,19 @@ struct __align__(16) ErWarp {
     uint64_t bar;
     int n[ER_NPLANES];
     int kept[ER_NPLANES];
-    int soff[ER_NPLANES];
-    int hoff[ER_NPLANES];
+    int soff[ER_NPLANES];   // start of each plane's image in buf
+    int hoff[ER_NPLANES];   // hits of the batch before each plane
+    uint16_t list[ER_MAX_STAGED_HITS];  // chamber hits in time, then the survivors: index in the batch
+    uint8_t plane[ER_MAX_STAGED_HITS];  // plane of each hit of the batch
     uint8_t keep[ER_MAX_STAGED_HITS];
-    uint16_t surv[ER_MAX_STAGED_HITS];
-    uint32_t seen[32][8];  // per-lane channel bitmap, 202 channels
+    uint8_t state[ER_MAX_STAGED_HITS];  // of list entries: ER_FIRST, ER_FAR, ER_CLOSED
+    uint32_t seen[ER_NPLANES][7];       // channels 0..201 of each plane's survivors
+    uint32_t first[ER_FIRST_WORDS];     // bit per hit of the batch: the first of its plane
+    float *slot[ER_NPLANES];
+    uint8_t occupied[ER_NPLANES];       // the batch's planes with hits
 };
+constexpr uint8_t ER_FIRST = 1, ER_FAR = 2, ER_CLOSED = 4;
+static_assert(7 * 32 >= 202, "channel bits");
 
 struct PlaneRef {
     float *slot;
@@ -68,94 +98,148 @@ __device__ __forceinline__ PlaneRef er_plane(const or_hits_view_t &hv, long e, i
     return r;
 }
 
-// event_reduction() on one staged plane (reconstruction_helper.cuh:168-361).
-// Returns the survivor count; keep[] gets 1/0 per hit, surv[] the survivor
-// indices in order.
-static __device__ int er_reduce_plane(const float *h, int n, int det, uint8_t *keep, uint16_t *surv, uint32_t *seen) {
-    auto chan = [&](int i) { return h[i]; };
+// The rules for a cluster of `cls` >= 2 in-time hits list[s..t] of one plane
+// (reference H:267-318); h = the plane's image, n its hits, first the batch
+// index of its first hit.
+static __device__ __forceinline__ void er_cluster(ErWarp &S, int s, int t, const float *h, int n, int first, int det) {
     auto pos = [&](int i) { return h[n + i]; };
     auto tdc = [&](int i) { return h[2 * n + i]; };
-    auto intime = [&](int i) { return (((int)h[3 * n + i]) & 2) != 0; };
     auto drift = [&](int i) { return h[4 * n + i]; };
-
-    int cl_first = 0, cl_last = 0, cls = 0;
-    for (int i = 0; i < n; ++i) {
-        keep[i] = 1;
-        if (!intime(i)) {  // H:198
-            keep[i] = 0;
-            continue;
-        }
-        // H:204-230 never changes a flag: uniqueID_curr is reset every hit.
-        if (det > OR_NCHAM) continue;
-        if (cls == 0) {  // H:241-243
-            cl_first = cl_last = i;
-            cls = 1;
-            continue;
-        }
-        const float dc = fabsf(chan(i) - chan(cl_last));
-        if (dc > 1 || i == n - 1) {  // H:258
-            if (i == n - 1 && dc <= 1) {
-                cl_last = i;
-                ++cls;
-            }
-            if (cls == 2) {  // H:267-295
-                const int a = cl_first, b = cl_last;
-                const float w_max = (float)(0.9 * 0.5 * (double)(pos(b) - pos(a)));
-                const float w_min = (float)(4.0 / 9.0 * (double)w_max);
-                if ((drift(a) > w_max && drift(b) > w_min) || (drift(a) > w_min && drift(b) > w_max)) {
-                    if (drift(a) > drift(b))
-                        keep[a] = 0;
-                    else
-                        keep[b] = 0;
-                } else {
-                    const float dt = tdc(a) - tdc(b);
-                    if ((((double)dt >= 0.0 && (double)dt < 8.0) || ((double)dt <= 0.0 && (double)dt > -8.0)) &&
-                        (det >= 19 && det <= 24)) {
-                        keep[a] = 0;
-                        keep[b] = 0;
-                    }
-                }
-            }
-            if (cls >= 3) {  // H:297-318: members are the in-time hits in [first, last]
-                float dt_mean = 0.0f;
-                int prev = cl_first;
-                for (int m = cl_first + 1; m <= cl_last; ++m) {
-                    if (!intime(m)) continue;
-                    const float d = tdc(m) - tdc(prev);
-                    dt_mean += ((double)d > 0.0 ? d : (tdc(prev) - tdc(m)));
-                    prev = m;
-                }
-                dt_mean = dt_mean / (float)(cls - 1);
-                const bool all = (double)dt_mean < 10.0;
-                for (int m = cl_first; m <= cl_last; ++m) {
-                    if (!intime(m)) continue;
-                    if (all || m != cl_first) keep[m] = 0;
-                }
-            }
-            cls = 0;
+    const int cls = t - s + 1;
+    const int a = S.list[s] - first, b = S.list[t] - first;
+    if (cls == 2) {  // H:267-295
+        const float w_max = (float)(0.9 * 0.5 * (double)(pos(b) - pos(a)));
+        const float w_min = (float)(4.0 / 9.0 * (double)w_max);
+        if ((drift(a) > w_max && drift(b) > w_min) || (drift(a) > w_min && drift(b) > w_max)) {
+            S.keep[first + (drift(a) > drift(b) ? a : b)] = 0;
         } else {
-            cl_last = i;
-            ++cls;
-        }
-    }
-    // H:334-349, first survivor per channel wins
-#pragma unroll
-    for (int w = 0; w < 8; ++w) seen[w] = 0u;
-    int nred = 0;
-    for (int i = 0; i < n; ++i) {
-        if (!keep[i]) continue;
-        const int c = (short)chan(i);
-        if (c >= 0 && c < 202) {
-            const uint32_t bit = 1u << (c & 31);
-            if (seen[c >> 5] & bit) {
-                keep[i] = 0;
-                continue;
+            const float dt = tdc(a) - tdc(b);
+            if ((((double)dt >= 0.0 && (double)dt < 8.0) || ((double)dt <= 0.0 && (double)dt > -8.0)) &&
+                (det >= 19 && det <= 24)) {
+                S.keep[first + a] = 0;
+                S.keep[first + b] = 0;
             }
-            seen[c >> 5] |= bit;
         }
-        surv[nred++] = (uint16_t)i;
+    } else if (cls >= 3) {  // H:297-318
+        float dt_mean = 0.0f;
+        int prev = a;
+        for (int k = s + 1; k <= t; ++k) {
+            const int m = S.list[k] - first;
+            const float d = tdc(m) - tdc(prev);
+            dt_mean += ((double)d > 0.0 ? d : (tdc(prev) - tdc(m)));
+            prev = m;
+        }
+        dt_mean = dt_mean / (float)(cls - 1);
+        const bool all = (double)dt_mean < 10.0;
+        for (int k = all ? s : s + 1; k <= t; ++k) S.keep[S.list[k]] = 0;
     }
-    return nred;
+}
+
+// event_reduction() (reconstruction_helper.cuh:168-361) on the staged planes
+// [p0, p1) of `hits` hits: S.kept and, per plane in order, the survivors'
+// batch indices in S.list.  The after-pulse branch (H:204-230) never changes a
+// flag: uniqueID_curr is reset every hit.
+static __device__ __forceinline__ void er_reduce(ErWarp &S, int p0, int p1, int hits) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = lanemask_lt();
+    for (int i = p0 * 7 + lane; i < p1 * 7; i += 32) S.seen[0][i] = 0u;
+    for (int i = lane; i < ER_FIRST_WORDS; i += 32) S.first[i] = 0u;
+    __syncwarp();
+    int nocc = 0;
+    for (int q0 = p0; q0 < p1; q0 += 32) {
+        const int p = q0 + lane;
+        const bool occ = p < p1 && S.n[p] > 0;
+        const unsigned m = __ballot_sync(0xffffffffu, occ);
+        if (p < p1) S.kept[p] = 0;
+        if (occ) {
+            S.occupied[nocc + __popc(m & lt)] = (uint8_t)p;
+            atomicOr(&S.first[S.hoff[p] >> 5], 1u << (S.hoff[p] & 31));
+        }
+        nocc += __popc(m);
+    }
+    __syncwarp();
+    // in-time hits; those of chambers are listed
+    int nlist = 0, started = 0;
+#pragma unroll 1
+    for (int b0 = 0; b0 < hits; b0 += 32) {
+        const int f = b0 + lane;
+        bool cham = false;
+        if (f < hits) {
+            // its plane: as many occupied planes start at or before it
+            const int p = S.occupied[started + __popc(S.first[b0 >> 5] & (lt | (1u << lane))) - 1];
+            const int n = S.n[p], i = f - S.hoff[p];
+            const bool intime = (((int)S.buf[S.soff[p] + 3 * n + i]) & 2) != 0;  // H:198
+            S.plane[f] = (uint8_t)p;
+            S.keep[f] = intime;
+            cham = intime && p < ER_NCHAMBERS;
+        }
+        started += __popc(S.first[b0 >> 5]);
+        const unsigned m = __ballot_sync(0xffffffffu, cham);
+        if (cham) S.list[nlist + __popc(m & lt)] = (uint16_t)f;
+        nlist += __popc(m);
+    }
+    __syncwarp();
+    // cluster state after each listed hit (H:241-258)
+    int run = 0;  // hits far from the one before, up to the last chunk's end
+#pragma unroll 1
+    for (int b0 = 0; b0 < nlist; b0 += 32) {
+        const int k = b0 + lane;
+        uint8_t st = ER_FIRST;
+        if (k < nlist && k > 0) {
+            const int f = S.list[k], g = S.list[k - 1], p = S.plane[f];
+            if (S.plane[g] == p) {
+                const float *h = S.buf + S.soff[p] - S.hoff[p];
+                st = fabsf(h[f] - h[g]) > 1 ? ER_FAR : 0;
+            }
+        }
+        const unsigned near = __ballot_sync(0xffffffffu, st != ER_FAR);
+        const int l = last_lane(near & (lt | (1u << lane)));
+        const int r = l >= 0 ? lane - l : run + lane + 1;
+        if ((st & ER_FAR) && (r & 1)) st |= ER_CLOSED;
+        if (k < nlist) S.state[k] = st;
+        run = __shfl_sync(0xffffffffu, r, 31);
+    }
+    __syncwarp();
+    // clusters, each at the hit that ends it
+#pragma unroll 1
+    for (int k = lane; k < nlist; k += 32) {
+        const uint8_t st = S.state[k];
+        const int f = S.list[k], p = S.plane[f], n = S.n[p], first = S.hoff[p];
+        int t = -1;
+        if (st & ER_CLOSED) t = k - 1;
+        else if (st == 0 && f - first == n - 1 && !(S.state[k - 1] & ER_CLOSED)) t = k;  // H:258, the plane's last hit
+        if (t < 0) continue;
+        int s = t;
+        while (!(S.state[s] & ER_FIRST) && !(S.state[s - 1] & ER_CLOSED)) --s;
+        if (t > s) er_cluster(S, s, t, S.buf + S.soff[p], n, first, c_er_det[p]);
+    }
+    __syncwarp();
+    // H:334-349, first survivor per channel wins
+    int ns = 0;
+#pragma unroll 1
+    for (int b0 = 0; b0 < hits; b0 += 32) {
+        const int f = b0 + lane;
+        bool k = f < hits && S.keep[f];
+        int p = 0, c = -1;
+        if (k) {
+            p = S.plane[f];
+            c = (short)S.buf[S.soff[p] + f - S.hoff[p]];
+            if (c < 0 || c >= 202) c = -1;
+        }
+        const unsigned peers = __match_any_sync(0xffffffffu, c >= 0 ? p * 256 + c : -1 - lane);
+        if (k && c >= 0) {
+            k = (peers & lt) == 0u && !((S.seen[p][c >> 5] >> (c & 31)) & 1u);
+        }
+        __syncwarp();
+        if (k) {
+            if (c >= 0) atomicOr(&S.seen[p][c >> 5], 1u << (c & 31));
+            atomicAdd(&S.kept[p], 1);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, k);
+        if (k) S.list[ns + __popc(m & lt)] = (uint16_t)f;
+        ns += __popc(m);
+        __syncwarp();
+    }
 }
 
 template <int W>
@@ -175,6 +259,7 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
             const PlaneRef r = er_plane(hv, e, c_er_det[p]);
             const int n = (int)*r.count;
             S.n[p] = n < r.cap ? n : r.cap;
+            S.slot[p] = r.slot;
         }
         __syncwarp();
         int p0 = 0;
@@ -219,8 +304,7 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
                 for (int p = p0 + lane; p < p1; p += 32) {
                     const int sz = (5 * S.n[p] + 3) & ~3;
                     if (sz == 0) continue;
-                    const PlaneRef r = er_plane(hv, e, c_er_det[p]);
-                    tma_load_1d(S.buf + S.soff[p], r.slot, (uint32_t)sz * 4u, &S.bar);
+                    tma_load_1d(S.buf + S.soff[p], S.slot[p], (uint32_t)sz * 4u, &S.bar);
                 }
                 if (!__all_sync(0xffffffffu, mbar_wait_bounded(&S.bar, phase, ER_WAIT_LIMIT))) {
                     // the wait gave up: raise the error word, then wait (again
@@ -233,33 +317,52 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
                 }
                 phase ^= 1u;
             }
-            for (int p = p0 + lane; p < p1; p += 32) {
-                S.kept[p] = er_reduce_plane(S.buf + S.soff[p], S.n[p], c_er_det[p], S.keep + S.hoff[p],
-                                            S.surv + S.hoff[p], S.seen[lane]);
-            }
-            __syncwarp();
-            // each lane writes back the planes it reduced
-            for (int p = p0 + lane; p < p1; p += 32) {
-                const int n = S.n[p], nk = S.kept[p];
-                const PlaneRef r = er_plane(hv, e, c_er_det[p]);
-                const float *src = S.buf + S.soff[p];
-                const uint16_t *sv = S.surv + S.hoff[p];
-                for (int f = 0; f < 5; ++f)
-                    for (int k = 0; k < nk; ++k) r.slot[f * nk + k] = src[f * n + sv[k]];
-                *r.count = (uint32_t)nk;
+            er_reduce(S, p0, p1, hits);
+            // write back the planes that lost hits: the survivors of plane p
+            // are list entries [at, at + kept)
+            int at = 0;
+#pragma unroll 1
+            for (int q0 = p0; q0 < p1; q0 += 32) {
+                const int p = q0 + lane;
+                const int nk = p < p1 ? S.kept[p] : 0;
+                int incl = nk;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, incl, d);
+                    if (lane >= d) incl += v;
+                }
+                const int start = at + incl - nk;
+                const bool less = p < p1 && nk < S.n[p];
+                if (p < p1) *er_plane(hv, e, c_er_det[p]).count = (uint32_t)nk;
+                for (unsigned m = __ballot_sync(0xffffffffu, less); m; m &= m - 1) {
+                    const int l = __ffs(m) - 1, q = q0 + l;
+                    const int k = __shfl_sync(0xffffffffu, nk, l), s0 = __shfl_sync(0xffffffffu, start, l);
+                    const int n = S.n[q];
+                    const float *src = S.buf + S.soff[q] - S.hoff[q];
+                    float *dst = S.slot[q];
+#pragma unroll 1
+                    for (int i = lane; i < k; i += 32) {
+                        const float *h = src + S.list[s0 + i];
+#pragma unroll
+                        for (int f = 0; f < 5; ++f) dst[f * k + i] = h[f * n];
+                    }
+                }
+                at += __shfl_sync(0xffffffffu, incl, 31);
             }
             __syncwarp();
             p0 = p1;
         }
-        // K:128-139: station sums of the reduced chamber counts
-        if (lane == 0) {
-            int m[4] = {0, 0, 0, 0};
-            for (int p = 0; p < 24; ++p) {
-                const int d = c_er_det[p];
-                const int st = d <= 12 ? 0 : (d - 7) / 6;
-                m[st] += S.kept[p];
-            }
-            toomany[e] = (uint8_t)((m[0] > MAXD0) || (m[1] > MAXD2) || (m[2] > MAXD3) || (m[3] > MAXD3));
+        // K:128-139: station sums of the reduced chamber counts, planes 0-5,
+        // 6-11, 12-17 and 18-23 of the list
+        {
+            const int lim = lane < 6 ? MAXD0 : lane < 12 ? MAXD2 : MAXD3;
+            int m = lane < ER_NCHAMBERS ? S.kept[lane] : 0;
+            const int st = lane / 6;
+            int sum = 0;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) sum += __shfl_sync(0xffffffffu, m, min(31, st * 6 + k));
+            const bool over = __any_sync(0xffffffffu, lane < ER_NCHAMBERS && sum > lim);
+            if (lane == 0) toomany[e] = (uint8_t)over;
         }
         __syncwarp();
     }
