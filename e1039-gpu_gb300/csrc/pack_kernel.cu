@@ -10,8 +10,15 @@
 // slot).  An event whose records are out of that order raises ERRW_INPUT
 // (or_stream_sync reports it as an argument error); its slots are then
 // undefined but every write stays inside them.  Records whose det is outside
-// 1..54 (they sort first or last) are skipped.  One warp per event: a shared-memory histogram per plane, an
-// exclusive scan, then coalesced field writes.
+// 1..54 (they sort first or last) are skipped.  One warp per event: the planes'
+// runs are where the det changes from one record to the next, then the field
+// writes, 128 records in flight in both passes.
+//
+// Bound: DRAM latency and the 200-byte pieces that an event's planes are
+// written in.  A histogram by shared-memory atomics (all lanes on one counter
+// where records are sorted), a scan by one lane and one record in flight per
+// lane took 685 us for 100,000 uneven events and, with the R-T spline, 166 us
+// for 16,001; this takes 580 and 141 us (two chunks in flight: 647 and 164).
 //
 // With an R-T table the drift field is computed from the tdc as the
 // reference host does while packing (online_reconstruction.cu:387-396); the
@@ -21,6 +28,8 @@
 namespace orgpu {
 
 constexpr int PK_WARPS = 8;
+constexpr int PK_AHEAD = 4;  // chunks of 32 records in flight per warp
+constexpr int PK_BLOCKS = 4; // per SM: 64 registers
 
 // Drift distance of a hit on plane det from the R-T calibration, or `drift`
 // unchanged when the plane has no profile (hodoscopes never have one).
@@ -60,80 +69,112 @@ static __device__ __forceinline__ bool rt_plane(int det) {
 }
 
 template <bool RT>
-__global__ void __launch_bounds__(PK_WARPS * 32)
+__global__ void __launch_bounds__(PK_WARPS * 32, PK_BLOCKS)
     pack_kernel(const or_hit_record_t *__restrict__ rec, const int64_t *__restrict__ off, int n_events,
                 const float *__restrict__ wire_pos_f, const or_rt_table_t *__restrict__ rt, or_hits_view_t hv,
                 uint32_t *__restrict__ errw) {
-    __shared__ int cnt[PK_WARPS][64];
-    __shared__ int start[PK_WARPS][64];
+    // first record of each plane, and the one after its last
+    __shared__ int first[PK_WARPS][64];
+    __shared__ int past[PK_WARPS][64];
     const int w = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     for (long e = (long)blockIdx.x * PK_WARPS + w; e < n_events; e += (long)gridDim.x * PK_WARPS) {
         const int64_t r0 = off[e], r1 = off[e + 1];
         const int nrec = (int)(r1 - r0);
-        cnt[w][lane] = 0;
-        cnt[w][lane + 32] = 0;
+        const or_hit_record_t *R = rec + r0;
+        first[w][lane] = past[w][lane] = 0;
+        first[w][lane + 32] = past[w][lane + 32] = 0;
         __syncwarp();
-        for (int r = lane; r < nrec; r += 32) {
-            const int d = rec[r0 + r].det;
-            if (d >= 1 && d < OR_NDET) atomicAdd(&cnt[w][d], 1);
-        }
-        __syncwarp();
-        // records are sorted by det: plane d's run starts at the sum of the
-        // counts of the planes before it (records with det out of range sort
-        // first or last and are skipped)
-        if (lane == 0) {
-            int lead = 0;
-            for (int r = 0; r < nrec && rec[r0 + r].det < 1; ++r) ++lead;
-            int s = lead;
-            for (int d = 1; d < OR_NDET; ++d) {
-                start[w][d] = s;
-                s += cnt[w][d];
+        // Records are sorted by det: a plane's run starts where det changes.
+        // Records with det out of range sort first or last and are skipped.
+        int carry = -0x10000;  // det of the record before the chunk
+#pragma unroll 1
+        for (int b0 = 0; b0 < nrec; b0 += 32 * PK_AHEAD) {
+            int d[PK_AHEAD];
+#pragma unroll
+            for (int i = 0; i < PK_AHEAD; ++i) {
+                const int r = b0 + 32 * i + lane;
+                d[i] = r < nrec ? (int)R[r].det : 0x10000;
+            }
+#pragma unroll
+            for (int i = 0; i < PK_AHEAD; ++i) {
+                const int r = b0 + 32 * i + lane;
+                int prev = __shfl_up_sync(0xffffffffu, d[i], 1);
+                if (lane == 0) prev = carry;
+                carry = __shfl_sync(0xffffffffu, d[i], 31);
+                if (d[i] != prev) {
+                    if (d[i] >= 1 && d[i] < OR_NDET) first[w][d[i]] = r;
+                    if (prev >= 1 && prev < OR_NDET) past[w][prev] = r;
+                }
             }
         }
+        if (lane == 0 && carry >= 1 && carry < OR_NDET) past[w][carry] = nrec;
         __syncwarp();
-        // counts (capped) for all 54 planes
+        // counts (capped) for all 54 planes; `past` is the count from here on
         for (int d = 1 + lane; d < OR_NDET; d += 32) {
-            const int n = cnt[w][d];
-            if (d <= OR_NCHAM)
-                hv.nhits_cham[e * OR_NCHAM + d - 1] = (uint32_t)min(n, OR_MAXHITS_CHAM);
-            else if (d <= OR_NCHAM + OR_NHODO)
-                hv.nhits_hodo[e * OR_NHODO + d - OR_NCHAM - 1] = (uint32_t)min(n, OR_MAXHITS_HODO);
-            else
-                hv.nhits_prop[e * OR_NPROP + d - OR_NCHAM - OR_NHODO - 1] = (uint32_t)min(n, OR_MAXHITS_PROP);
+            const int cap = d <= OR_NCHAM ? OR_MAXHITS_CHAM : d <= OR_NCHAM + OR_NHODO ? OR_MAXHITS_HODO : OR_MAXHITS_PROP;
+            const int n = max(0, min(past[w][d] - first[w][d], cap));
+            past[w][d] = n;
+            if (d <= OR_NCHAM) hv.nhits_cham[e * OR_NCHAM + d - 1] = (uint32_t)n;
+            else if (d <= OR_NCHAM + OR_NHODO) hv.nhits_hodo[e * OR_NHODO + d - OR_NCHAM - 1] = (uint32_t)n;
+            else hv.nhits_prop[e * OR_NPROP + d - OR_NCHAM - OR_NHODO - 1] = (uint32_t)n;
         }
+        __syncwarp();
         bool unsorted = false;
-        for (int r = lane; r < nrec; r += 32) {
-            const or_hit_record_t h = rec[r0 + r];
-            if (r > 0) {
-                const or_hit_record_t q = rec[r0 + r - 1];
-                unsorted |= h.det < q.det || (h.det == q.det && (h.elem < q.elem || (h.elem == q.elem && h.tdc < q.tdc)));
+        int cd = -0x10000, ce = 0;  // the record before the chunk: det, elem, tdc
+        float ct = 0.f;
+#pragma unroll 1
+        for (int b0 = 0; b0 < nrec; b0 += 32 * PK_AHEAD) {
+            or_hit_record_t h[PK_AHEAD];
+            float pos[PK_AHEAD];
+#pragma unroll
+            for (int i = 0; i < PK_AHEAD; ++i) {
+                const int r = b0 + 32 * i + lane;
+                h[i].det = (int16_t)0x7FFF;
+                h[i].elem = 0;
+                if (r < nrec) h[i] = R[r];
             }
-            const int d = h.det;
-            if (d < 1 || d >= OR_NDET) continue;
-            const int k = r - start[w][d];
-            float *slot;
-            int cap;
-            if (d <= OR_NCHAM) {
-                slot = hv.hits_cham + e * OR_EVT_CHAM_FLOATS + (long)OR_NHITSPARAM * OR_MAXHITS_CHAM * (d - 1);
-                cap = OR_MAXHITS_CHAM;
-            } else if (d <= OR_NCHAM + OR_NHODO) {
-                slot = hv.hits_hodo + e * OR_EVT_HODO_FLOATS + (long)OR_NHITSPARAM * OR_MAXHITS_HODO * (d - OR_NCHAM - 1);
-                cap = OR_MAXHITS_HODO;
-            } else {
-                slot = hv.hits_prop + e * OR_EVT_PROP_FLOATS +
-                       (long)OR_NHITSPARAM * OR_MAXHITS_PROP * (d - OR_NCHAM - OR_NHODO - 1);
-                cap = OR_MAXHITS_PROP;
+#pragma unroll
+            for (int i = 0; i < PK_AHEAD; ++i) {
+                const int d = h[i].det, el = h[i].elem;
+                const bool in = d >= 1 && d < OR_NDET && el >= 0 && el < OR_WIREPOS_STRIDE;
+                pos[i] = in ? __ldg(wire_pos_f + d * OR_WIREPOS_STRIDE + el) : 0.f;
             }
-            const int n = min(cnt[w][d], cap);
-            if (k < 0 || k >= n) continue;  // k < 0 only for records out of order
-            const int el = h.elem;
-            const float pos = (el >= 0 && el < OR_WIREPOS_STRIDE) ? wire_pos_f[d * OR_WIREPOS_STRIDE + el] : 0.f;
-            slot[k] = (float)el;
-            slot[n + k] = pos;
-            slot[2 * n + k] = h.tdc;
-            slot[3 * n + k] = (float)h.flag;
-            slot[4 * n + k] = (RT && rt_plane(d)) ? rt_drift(rt, d, h.tdc, h.drift) : h.drift;
+#pragma unroll
+            for (int i = 0; i < PK_AHEAD; ++i) {
+                const int r = b0 + 32 * i + lane;
+                const int d = h[i].det, el = h[i].elem;
+                const float tdc = h[i].tdc;
+                int pd = __shfl_up_sync(0xffffffffu, d, 1), pe = __shfl_up_sync(0xffffffffu, el, 1);
+                float pt = __shfl_up_sync(0xffffffffu, tdc, 1);
+                if (lane == 0) {
+                    pd = cd;
+                    pe = ce;
+                    pt = ct;
+                }
+                cd = __shfl_sync(0xffffffffu, d, 31);
+                ce = __shfl_sync(0xffffffffu, el, 31);
+                ct = __shfl_sync(0xffffffffu, tdc, 31);
+                if (r >= nrec) continue;
+                unsorted |= d < pd || (d == pd && (el < pe || (el == pe && tdc < pt)));
+                if (d < 1 || d >= OR_NDET) continue;
+                const int k = r - first[w][d], n = past[w][d];
+                if (k < 0 || k >= n) continue;  // beyond the slot, or out of order
+                float *slot;
+                if (d <= OR_NCHAM)
+                    slot = hv.hits_cham + e * OR_EVT_CHAM_FLOATS + (long)OR_NHITSPARAM * OR_MAXHITS_CHAM * (d - 1);
+                else if (d <= OR_NCHAM + OR_NHODO)
+                    slot = hv.hits_hodo + e * OR_EVT_HODO_FLOATS +
+                           (long)OR_NHITSPARAM * OR_MAXHITS_HODO * (d - OR_NCHAM - 1);
+                else
+                    slot = hv.hits_prop + e * OR_EVT_PROP_FLOATS +
+                           (long)OR_NHITSPARAM * OR_MAXHITS_PROP * (d - OR_NCHAM - OR_NHODO - 1);
+                slot[k] = (float)el;
+                slot[n + k] = pos[i];
+                slot[2 * n + k] = tdc;
+                slot[3 * n + k] = (float)h[i].flag;
+                slot[4 * n + k] = (RT && rt_plane(d)) ? rt_drift(rt, d, tdc, h[i].drift) : h[i].drift;
+            }
         }
         if (__any_sync(0xffffffffu, unsorted) && lane == 0) atomicOr(errw, ERRW_INPUT);
         __syncwarp();
