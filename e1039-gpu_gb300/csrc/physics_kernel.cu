@@ -12,7 +12,7 @@
 //    the point of closest approach to the beam line: stationID 7, vertex
 //    position and momentum.  The reference gives a thread to each slot, so a
 //    warp works for the one or two lanes whose slot holds a global track;
-//    here a warp gathers the global tracks of 32 events into a shared list
+//    here a warp gathers the global tracks of some events into a shared list
 //    and swims them one per lane, which keeps the lanes of the double-
 //    precision loop busy (FP64 is the scarce unit of this GPU).  The swim is
 //    not stored: the closest-approach scan visits the points in step order
@@ -22,8 +22,8 @@
 //    order by its own lane, as the reference's pair loop carries state from
 //    one pair to the next (the swum momenta of the current track stay in
 //    p_pos / p_neg).
-//  - Histograms: one warp per event, lanes over the bins of one (trigger,
-//    variable) table; counts go in with atomics, so the result is the exact
+//  - Histograms: one warp per event, lanes over the (trigger, variable)
+//    tables, each searched by halves; counts go in with atomics, so the result is the exact
 //    count whatever the order (the reference's plain "+=" from concurrent
 //    blocks loses updates).
 //
@@ -83,12 +83,262 @@ __device__ __forceinline__ double dedx_poly(double p) {
 }
 
 // ---------------------------------------------------------------------------
+// float results of double expressions
+
+// A value as an unevaluated sum of two floats, |l| <= ulp(h) / 2, to some 44
+// bits: the statements of a step that the reference evaluates in double and
+// stores in a float are evaluated this way first (error-free sums and
+// products: T. J. Dekker, Numer. Math. 18, 1971; D. E. Knuth, TAOCP vol. 2,
+// 4.2.2), and in double only where that leaves the float's rounding open.  The
+// results are the same bits; the FP64 pipe takes 64 cycles per warp
+// instruction (measured, whatever the active lanes), so a step's 60 of them
+// were all its time.
+struct FF {
+    float h, l;
+};
+__device__ __forceinline__ FF ff_sum(float a, float b) {  // |a|, |b| in any order
+    const float s = a + b, t = s - a;
+    return FF{s, (a - (s - t)) + (b - t)};
+}
+__device__ __forceinline__ FF ff_fast(float a, float b) {  // |a| >= |b|
+    const float s = a + b;
+    return FF{s, b - (s - a)};
+}
+__device__ __forceinline__ FF ff_mul(FF a, float b) {
+    const float p = a.h * b;
+    return ff_fast(p, __fmaf_rn(a.h, b, -p) + a.l * b);
+}
+__device__ __forceinline__ FF ff_add(FF a, FF b) {
+    const FF s = ff_sum(a.h, b.h);
+    return ff_fast(s.h, s.l + (a.l + b.l));
+}
+__host__ __device__ constexpr FF ff_const(double c) { return FF{(float)c, (float)(c - (double)(float)c)}; }
+
+// Whether v.h is the float nearest to every number within 2^-37 |v.h| of the
+// sum: the rest must stay clear of half the last place by that much (and of a
+// quarter below a power of two).
+__device__ __forceinline__ bool ff_sure(FF v) {
+    const unsigned u = __float_as_uint(v.h) & 0x7fffffffu;
+    const unsigned e = u & 0x7f800000u;
+    const float half = __uint_as_float(e - (24u << 23)) * ((u & 0x7fffffu) ? 1.f - 0x1p-11f : 0.5f - 0x1p-11f);
+    return (e - (40u << 23) <= (210u << 23)) & (fabsf(v.l) < half);
+}
+
+// ---------------------------------------------------------------------------
 // vertexing (K:2594-2803)
 
 #ifndef OR_VTX_GROUP
 #define OR_VTX_GROUP 16
 #endif
 
+// The z of every step: the same subtractions for every track.
+struct VtxZ {
+    double z[phys::NSTEPS_FMAG + phys::NSTEPS_TARGET + 1];
+    int first_half, second_half;  // steps whose first (second) half ends above the hole's length
+};
+constexpr VtxZ vtx_z() {
+    using namespace phys;
+    VtxZ o{};
+    double z = FMAG_LENGTH;
+    o.z[0] = z;
+    for (int k = 1; k <= NSTEPS_FMAG; ++k) {
+        const double b = z - STEP_FMAG;
+        z = b - STEP_FMAG;
+        o.z[k] = z;
+        if (b > FMAG_HOLE_LENGTH) o.first_half = k;
+        if (z > FMAG_HOLE_LENGTH) o.second_half = k;
+    }
+    for (int k = NSTEPS_FMAG + 1; k <= NSTEPS_FMAG + NSTEPS_TARGET; ++k) {
+        z = z - STEP_TARGET;
+        o.z[k] = z;
+    }
+    return o;
+}
+__device__ __constant__ VtxZ c_vtx = vtx_z();
+constexpr int VTX_FIRST = vtx_z().first_half, VTX_SECOND = vtx_z().second_half;
+
+// The helpers below work on the bits of doubles with integer and float
+// instructions, without branches; each clears `ok` outside the range it is
+// exact for, and its caller then evaluates the double expression.
+
+// The double expressions are calls, so that they are not evaluated beside the
+// others (inlined, the compiler did: a step's three square roots took 900
+// cycles each instead of 300).
+__device__ __noinline__ double slow_sqrt(double s) { return sqrt(s); }
+__device__ __noinline__ double slow_div(double m, double p) { return m / p; }
+__device__ __noinline__ double slow_loss(double ptot, float len) { return ptot + dedx_poly(ptot) * len; }
+__device__ __noinline__ float slow_length(double t, double c1, double c2) { return t * t + c1 + c2; }
+__device__ __noinline__ bool slow_closer(float away, double mx, double px, double py, double bx, double by, bool first) {
+    using namespace phys;
+    const double dca2 = (px - X_BEAM) * (px - X_BEAM) + (py - Y_BEAM) * (py - Y_BEAM);
+    const double dca2_min = first ? 1.e18 : (bx - X_BEAM) * (bx - X_BEAM) + (by - Y_BEAM) * (by - Y_BEAM);
+    return !(away * mx < 0.) && dca2 < dca2_min;
+}
+
+// whether the exponent field of a double lies in [lo, hi)
+__device__ __forceinline__ bool dbl_range(int hi_word, int lo, int hi) {
+    return (unsigned)(((hi_word >> 20) & 0x7FF) - lo) < (unsigned)(hi - lo);
+}
+__device__ __forceinline__ bool dbl_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+// a double's leading bits as a float (error below 2^-23)
+__device__ __forceinline__ float dbl_lead(double x, bool &ok) {
+    const int hi = __double2hiint(x);
+    ok &= dbl_range(hi, 896 + 10, 896 + 245);
+    // the exponent's low nine bits lead; 0x380 less (modulo 2^9) is the float's
+    const unsigned m = __funnelshift_l((unsigned)__double2loint(x), (unsigned)hi, 3) + 0x40000000u;
+    return __int_as_float((hi & 0x80000000) | (int)(m & 0x7FFFFFFFu));
+}
+// a double as two floats, to 46 bits
+__device__ __forceinline__ FF dbl_ff(double x, bool &ok) {
+    const int hi = __double2hiint(x);
+    const unsigned lo = (unsigned)__double2loint(x);
+    ok &= dbl_range(hi, 896 + 60, 896 + 245);
+    const float h = dbl_lead(x, ok);
+    // 23 of the 29 bits left, as the fraction of h's last place
+    const int u = (__float_as_int(h) & 0xFF800000) - (23 << 23);
+    return FF{h, __int_as_float(u | (int)((lo >> 6) & 0x7FFFFF)) - __int_as_float(u)};
+}
+// a float as a double (normal numbers)
+__device__ __forceinline__ double flt_dbl(float x) {
+    const int u = __float_as_int(x), e = (u >> 23) & 0xFF;
+    if (e == 0 || e == 255) return (double)x;
+    return __hiloint2double((u & 0x80000000) | ((u & 0x7FFFFFFF) >> 3) + 0x38000000, u << 29);
+}
+// x plus k units of its last place
+__device__ __forceinline__ double dbl_ulps(double x, int k) {
+    return __longlong_as_double(__double_as_longlong(x) + k);
+}
+// whether no power of two is within 2048 units of x
+__device__ __forceinline__ bool dbl_inside(double x) {
+    return (((unsigned long long)__double_as_longlong(x) + 2048) & 0xFFFFFFFFFFFFFull) >= 4096;
+}
+// the nearest integer, |x| < 2^22
+__device__ __forceinline__ int flt_round(float x) { return __float_as_int(x + 0x1.8p23f) - 0x4B400000; }
+
+// m / p for m = the rounded product q * p: the quotient is q or a neighbour,
+// decided by the product's rounding error, one FMA (P. Markstein, IA-64 and
+// Elementary Functions, 2000, ch. 8: the remainder of an approximate quotient
+// is exact).
+__device__ __forceinline__ double vtx_ratio(double m, double p, double q, bool &sure) {
+    const double r = __fma_rn(-q, p, m);
+    const int hq = __double2hiint(q);
+    bool ok = dbl_inside(q) & dbl_range(hq, 896 + 30, 896 + 200);
+    const float pf = dbl_lead(p, ok);
+    ok &= (pf > 0x1p-20f) & (pf < 0x1p20f);
+    const bool exact = ok & dbl_zero(r);
+    const float rf = dbl_lead(r, ok);
+    // half a unit of q's last place, times p; scaled by 2^60 with r
+    const int e = (hq >> 20) & 0x7FF;
+    const float half = pf * __int_as_float((e - 896 - 53 + 60) << 23);
+    const float rs = fabsf(rf) * 0x1p60f;
+    ok &= (rs < half * (1.f - 0x1p-16f)) | (rs > half * (1.f + 0x1p-16f));
+    const int k = (rs < half) | exact ? 0 : ((__float_as_int(rf) ^ hq) < 0 ? -1 : 1);
+    sure = ok | exact;
+    return dbl_ulps(q, k);
+}
+
+// h + c (|c| some 2^-22 of h) as a double; `scale` becomes one over a unit of
+// its last place
+__device__ __forceinline__ double dbl_join(float h, float c, float &scale, bool &ok) {
+    const int u = __float_as_int(h), e = u & 0x7F800000;
+    ok &= (unsigned)(e - ((127 - 40) << 23)) < (80u << 23);
+    scale = __int_as_float(((52 + 127 + 127) << 23) - e);
+    const float ks = (u < 0 ? -c : c) * (0x1p-9f * scale);  // in units of 2^9
+    const float k1 = (ks + 0x1.8p23f) - 0x1.8p23f;
+    const int lo = flt_round((ks - k1) * 0x1p9f);
+    const double x = __hiloint2double((u & 0x80000000) | ((u & 0x7FFFFFFF) >> 3) + 0x38000000, u << 29);
+    const double g = __longlong_as_double(__double_as_longlong(x) + (long long)flt_round(ks) * 512 + lo);
+    ok &= dbl_inside(g) & (((__double2hiint(g) ^ __double2hiint(x)) & 0x7FF00000) == 0) & (fabsf(ks) < 0x1p22f);
+    return g;
+}
+// moves g by x units of its last place, x known to 2^-9, rounded to whole
+// units; `ok` is cleared when the rounding is not sure
+__device__ __forceinline__ double dbl_settle(double g, float x, bool &ok) {
+    const float k = (x + 0x1.8p23f) - 0x1.8p23f;
+    ok &= (fabsf(x) < 1024.f) & (fabsf(x - k) < 0.498f);
+    return dbl_ulps(g, flt_round(x));
+}
+
+// sqrt(s): two floats' worth of it, then one FMA gives what is left, exactly
+// enough to round.  y is 1 / sqrt(s) to a float.
+__device__ __forceinline__ double vtx_sqrt(double s, float &y, bool &sure) {
+    bool ok = true;
+    const FF a = dbl_ff(s, ok);
+    y = rsqrtf(a.h);
+    const float h = a.h * y, c = (__fmaf_rn(-h, h, a.h) + a.l) * (0.5f * y);
+    float scale;
+    const double g = dbl_join(h, c, scale, ok);
+    const double d = __fma_rn(-g, g, s);
+    const bool exact = ok & dbl_zero(d);
+    const double r = dbl_settle(g, dbl_lead(d, ok) * (0.5f * y) * scale, ok);
+    sure = ok | exact;
+    return exact ? g : r;
+}
+
+// m / p, y being 1 / p to a float, the same way
+__device__ __forceinline__ double vtx_div(double m, double p, float y, bool &sure) {
+    bool ok = y > 0.f;
+    const FF a = dbl_ff(m, ok), b = dbl_ff(p, ok);
+    const float h = a.h * y, c = (__fmaf_rn(-h, b.h, a.h) + (a.l - h * b.l)) * y;
+    float scale;
+    const double q = dbl_join(h, c, scale, ok);
+    const double d = __fma_rn(-q, p, m);
+    const bool exact = ok & dbl_zero(d);
+    const float x = dbl_lead(d, ok) * y * scale;
+    const double r = dbl_settle(q, h < 0.f ? -x : x, ok);
+    sure = ok | exact;
+    return exact ? q : r;
+}
+
+// (float)(t * t + c), c = the other two squares' sum
+__device__ __forceinline__ float vtx_length(double t, FF c, bool &sure) {
+    bool ok = true;
+    const FF a = dbl_ff(t, ok);
+    const float p = a.h * a.h;
+    const FF v = ff_add(ff_fast(p, __fmaf_rn(a.h, a.h, -p) + 2.f * a.h * a.l), c);
+    sure = ok & ff_sure(v);
+    return v.h;
+}
+
+// ptot + dedx_poly(ptot) * len.  For 4 <= ptot < 128 the loss is formed in
+// fixed point (Horner in units of 2^-67) and added to ptot's significand with
+// ten more bits; the double expression's own rounding errors come to at most
+// `margin` of those units (a bound over each binade: j roundings in the
+// power j, one in each of the four sums, one in the product by len < 3, plus
+// two units for the truncations here), so the sum decides the result unless it is that close to
+// the middle of two doubles (some 2 % of the tracks' steps).
+__host__ __device__ constexpr long long loss_coef(double c) { return (long long)(c * 0x1p67); }
+__device__ __forceinline__ double vtx_loss(double ptot, float len, bool &sure) {
+    using namespace phys;
+    const long long bits = __double_as_longlong(ptot);
+    const int k = (int)(bits >> 52) - 1023, ul = __float_as_int(len);
+    const unsigned long long m = (bits & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+    const long long x = (long long)(m << ((k + 4) & 15));  // ptot / 128 in units of 2^-63
+    long long a = loss_coef(DEDX_UNIT_4 * 0x1p28);
+    a = __mul64hi(a, x) * 2 + loss_coef(DEDX_UNIT_3 * 0x1p21);
+    a = __mul64hi(a, x) * 2 + loss_coef(DEDX_UNIT_2 * 0x1p14);
+    a = __mul64hi(a, x) * 2 + loss_coef(DEDX_UNIT_1 * 0x1p7);
+    a = __mul64hi(a, x) * 2 + loss_coef(DEDX_UNIT_0);
+    const long long v = __mul64hi(a, (long long)((ul & 0x7FFFFF) | 0x800000) << 39);  // units of 2^-64
+    const unsigned long long w = (m << 10) + (unsigned long long)(v >> ((k + 2) & 15));
+    const unsigned long long r = (w + 512) >> 10;
+    // the error bound of the double expression: 30, 17, 10, 7, 9 units for k = 2 .. 6
+    const int margin = max(10, 136 >> (k & 7));
+    sure = ((unsigned)(k - 2) <= 4u) & (ul >= 0x40000000) & (ul < 0x40400000) & ((r >> 52) == 1) &
+           (abs((int)(w & 1023) - 512) > margin);
+    return __longlong_as_double((bits & 0x7FF0000000000000ll) | (long long)(r & 0xFFFFFFFFFFFFFull));
+}
+
+// The swim of one track.  An FP64 instruction takes a warp 64 cycles of its
+// quarter of the SM, whatever its active lanes (measured), so what need not be
+// FP64 to give the same bits is not: the z of a step is a constant, its hole
+// test too; roots and quotients are two floats' worth refined by one FMA; the
+// slope of a step is the quotient of a product by its factor; path lengths are
+// floats; the energy loss is formed in fixed point; and a point is compared
+// with the closest so far by leading bits.  Each of these knows when it cannot
+// decide the last bit, and the double expression does then.  Some 25 FP64
+// instructions a magnet step remain of 147, 2 of 9 a target step.  Bound: the
+// chain of one step into the next, some 4,000 cycles.
 __device__ void vertex_track(float *T, const float *z) {
     using namespace phys;
     const float x0 = T[OR_TRK_X0], y0 = T[OR_TRK_Y0], tx = T[OR_TRK_TX], ty = T[OR_TRK_TY];
@@ -100,71 +350,117 @@ __device__ void vertex_track(float *T, const float *z) {
     const double s0 = charge * invP * sqrtf((1.f + tx_st1 * tx_st1) / (1.f + tx_st1 * tx_st1 + ty * ty));
     const double s1 = tx_st1, s2 = ty;
     const double s3 = (float)z_0 * tx_st1 + x0_st1, s4 = (float)z_0 * ty + y0;
-    double px = s3 + s1 * (FMAG_LENGTH - z_0), py = s4 + s2 * (FMAG_LENGTH - z_0), pz = FMAG_LENGTH;
+    double px = s3 + s1 * (FMAG_LENGTH - z_0), py = s4 + s2 * (FMAG_LENGTH - z_0);
     const double pz_0 = 1.f / (fabs(s0) * sqrtf(1.f + s1 * s1 + s2 * s2));
     double mx = pz_0 * s1, my = pz_0 * s2, mz = pz_0;
-    double dca2_min = 1.e18;
-    bool found = false;
-    double v[6];
-    auto visit = [&]() {
-        if (!(FMAGSTR * charge * mx < 0.)) {
-            const double dca2 = (px - X_BEAM) * (px - X_BEAM) + (py - Y_BEAM) * (py - Y_BEAM);
-            if (dca2 < dca2_min) {
-                dca2_min = dca2;
-                found = true;
-                v[0] = px; v[1] = py; v[2] = pz;
-                v[3] = mx; v[4] = my; v[5] = mz;
-            }
+    // the closest point: its place, momentum and step; step -1: none yet
+    double bx = 0., by = 0., bmx = 0., bmy = 0., bmz = 0.;
+    float best = 1.e18f;  // leading bits of its squared distance; NaN: not known
+    int bstep = -1;
+    const float away = FMAGSTR * charge;
+    const bool away_ok = (fabsf(away) > 0x1p-100f) & (fabsf(away) < 0x1p100f);
+    static_assert(X_BEAM == 0.f && Y_BEAM == 0.f, "the leading bits are those of the distance");
+    auto visit = [&](int step) {
+        // FMAGSTR * charge * mx < 0, by signs where the product cannot vanish
+        const int hm = __double2hiint(mx);
+        const bool out = (hm ^ __float_as_int(away)) < 0;
+        bool ok = true;
+        const float fx = dbl_lead(px, ok), fy = dbl_lead(py, ok);
+        const float d = fx * fx + fy * fy;
+        ok &= (d > 1e-20f) & (d < 1e30f);
+        const bool nearer = d < best * (1.f - 0x1p-16f), farther = d > best * (1.f + 0x1p-16f);
+        bool take = !out & nearer;
+        if (!(away_ok & dbl_range(hm, 100, 0x7FF) & (out | (ok & (nearer | farther)))))
+            take = slow_closer(away, mx, px, py, bx, by, bstep < 0);
+        if (take) {
+            best = ok ? d : __int_as_float(0x7FFFFFFF);
+            bstep = step;
+            bx = px; by = py;
+            bmx = mx; bmy = my; bmz = mz;
         }
     };
-    visit();
+    visit(0);
+    const double kick = 2.f * charge * PTKICK_UNIT * STEP_FMAG;
+    const double t1 = ty * STEP_FMAG, t11 = t1 * t1, t12 = STEP_FMAG * STEP_FMAG;
+    const double csum = t11 + t12, tyy = ty * ty;
+    const FF c = FF{(float)csum, (float)(csum - (double)(float)csum)};
+    double slope = s1;  // mx = mz * slope, rounded
+#pragma unroll 1
     for (int step = 1; step <= NSTEPS_FMAG; ++step) {
-        const double tx_i = mx / mz;
-        const double tx_f = tx_i + 2.f * charge * PTKICK_UNIT * STEP_FMAG / sqrt(mx * mx + mz * mz);
-        const double t10 = tx_i * STEP_FMAG, t11 = ty * STEP_FMAG, t12 = STEP_FMAG;
-        const double b0 = px - t10, b1 = py - t11, b2 = pz - t12;
-        const double ptot_i = sqrt(mx * mx + my * my + mz * mz);
-        double ptot_b = ptot_i;
-        if (b2 > FMAG_HOLE_LENGTH || b0 * b0 + b1 * b1 > FMAG_HOLE_RADIUS)
-            ptot_b += dedx_poly(ptot_i) * sqrtf(t10 * t10 + t11 * t11 + t12 * t12);
-        const double t20 = tx_f * STEP_FMAG, t21 = ty * STEP_FMAG, t22 = STEP_FMAG;
+        // what depends on the same values side by side, then one branch for
+        // the lanes that need the double expressions
+        const double mxx = mx * mx, mzz = mz * mz, sxz = mxx + mzz, sxyz = mxx + my * my + mzz;
+        float y_xz, y_p, y_n;
+        bool ok1, ok2, ok3, ok4;
+        double tx_i = vtx_ratio(mx, mz, slope, ok1);
+        double pxz = vtx_sqrt(sxz, y_xz, ok2), ptot_i = vtx_sqrt(sxyz, y_p, ok3);
+        if (!(ok1 & ok2 & ok3)) {
+            if (!ok1) tx_i = slow_div(mx, mz);
+            if (!ok2) pxz = slow_sqrt(sxz);
+            if (!ok3) ptot_i = slow_sqrt(sxyz);
+        }
+        double turn = vtx_div(kick, pxz, y_xz, ok1);
+        const double t10 = tx_i * STEP_FMAG, b0 = px - t10, b1 = py - t1;
+        float q1 = vtx_length(t10, c, ok2);
+        if (!(ok1 & ok2)) {
+            if (!ok1) turn = slow_div(kick, pxz);
+            if (!ok2) q1 = slow_length(t10, t11, t12);
+        }
+        const double tx_f = tx_i + turn, t20 = tx_f * STEP_FMAG, snorm = 1.f + tx_f * tx_f + tyy;
+        double norm = vtx_sqrt(snorm, y_n, ok1);
+        float q2 = vtx_length(t20, c, ok2);
+        const float len1 = sqrtf(q1);
+        double ptot_b = vtx_loss(ptot_i, len1, ok3);
+        const bool in1 = step <= VTX_FIRST || b0 * b0 + b1 * b1 > FMAG_HOLE_RADIUS;
+        if (!(ok1 & ok2 & (ok3 | !in1))) {
+            if (!ok1) norm = slow_sqrt(snorm);
+            if (!ok2) q2 = slow_length(t20, t11, t12);
+            if (!ok3) ptot_b = slow_loss(ptot_i, len1);
+        }
+        if (!in1) ptot_b = ptot_i;
         px = b0 - t20;
-        py = b1 - t21;
-        pz = b2 - t22;
-        double ptot_f = ptot_b;
-        if (pz > FMAG_HOLE_LENGTH || px * px + py * py > FMAG_HOLE_RADIUS)
-            ptot_f += dedx_poly(ptot_b) * sqrtf(t20 * t20 + t21 * t21 + t22 * t22);
-        const double pz_f = ptot_f / sqrt(1.f + tx_f * tx_f + ty * ty);
+        py = b1 - t1;
+        const float len2 = sqrtf(q2);
+        double ptot_f = vtx_loss(ptot_b, len2, ok4);
+        const bool in2 = step <= VTX_SECOND || px * px + py * py > FMAG_HOLE_RADIUS;
+        if (!ok4 & in2) ptot_f = slow_loss(ptot_b, len2);
+        if (!in2) ptot_f = ptot_b;
+        double pz_f = vtx_div(ptot_f, norm, y_n, ok1);
+        if (!ok1) pz_f = slow_div(ptot_f, norm);
         mx = pz_f * tx_f;
         my = pz_f * ty;
         mz = pz_f;
-        visit();
+        slope = tx_f;
+        visit(step);
     }
-    for (int step = NSTEPS_FMAG + 1; step <= NSTEPS_FMAG + NSTEPS_TARGET; ++step) {
-        const double tx_i = mx / mz;
-        px = px - tx_i * STEP_TARGET;
-        py = py - ty * STEP_TARGET;
-        pz = pz - STEP_TARGET;
-        visit();
+    {
+        const double dx = mx / mz * STEP_TARGET, dy = ty * STEP_TARGET;
+#pragma unroll 1
+        for (int step = NSTEPS_FMAG + 1; step <= NSTEPS_FMAG + NSTEPS_TARGET; ++step) {
+            px = px - dx;
+            py = py - dy;
+            visit(step);
+        }
     }
-    if (!found) {  // the last point (K:2752)
-        v[0] = px; v[1] = py; v[2] = pz;
-        v[3] = mx; v[4] = my; v[5] = mz;
+    if (bstep < 0) {  // the last point (K:2752)
+        bstep = NSTEPS_FMAG + NSTEPS_TARGET;
+        bx = px; by = py;
+        bmx = mx; bmy = my; bmz = mz;
     }
     T[OR_TRK_STID] = 7.f;  // K:2796
-    T[OR_TRK_VX] = (float)v[0];
-    T[OR_TRK_VX + 1] = (float)v[1];
-    T[OR_TRK_VX + 2] = (float)v[2];
-    T[OR_TRK_PX] = (float)v[3];
-    T[OR_TRK_PX + 1] = (float)v[4];
-    T[OR_TRK_PX + 2] = (float)v[5];
+    T[OR_TRK_VX] = (float)bx;
+    T[OR_TRK_VX + 1] = (float)by;
+    T[OR_TRK_VX + 2] = (float)c_vtx.z[bstep];
+    T[OR_TRK_PX] = (float)bmx;
+    T[OR_TRK_PX + 1] = (float)bmy;
+    T[OR_TRK_PX + 2] = (float)bmz;
 }
 
 // One warp per block, so that the warps spread over the SMs before they
 // share one: the swim is bound by the FP64 pipes, one to each quarter of an
-// SM (a warp's swim takes some 460 us of one, whatever its lanes), and
+// SM (a warp's swim takes some 240 us of one, whatever its lanes), and
 // blocks of four warps left half of the SMs idle (10,000 events: 1,016 us;
-// now 652 us, 2,000 events 1,012 -> 463 us).  A warp gathers the
+// now 332 us, 2,000 events 1,012 -> 244 us).  A warp gathers the
 // tracks (stationID >= 6) of `group` events, lane = slot, into a shared list
 // and swims them one per lane.
 __global__ void __launch_bounds__(32)
@@ -263,40 +559,85 @@ constexpr float HOLE_LENGTH_F = 0x1.bf0a3cp+4f, HOLE_RADIUS_F = 0x1.451eb8p+0f;
 static_assert((double)HOLE_LENGTH_F <= phys::FMAG_HOLE_LENGTH && (double)0x1.bf0a3ep+4f > phys::FMAG_HOLE_LENGTH, "");
 static_assert((double)HOLE_RADIUS_F <= phys::FMAG_HOLE_RADIUS && (double)0x1.451ebap+0f > phys::FMAG_HOLE_RADIUS, "");
 
-// one FMag step (H:1290-1333); d1 = the linear energy-loss coefficient of the
-// first update, DEDX_UNIT_2 for the reference's second track (H:1354)
-__device__ __forceinline__ void dim_fmag_step(SwimPt &s, float charge, float ty, double d1) {
+// p(ptot) of the energy loss (dedx_poly with the linear coefficient d1)
+__device__ __forceinline__ FF ff_dedx(float p, FF d1) {
     using namespace phys;
+    constexpr FF d0 = ff_const(DEDX_UNIT_0), d2 = ff_const(DEDX_UNIT_2), d3 = ff_const(DEDX_UNIT_3),
+                 d4 = ff_const(DEDX_UNIT_4);
+    FF a = ff_add(ff_mul(d4, p), d3);
+    a = ff_add(ff_mul(a, p), d2);
+    a = ff_add(ff_mul(a, p), d1);
+    return ff_add(ff_mul(a, p), d0);
+}
+
+// (float)(ptot + p(ptot) * len) as the reference rounds it
+__device__ __forceinline__ float dim_energy(float ptot, float len, double d1, FF d1f) {
+    using namespace phys;
+    const FF v = ff_add(ff_mul(ff_dedx(ptot, d1f), len), FF{ptot, 0.f});
+    // up to these bounds the loss stays well below ptot, and the polynomial's
+    // terms below 2^6
+    if (ptot < 1000.f && len < 16.f && ff_sure(v)) return v.h;
+    return (float)(ptot + (DEDX_UNIT_0 + d1 * ptot + DEDX_UNIT_2 * ptot * ptot + DEDX_UNIT_3 * ptot * ptot * ptot +
+                           DEDX_UNIT_4 * ptot * ptot * ptot * ptot) *
+                              len);
+}
+
+// (float)(t * STEP_FMAG)
+__device__ __forceinline__ float dim_step(float t) {
+    using namespace phys;
+    const FF v = ff_mul(ff_const(STEP_FMAG), t);
+    if (ff_sure(v)) return v.h;
+    return (float)(t * STEP_FMAG);
+}
+
+// (float)(tx + kick / len)
+__device__ __forceinline__ float dim_kick(float tx, double kick, FF kf, float len) {
+    const float q = kf.h / len;
+    const FF s = ff_sum(tx, q);
+    const FF v = ff_fast(s.h, s.l + (__fmaf_rn(-q, len, kf.h) + kf.l) / len);
+    // (a sum that all but cancels keeps the quotient's error)
+    if (fabsf(v.h) > 0x1p-8f * fabsf(q) && ff_sure(v)) return v.h;
+    return (float)(tx + kick / len);
+}
+
+// What a track's steps have in common.
+struct DimTrack {
+    float charge, ty, t1;  // t1 = (float)(ty * STEP_FMAG)
+    double kick, d1;       // d1 = the linear energy-loss coefficient of the first update, DEDX_UNIT_2 for the
+    FF kickf, d1f;         // reference's second track (H:1354)
+};
+
+// one FMag step (H:1290-1333)
+__device__ __forceinline__ void dim_fmag_step(SwimPt &s, const DimTrack &k) {
+    using namespace phys;
+    const float t2 = (float)STEP_FMAG;
     const float tx_i = s.mx / s.mz;
-    const float tx_f = (float)(tx_i + 2.f * charge * PTKICK_UNIT * STEP_FMAG / sqrtf(s.mx * s.mx + s.mz * s.mz));
-    const float t10 = (float)(tx_i * STEP_FMAG), t11 = (float)(ty * STEP_FMAG), t12 = (float)STEP_FMAG;
-    const float b0 = s.x - t10, b1 = s.y - t11, b2 = s.z - t12;
+    const float tx_f = dim_kick(tx_i, k.kick, k.kickf, sqrtf(s.mx * s.mx + s.mz * s.mz));
+    const float t10 = dim_step(tx_i);
+    const float b0 = s.x - t10, b1 = s.y - k.t1, b2 = s.z - t2;
     const float ptot_i = sqrtf(s.mx * s.mx + s.my * s.my + s.mz * s.mz);
     float ptot_b = ptot_i;
     if (b2 > HOLE_LENGTH_F || b0 * b0 + b1 * b1 > HOLE_RADIUS_F)
-        ptot_b = (float)(ptot_b + (DEDX_UNIT_0 + d1 * ptot_i + DEDX_UNIT_2 * ptot_i * ptot_i +
-                                   DEDX_UNIT_3 * ptot_i * ptot_i * ptot_i + DEDX_UNIT_4 * ptot_i * ptot_i * ptot_i * ptot_i) *
-                                      sqrtf(t10 * t10 + t11 * t11 + t12 * t12));
-    const float t20 = (float)(tx_f * STEP_FMAG), t21 = (float)(ty * STEP_FMAG), t22 = (float)STEP_FMAG;
+        ptot_b = dim_energy(ptot_i, sqrtf(t10 * t10 + k.t1 * k.t1 + t2 * t2), k.d1, k.d1f);
+    const float t20 = dim_step(tx_f);
     s.x = b0 - t20;
-    s.y = b1 - t21;
-    s.z = b2 - t22;
+    s.y = b1 - k.t1;
+    s.z = b2 - t2;
     float ptot_f = ptot_b;
     if (s.z > HOLE_LENGTH_F || s.x * s.x + s.y * s.y > HOLE_RADIUS_F)
-        ptot_f = (float)(ptot_f + dedx_poly(ptot_b) * sqrtf(t20 * t20 + t21 * t21 + t22 * t22));
-    const float pz_f = ptot_f / sqrtf(1.f + tx_f * tx_f + ty * ty);
+        ptot_f = dim_energy(ptot_f, sqrtf(t20 * t20 + k.t1 * k.t1 + t2 * t2), DEDX_UNIT_1, ff_const(DEDX_UNIT_1));
+    const float pz_f = ptot_f / sqrtf(1.f + tx_f * tx_f + k.ty * k.ty);
     s.mx = pz_f * tx_f;
-    s.my = pz_f * ty;
+    s.my = pz_f * k.ty;
     s.mz = pz_f;
 }
 
-__device__ __forceinline__ void dim_target_step(SwimPt &s, float ty) {  // H:1395-1408
-    using namespace phys;
-    const float tx_i = s.mx / s.mz;
-    const float t0 = (float)(tx_i * STEP_TARGET), t1 = (float)(ty * STEP_TARGET), t2 = (float)STEP_TARGET;
-    s.x = s.x - t0;
+// H:1395-1408; a float times 5.0 rounds once, in float or in double
+static_assert(phys::STEP_TARGET == 5.0, "");
+__device__ __forceinline__ void dim_target_step(SwimPt &s, float tx_i, float t1) {
+    s.x = s.x - tx_i * 5.f;
     s.y = s.y - t1;
-    s.z = s.z - t2;
+    s.z = s.z - 5.f;
 }
 
 // a pair's two swims, one per lane, and the point of closest approach
@@ -312,14 +653,27 @@ struct SwimResult {
 // the linear energy-loss coefficient of the first update of a step.
 __device__ __noinline__ void pair_swim(SwimPt s, float charge, float ty, double d1, SwimResult &o) {
     using namespace phys;
+    DimTrack k;
+    k.charge = charge;
+    k.ty = ty;
+    k.t1 = (float)(ty * STEP_FMAG);
+    k.kick = 2.f * charge * PTKICK_UNIT * STEP_FMAG;
+    k.kickf = FF{(float)k.kick, (float)(k.kick - (double)(float)k.kick)};
+    k.d1 = d1;
+    k.d1f = FF{(float)d1, (float)(d1 - (double)(float)d1)};
+    float tx_t = 0.f;  // the slope in the target steps, which keep the momentum
     float dca2_min = 1.e18f;
     SwimPt b = s;
     int found = 0;
     float z66 = 0.f;
 #pragma unroll 1
     for (int j = 0; j <= NSTEPS_FMAG + NSTEPS_TARGET; ++j) {
-        if (j >= 1 && j <= NSTEPS_FMAG) dim_fmag_step(s, charge, ty, d1);
-        else if (j > NSTEPS_FMAG) dim_target_step(s, ty);
+        if (j >= 1 && j <= NSTEPS_FMAG) {
+            dim_fmag_step(s, k);
+            if (j == NSTEPS_FMAG) tx_t = s.mx / s.mz;
+        } else if (j > NSTEPS_FMAG) {
+            dim_target_step(s, tx_t, ty * 5.f);
+        }
         if (j == 66) z66 = s.z;
         const int away = FMAGSTR * charge * s.mx < 0.f;
         const float ox = __shfl_xor_sync(0xffffffffu, s.x, 1), oy = __shfl_xor_sync(0xffffffffu, s.y, 1);
@@ -474,7 +828,7 @@ static_assert(OR_DIM_GROUP <= 32 && DIM_LIST >= OR_TRKMAX, "lane = event; one ev
 // j; opposite charges), sixteen pairs over the events at a time being swum
 // by the whole warp.  A thread per event swimming its pairs one after the
 // other, both tracks in turn, in blocks of 128 took 947 us for 10,000 events
-// and for 2,000; this takes 300 and 227 us.
+// and for 2,000; this takes 136 and 126 us.
 __global__ void __launch_bounds__(32)
     dimuon_kernel(const or_plane_t *__restrict__ gplane, or_tracks_view_t tv, or_dimuons_view_t dv,
                   const uint8_t *__restrict__ toomany, int n_events, int group) {
@@ -664,7 +1018,7 @@ __device__ __constant__ unsigned char c_hist_dim[12] = {OR_DIM_MASS, OR_DIM_XF, 
 // dimuon, and each searches its table.  Bound: the search's L1 latency and
 // the atomics.  With the lanes over the bins of one table at a time, every
 // table of every value was read whole: 151 us for 10,000 one-dimuon events;
-// this takes 36 us.
+// this takes 35 us.
 template <int W>
 __global__ void __launch_bounds__(W * 32)
     hist_kernel(or_tracks_view_t tv, or_dimuons_view_t dv, const int32_t *__restrict__ trigger_bits,
@@ -737,9 +1091,11 @@ __global__ void __launch_bounds__(W * 32)
 cudaError_t launch_vertexing(const or_plane_t *d_plane, or_tracks_view_t tv, const uint8_t *toomany, int n_events,
                              cudaStream_t stream, int sm_count) {
     if (n_events <= 0) return cudaSuccess;
-    // events per warp: a warp per SM first, and at most OR_VTX_GROUP events,
-    // whose tracks fill about one warp
-    const int group = std::max(1, std::min(OR_VTX_GROUP, n_events / sm_count));
+    // events per warp: a warp to each quarter of an SM first, and at most
+    // OR_VTX_GROUP events, whose tracks fill about one warp (2,000 events, 2 /
+    // 4 / 8 / 13 events a warp: 300 / 244 / 253 / 274 us; 10,000 events, 4 / 8
+    // / 16 / 32: 764 / 455 / 332 / 559 us)
+    const int group = std::max(1, std::min(OR_VTX_GROUP, (n_events + 4 * sm_count - 1) / (4 * sm_count)));
     const long blocks = std::min(((long)n_events + group - 1) / group, (long)sm_count * 32);
     vertex_kernel<<<(unsigned)blocks, 32, 0, stream>>>(d_plane, tv, toomany, n_events, group);
     return cudaGetLastError();
