@@ -17,28 +17,35 @@
 //     such hits has an odd length (a hit that closes a cluster does not start
 //     the next one, so in a run every second hit opens one), else "open":
 //     the run's length is a ballot and a carry;
-//   - a hit that closes a cluster, or ends its plane inside one, walks back
-//     to the cluster's first hit and applies the 2-hit or the n-hit rule;
-//   - the first survivor of a channel is the first lane of its
-//     __match_any_sync group whose bit in the plane's map is not set yet.
+//   - a hit that closes a cluster, or ends its plane inside one, lists the
+//     cluster, whose first hit is the last cluster start before it (a ballot
+//     and a carry); the 2-hit and the n-hit rule then take a lane per listed
+//     cluster, in floats (pairs of floats where the reference rounds double
+//     products);
+//   - the first survivor of a channel: where every plane's channels ascend
+//     (a sorted event) the hits of a channel follow one another, and it is the
+//     first kept one of its run; else the lane that sets the channel's bit in
+//     the plane's map, or the first of the lanes of a chunk that share it.
 // Survivors are written back with the new SoA stride into the same slot,
 // consecutive lanes to consecutive words; a plane that keeps all its hits is
 // not written.  Bytes beyond the survivors are left as they were, as the
 // reference leaves them.
 //
-// Bound: instruction issue and shared-memory latency.  One lane per plane
-// running the state machine hit by hit, and writing its plane alone, left
-// most lanes idle, above all in events of many hits, whose batches hold few
-// planes: 2.82 ms for 100,000 uneven events, 972 us for 20,000 of high
-// occupancy, 245 us for 333 uneven ones; this takes 1.60 ms, 566 us and
-// 144 us.
+// Bound: instruction issue, and shared-memory latency behind it (the SM's
+// schedulers issue in 60 % of the cycles; more warps per SM changed nothing).
+// For 100,000 uneven events, 20,000 of high occupancy, 333 uneven and 10,000
+// dimuon ones, in us:
+//   a lane per plane running the state machine          2,820  972  245   99
+//   flat hits, each end walking back to its cluster's
+//   start, channels by __match_any_sync                 1,600  564  144   64
+//   clusters listed, runs of one channel by ballot      1,050  355   80   50
 #include "or_device.cuh"
 
 namespace orgpu {
 
 // Staging buffer per warp: the smallest that holds a full chamber plane.  More
-// batches per event, but more warps per SM (100,000 uneven events 1.60 ms; 1.88
-// at 6 KB, 2.01 at 8 KB).
+// batches per event, but more warps per SM (with the second form above 100,000
+// uneven events took 1.60 ms; 1.88 at 6 KB, 2.01 at 8 KB).
 constexpr int ER_BUF_FLOATS = 1024;
 constexpr int ER_MAX_STAGED_HITS = ER_BUF_FLOATS / 5 + 8;
 constexpr int ER_FIRST_WORDS = (ER_MAX_STAGED_HITS + 31) / 32;
@@ -56,20 +63,22 @@ __device__ __constant__ unsigned char c_er_det[ER_NPLANES] = {
 struct __align__(16) ErWarp {
     float buf[ER_BUF_FLOATS];
     uint64_t bar;
-    int n[ER_NPLANES];
-    int kept[ER_NPLANES];
-    int soff[ER_NPLANES];   // start of each plane's image in buf
-    int hoff[ER_NPLANES];   // hits of the batch before each plane
+    int16_t n[ER_NPLANES];
+    int16_t kept[ER_NPLANES];
+    int16_t at[ER_NPLANES];     // survivors of the batch before each plane
+    int16_t soff[ER_NPLANES];   // start of each plane's image in buf
+    int16_t hoff[ER_NPLANES];   // hits of the batch before each plane
     uint16_t list[ER_MAX_STAGED_HITS];  // chamber hits in time, then the survivors: index in the batch
     uint8_t plane[ER_MAX_STAGED_HITS];  // plane of each hit of the batch
     uint8_t keep[ER_MAX_STAGED_HITS];
-    uint8_t state[ER_MAX_STAGED_HITS];  // of list entries: ER_FIRST, ER_FAR, ER_CLOSED
+    uint8_t chan[ER_MAX_STAGED_HITS];   // its channel, 255 outside 0..201
+    uint8_t cl[ER_MAX_STAGED_HITS / 2][2];  // clusters of two or more: first and last list entry
     uint32_t seen[ER_NPLANES][7];       // channels 0..201 of each plane's survivors
     uint32_t first[ER_FIRST_WORDS];     // bit per hit of the batch: the first of its plane
     float *slot[ER_NPLANES];
     uint8_t occupied[ER_NPLANES];       // the batch's planes with hits
 };
-constexpr uint8_t ER_FIRST = 1, ER_FAR = 2, ER_CLOSED = 4;
+static_assert(ER_MAX_STAGED_HITS <= 256, "a list entry fits a byte");
 static_assert(7 * 32 >= 202, "channel bits");
 
 struct PlaneRef {
@@ -98,6 +107,15 @@ __device__ __forceinline__ PlaneRef er_plane(const or_hits_view_t &hv, long e, i
     return r;
 }
 
+// (float)(c * x); the double product's rounding of a float is its second, so
+// pairs of floats decide it nearly always (an FP64 instruction takes 64 cycles)
+__device__ __noinline__ float er_scale_double(double c, float x) { return (float)(c * (double)x); }
+__device__ __forceinline__ float er_scale(double c, FF cf, float x) {
+    const FF v = ff_mul(cf, x);
+    if (x == 0.f) return x;
+    return ff_sure(v) ? v.h : er_scale_double(c, x);
+}
+
 // The rules for a cluster of `cls` >= 2 in-time hits list[s..t] of one plane
 // (reference H:267-318); h = the plane's image, n its hits, first the batch
 // index of its first hit.
@@ -108,13 +126,14 @@ static __device__ __forceinline__ void er_cluster(ErWarp &S, int s, int t, const
     const int cls = t - s + 1;
     const int a = S.list[s] - first, b = S.list[t] - first;
     if (cls == 2) {  // H:267-295
-        const float w_max = (float)(0.9 * 0.5 * (double)(pos(b) - pos(a)));
-        const float w_min = (float)(4.0 / 9.0 * (double)w_max);
+        constexpr FF half = ff_const(0.9 * 0.5), ninths = ff_const(4.0 / 9.0);
+        const float w_max = er_scale(0.9 * 0.5, half, pos(b) - pos(a));
+        const float w_min = er_scale(4.0 / 9.0, ninths, w_max);
         if ((drift(a) > w_max && drift(b) > w_min) || (drift(a) > w_min && drift(b) > w_max)) {
             S.keep[first + (drift(a) > drift(b) ? a : b)] = 0;
         } else {
             const float dt = tdc(a) - tdc(b);
-            if ((((double)dt >= 0.0 && (double)dt < 8.0) || ((double)dt <= 0.0 && (double)dt > -8.0)) &&
+            if (((dt >= 0.f && dt < 8.f) || (dt <= 0.f && dt > -8.f)) &&
                 (det >= 19 && det <= 24)) {
                 S.keep[first + a] = 0;
                 S.keep[first + b] = 0;
@@ -126,23 +145,22 @@ static __device__ __forceinline__ void er_cluster(ErWarp &S, int s, int t, const
         for (int k = s + 1; k <= t; ++k) {
             const int m = S.list[k] - first;
             const float d = tdc(m) - tdc(prev);
-            dt_mean += ((double)d > 0.0 ? d : (tdc(prev) - tdc(m)));
+            dt_mean += (d > 0.f ? d : (tdc(prev) - tdc(m)));
             prev = m;
         }
         dt_mean = dt_mean / (float)(cls - 1);
-        const bool all = (double)dt_mean < 10.0;
+        const bool all = dt_mean < 10.f;
         for (int k = all ? s : s + 1; k <= t; ++k) S.keep[S.list[k]] = 0;
     }
 }
 
 // event_reduction() (reconstruction_helper.cuh:168-361) on the staged planes
-// [p0, p1) of `hits` hits: S.kept and, per plane in order, the survivors'
-// batch indices in S.list.  The after-pulse branch (H:204-230) never changes a
+// [p0, p1) of `hits` hits: S.kept, S.at and, per plane in order, the
+// survivors' batch indices in S.list; returns their number.  The after-pulse branch (H:204-230) never changes a
 // flag: uniqueID_curr is reset every hit.
-static __device__ __forceinline__ void er_reduce(ErWarp &S, int p0, int p1, int hits) {
+static __device__ __forceinline__ int er_reduce(ErWarp &S, int p0, int p1, int hits) {
     const int lane = threadIdx.x & 31;
     const unsigned lt = lanemask_lt();
-    for (int i = p0 * 7 + lane; i < p1 * 7; i += 32) S.seen[0][i] = 0u;
     for (int i = lane; i < ER_FIRST_WORDS; i += 32) S.first[i] = 0u;
     __syncwarp();
     int nocc = 0;
@@ -158,88 +176,145 @@ static __device__ __forceinline__ void er_reduce(ErWarp &S, int p0, int p1, int 
         nocc += __popc(m);
     }
     __syncwarp();
-    // in-time hits; those of chambers are listed
+    // in-time hits; those of chambers are listed.  `up`: the channels of
+    // every plane are in ascending order, as a sorted event's are
     int nlist = 0, started = 0;
+    bool up = true;
+    float before = 0.f;  // the last chunk's last channel
 #pragma unroll 1
     for (int b0 = 0; b0 < hits; b0 += 32) {
         const int f = b0 + lane;
         bool cham = false;
+        float x = 0.f;
         if (f < hits) {
             // its plane: as many occupied planes start at or before it
             const int p = S.occupied[started + __popc(S.first[b0 >> 5] & (lt | (1u << lane))) - 1];
             const int n = S.n[p], i = f - S.hoff[p];
             const bool intime = (((int)S.buf[S.soff[p] + 3 * n + i]) & 2) != 0;  // H:198
+            x = S.buf[S.soff[p] + i];
+            const int c = (short)x;
             S.plane[f] = (uint8_t)p;
+            S.chan[f] = (uint8_t)(c >= 0 && c < 202 ? c : 255);
             S.keep[f] = intime;
             cham = intime && p < ER_NCHAMBERS;
         }
+        float y = __shfl_up_sync(0xffffffffu, x, 1);
+        if (lane == 0) y = before;
+        before = __shfl_sync(0xffffffffu, x, 31);
+        up &= f >= hits || (x > -32768.f && x < 32768.f && (((S.first[b0 >> 5] >> lane) & 1u) || y <= x));
         started += __popc(S.first[b0 >> 5]);
         const unsigned m = __ballot_sync(0xffffffffu, cham);
         if (cham) S.list[nlist + __popc(m & lt)] = (uint16_t)f;
         nlist += __popc(m);
     }
     __syncwarp();
-    // cluster state after each listed hit (H:241-258)
+    // cluster state after each listed hit (H:241-258), and the clusters of two
+    // or more, each at the hit that ends it: a cluster starts at its plane's
+    // first listed hit or after a hit that closed one
     int run = 0;  // hits far from the one before, up to the last chunk's end
+    int begin = 0, ncl = 0;
+    unsigned after = 0u;  // the last chunk's last hit closed a cluster
 #pragma unroll 1
     for (int b0 = 0; b0 < nlist; b0 += 32) {
         const int k = b0 + lane;
-        uint8_t st = ER_FIRST;
-        if (k < nlist && k > 0) {
-            const int f = S.list[k], g = S.list[k - 1], p = S.plane[f];
-            if (S.plane[g] == p) {
+        bool first = true, far = false, last = false;
+        if (k < nlist) {
+            const int f = S.list[k], p = S.plane[f];
+            last = f - S.hoff[p] == S.n[p] - 1;
+            const int g = k > 0 ? S.list[k - 1] : f;
+            if (k > 0 && S.plane[g] == p) {
                 const float *h = S.buf + S.soff[p] - S.hoff[p];
-                st = fabsf(h[f] - h[g]) > 1 ? ER_FAR : 0;
+                first = false;
+                far = fabsf(h[f] - h[g]) > 1;
             }
         }
-        const unsigned near = __ballot_sync(0xffffffffu, st != ER_FAR);
-        const int l = last_lane(near & (lt | (1u << lane)));
+        const unsigned le = lt | (1u << lane);
+        const unsigned near = ~__ballot_sync(0xffffffffu, far);
+        const int l = last_lane(near & le);
         const int r = l >= 0 ? lane - l : run + lane + 1;
-        if ((st & ER_FAR) && (r & 1)) st |= ER_CLOSED;
-        if (k < nlist) S.state[k] = st;
+        const bool closes = far && (r & 1);
+        const unsigned closed = __ballot_sync(0xffffffffu, closes);
+        const unsigned starts = __ballot_sync(0xffffffffu, first && k < nlist) | (closed << 1) | after;
+        // [s, t] ends here: before the hit that closes it, or with the plane
+        const int m = last_lane(starts & (closes ? lt : le));
+        const int s = m >= 0 ? b0 + m : begin;
+        const int t = closes ? k - 1 : !first && !far && last ? k : -1;
+        const unsigned cm = __ballot_sync(0xffffffffu, t > s);
+        if (t > s) {
+            uint8_t *c = S.cl[ncl + __popc(cm & lt)];
+            c[0] = (uint8_t)s;
+            c[1] = (uint8_t)t;
+        }
+        ncl += __popc(cm);
+        const int mm = last_lane(starts);
+        if (mm >= 0) begin = b0 + mm;
+        after = closed >> 31;
         run = __shfl_sync(0xffffffffu, r, 31);
     }
     __syncwarp();
-    // clusters, each at the hit that ends it
 #pragma unroll 1
-    for (int k = lane; k < nlist; k += 32) {
-        const uint8_t st = S.state[k];
-        const int f = S.list[k], p = S.plane[f], n = S.n[p], first = S.hoff[p];
-        int t = -1;
-        if (st & ER_CLOSED) t = k - 1;
-        else if (st == 0 && f - first == n - 1 && !(S.state[k - 1] & ER_CLOSED)) t = k;  // H:258, the plane's last hit
-        if (t < 0) continue;
-        int s = t;
-        while (!(S.state[s] & ER_FIRST) && !(S.state[s - 1] & ER_CLOSED)) --s;
-        if (t > s) er_cluster(S, s, t, S.buf + S.soff[p], n, first, c_er_det[p]);
+    for (int k = lane; k < ncl; k += 32) {
+        const int s = S.cl[k][0], t = S.cl[k][1], p = S.plane[S.list[s]];
+        er_cluster(S, s, t, S.buf + S.soff[p], S.n[p], S.hoff[p], c_er_det[p]);
     }
     __syncwarp();
     // H:334-349, first survivor per channel wins
     int ns = 0;
+    up = __all_sync(0xffffffffu, up);
+    if (!up) {
+        for (int i = p0 * 7 + lane; i < p1 * 7; i += 32) S.seen[0][i] = 0u;
+        __syncwarp();
+    }
+    int chan = -1;      // the last chunk's last channel, and
+    bool taken = false;  // whether it has a survivor
 #pragma unroll 1
     for (int b0 = 0; b0 < hits; b0 += 32) {
         const int f = b0 + lane;
-        bool k = f < hits && S.keep[f];
-        int p = 0, c = -1;
-        if (k) {
+        int p = 0, c = 255;
+        bool k = false, first = true;
+        if (f < hits) {
             p = S.plane[f];
-            c = (short)S.buf[S.soff[p] + f - S.hoff[p]];
-            if (c < 0 || c >= 202) c = -1;
+            k = S.keep[f];
+            c = S.chan[f];
+            first = (S.first[b0 >> 5] >> lane) & 1u;
         }
-        const unsigned peers = __match_any_sync(0xffffffffu, c >= 0 ? p * 256 + c : -1 - lane);
-        if (k && c >= 0) {
-            k = (peers & lt) == 0u && !((S.seen[p][c >> 5] >> (c & 31)) & 1u);
-        }
-        __syncwarp();
-        if (k) {
-            if (c >= 0) atomicOr(&S.seen[p][c >> 5], 1u << (c & 31));
-            atomicAdd(&S.kept[p], 1);
+        if (up) {
+            // hits of one channel follow one another
+            int d = __shfl_up_sync(0xffffffffu, c, 1);
+            if (lane == 0) d = chan;
+            const unsigned starts = __ballot_sync(0xffffffffu, first || c != d);
+            const unsigned all = __ballot_sync(0xffffffffu, k);
+            const int l = last_lane(starts & (lt | (1u << lane)));
+            const unsigned same = lt & (l >= 0 ? ~0u << l : ~0u);  // its channel's hits before it
+            bool had = (all & same) != 0u || (l < 0 && taken);
+            if (c != 255) k = k && !had;
+            chan = __shfl_sync(0xffffffffu, c, 31);
+            taken = __shfl_sync(0xffffffffu, had || ((all >> lane) & 1u), 31);
+        } else {
+            if (!k) c = 255;
+            // a lane that finds its channel's bit set is a later hit of the
+            // channel, or shares it with lanes of this chunk: of those the
+            // first survives, unless the bit was set before
+            if (c != 255) k = !((atomicOr(&S.seen[p][c >> 5], 1u << (c & 31)) >> (c & 31)) & 1u);
+            if (__any_sync(0xffffffffu, c != 255 && !k)) {
+                const unsigned peers = __match_any_sync(0xffffffffu, c != 255 ? p * 256 + c : -1 - lane);
+                const unsigned set = __ballot_sync(0xffffffffu, k) & peers;
+                if (c != 255) k = set != 0u && (peers & lt) == 0u;
+            }
         }
         const unsigned m = __ballot_sync(0xffffffffu, k);
-        if (k) S.list[ns + __popc(m & lt)] = (uint16_t)f;
+        const int j = ns + __popc(m & lt);
+        if (k) S.list[j] = (uint16_t)f;
+        if (f < hits && first) S.at[p] = (int16_t)j;
         ns += __popc(m);
         __syncwarp();
     }
+    for (int o = lane; o < nocc; o += 32) {
+        const int p = S.occupied[o];
+        S.kept[p] = (int16_t)((o + 1 < nocc ? S.at[S.occupied[o + 1]] : ns) - S.at[p]);
+    }
+    __syncwarp();
+    return ns;
 }
 
 template <int W>
@@ -258,7 +333,7 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
         for (int p = lane; p < ER_NPLANES; p += 32) {
             const PlaneRef r = er_plane(hv, e, c_er_det[p]);
             const int n = (int)*r.count;
-            S.n[p] = n < r.cap ? n : r.cap;
+            S.n[p] = (int16_t)(n < r.cap ? n : r.cap);
             S.slot[p] = r.slot;
         }
         __syncwarp();
@@ -285,8 +360,8 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
                 const bool fit = off + csz <= ER_BUF_FLOATS;
                 const int nfit = __popc(__ballot_sync(0xffffffffu, fit));
                 if (fit) {
-                    S.soff[p] = off + csz - sz_l;
-                    S.hoff[p] = hits + cn - n_l;
+                    S.soff[p] = (int16_t)(off + csz - sz_l);
+                    S.hoff[p] = (int16_t)(hits + cn - n_l);
                 }
                 if (nfit == 0) break;
                 off += __shfl_sync(0xffffffffu, csz, nfit - 1);
@@ -317,37 +392,17 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
                 }
                 phase ^= 1u;
             }
-            er_reduce(S, p0, p1, hits);
-            // write back the planes that lost hits: the survivors of plane p
-            // are list entries [at, at + kept)
-            int at = 0;
+            const int ns = er_reduce(S, p0, p1, hits);
+            for (int p = p0 + lane; p < p1; p += 32) *er_plane(hv, e, c_er_det[p]).count = (uint32_t)S.kept[p];
+            // write back the planes that lost hits
 #pragma unroll 1
-            for (int q0 = p0; q0 < p1; q0 += 32) {
-                const int p = q0 + lane;
-                const int nk = p < p1 ? S.kept[p] : 0;
-                int incl = nk;
+            for (int j = lane; j < ns; j += 32) {
+                const int f = S.list[j], p = S.plane[f], n = S.n[p], k = S.kept[p];
+                if (k == n) continue;
+                const float *src = S.buf + S.soff[p] - S.hoff[p] + f;
+                float *dst = S.slot[p] + j - S.at[p];
 #pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, incl, d);
-                    if (lane >= d) incl += v;
-                }
-                const int start = at + incl - nk;
-                const bool less = p < p1 && nk < S.n[p];
-                if (p < p1) *er_plane(hv, e, c_er_det[p]).count = (uint32_t)nk;
-                for (unsigned m = __ballot_sync(0xffffffffu, less); m; m &= m - 1) {
-                    const int l = __ffs(m) - 1, q = q0 + l;
-                    const int k = __shfl_sync(0xffffffffu, nk, l), s0 = __shfl_sync(0xffffffffu, start, l);
-                    const int n = S.n[q];
-                    const float *src = S.buf + S.soff[q] - S.hoff[q];
-                    float *dst = S.slot[q];
-#pragma unroll 1
-                    for (int i = lane; i < k; i += 32) {
-                        const float *h = src + S.list[s0 + i];
-#pragma unroll
-                        for (int f = 0; f < 5; ++f) dst[f * k + i] = h[f * n];
-                    }
-                }
-                at += __shfl_sync(0xffffffffu, incl, 31);
+                for (int q = 0; q < 5; ++q) dst[q * k] = src[q * n];
             }
             __syncwarp();
             p0 = p1;

@@ -83,48 +83,6 @@ __device__ __forceinline__ double dedx_poly(double p) {
 }
 
 // ---------------------------------------------------------------------------
-// float results of double expressions
-
-// A value as an unevaluated sum of two floats, |l| <= ulp(h) / 2, to some 44
-// bits: the statements of a step that the reference evaluates in double and
-// stores in a float are evaluated this way first (error-free sums and
-// products: T. J. Dekker, Numer. Math. 18, 1971; D. E. Knuth, TAOCP vol. 2,
-// 4.2.2), and in double only where that leaves the float's rounding open.  The
-// results are the same bits; the FP64 pipe takes 64 cycles per warp
-// instruction (measured, whatever the active lanes), so a step's 60 of them
-// were all its time.
-struct FF {
-    float h, l;
-};
-__device__ __forceinline__ FF ff_sum(float a, float b) {  // |a|, |b| in any order
-    const float s = a + b, t = s - a;
-    return FF{s, (a - (s - t)) + (b - t)};
-}
-__device__ __forceinline__ FF ff_fast(float a, float b) {  // |a| >= |b|
-    const float s = a + b;
-    return FF{s, b - (s - a)};
-}
-__device__ __forceinline__ FF ff_mul(FF a, float b) {
-    const float p = a.h * b;
-    return ff_fast(p, __fmaf_rn(a.h, b, -p) + a.l * b);
-}
-__device__ __forceinline__ FF ff_add(FF a, FF b) {
-    const FF s = ff_sum(a.h, b.h);
-    return ff_fast(s.h, s.l + (a.l + b.l));
-}
-__host__ __device__ constexpr FF ff_const(double c) { return FF{(float)c, (float)(c - (double)(float)c)}; }
-
-// Whether v.h is the float nearest to every number within 2^-37 |v.h| of the
-// sum: the rest must stay clear of half the last place by that much (and of a
-// quarter below a power of two).
-__device__ __forceinline__ bool ff_sure(FF v) {
-    const unsigned u = __float_as_uint(v.h) & 0x7fffffffu;
-    const unsigned e = u & 0x7f800000u;
-    const float half = __uint_as_float(e - (24u << 23)) * ((u & 0x7fffffu) ? 1.f - 0x1p-11f : 0.5f - 0x1p-11f);
-    return (e - (40u << 23) <= (210u << 23)) & (fabsf(v.l) < half);
-}
-
-// ---------------------------------------------------------------------------
 // vertexing (K:2594-2803)
 
 #ifndef OR_VTX_GROUP
