@@ -14,11 +14,15 @@
 // runs are where the det changes from one record to the next, then the field
 // writes, 128 records in flight in both passes.
 //
-// Bound: DRAM latency and the 200-byte pieces that an event's planes are
-// written in.  A histogram by shared-memory atomics (all lanes on one counter
-// where records are sorted), a scan by one lane and one record in flight per
-// lane took 685 us for 100,000 uneven events and, with the R-T spline, 166 us
-// for 16,001; this takes 580 and 141 us (two chunks in flight: 647 and 164).
+// Bound: the pieces of 100 to 600 bytes, off sector boundaries, that an
+// event's planes are written in (3.5 of 6.9 TB/s; staging the records in
+// shared memory by bulk copies, so that no read waits, changed nothing: 519
+// us).  A histogram by shared-memory atomics (all lanes on one counter where
+// records are sorted), a scan by one lane and one record in flight per lane
+// took 685 us for 100,000 uneven events and, with the R-T spline, 166 us for
+// 16,001; plane runs from neighbours and 128 records in flight 600 and 143
+// us; whole-record loads, 512 planes in flight and a block per eight events
+// 513 and 122 us (20,000 events of high occupancy 259 -> 236 us).
 //
 // With an R-T table the drift field is computed from the tdc as the
 // reference host does while packing (online_reconstruction.cu:387-396); the
@@ -28,7 +32,8 @@
 namespace orgpu {
 
 constexpr int PK_WARPS = 8;
-constexpr int PK_AHEAD = 4;  // chunks of 32 records in flight per warp
+constexpr int PK_DETS = 16;  // chunks of 32 records whose plane is in flight per warp
+constexpr int PK_AHEAD = 4;  // ... and whose fields are
 constexpr int PK_BLOCKS = 4; // per SM: 64 registers
 
 // Drift distance of a hit on plane det from the R-T calibration, or `drift`
@@ -68,7 +73,21 @@ static __device__ __forceinline__ bool rt_plane(int det) {
     return (det >= 1 && det <= OR_NCHAM) || (det > OR_NCHAM + OR_NHODO && det < OR_NDET);
 }
 
-template <bool RT>
+// One record; `AL`: the records are 16-byte aligned, one load each
+template <bool AL>
+static __device__ __forceinline__ or_hit_record_t pk_record(const or_hit_record_t *R) {
+    if (!AL) return *R;
+    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(R));
+    or_hit_record_t h;
+    h.det = (int16_t)(v.x & 0xffffu);
+    h.elem = (int16_t)(v.x >> 16);
+    h.tdc = __uint_as_float(v.y);
+    h.drift = __uint_as_float(v.z);
+    h.flag = (int32_t)v.w;
+    return h;
+}
+
+template <bool RT, bool AL>
 __global__ void __launch_bounds__(PK_WARPS * 32, PK_BLOCKS)
     pack_kernel(const or_hit_record_t *__restrict__ rec, const int64_t *__restrict__ off, int n_events,
                 const float *__restrict__ wire_pos_f, const or_rt_table_t *__restrict__ rt, or_hits_view_t hv,
@@ -89,15 +108,15 @@ __global__ void __launch_bounds__(PK_WARPS * 32, PK_BLOCKS)
         // Records with det out of range sort first or last and are skipped.
         int carry = -0x10000;  // det of the record before the chunk
 #pragma unroll 1
-        for (int b0 = 0; b0 < nrec; b0 += 32 * PK_AHEAD) {
-            int d[PK_AHEAD];
+        for (int b0 = 0; b0 < nrec; b0 += 32 * PK_DETS) {
+            int d[PK_DETS];
 #pragma unroll
-            for (int i = 0; i < PK_AHEAD; ++i) {
+            for (int i = 0; i < PK_DETS; ++i) {
                 const int r = b0 + 32 * i + lane;
                 d[i] = r < nrec ? (int)R[r].det : 0x10000;
             }
 #pragma unroll
-            for (int i = 0; i < PK_AHEAD; ++i) {
+            for (int i = 0; i < PK_DETS; ++i) {
                 const int r = b0 + 32 * i + lane;
                 int prev = __shfl_up_sync(0xffffffffu, d[i], 1);
                 if (lane == 0) prev = carry;
@@ -132,7 +151,7 @@ __global__ void __launch_bounds__(PK_WARPS * 32, PK_BLOCKS)
                 const int r = b0 + 32 * i + lane;
                 h[i].det = (int16_t)0x7FFF;
                 h[i].elem = 0;
-                if (r < nrec) h[i] = R[r];
+                if (r < nrec) h[i] = pk_record<AL>(R + r);
             }
 #pragma unroll
             for (int i = 0; i < PK_AHEAD; ++i) {
@@ -206,9 +225,11 @@ __global__ void __launch_bounds__(PK_WARPS * 32)
     }
 }
 
+// Blocks beyond the resident ones even out events of different size (100,000
+// uneven events: 8 blocks to an SM 582 us, 32: 542, one event per warp: 513).
 static long pack_blocks(int n_events, int sm_count) {
     long blocks = (n_events + PK_WARPS - 1) / PK_WARPS;
-    const long cap = (long)sm_count * 8;
+    const long cap = (long)sm_count * 512;
     return blocks > cap ? cap : blocks;
 }
 
@@ -217,10 +238,13 @@ cudaError_t launch_pack(const or_hit_record_t *rec, const int64_t *off, int n_ev
                         int sm_count) {
     if (n_events <= 0) return cudaSuccess;
     const unsigned blocks = (unsigned)pack_blocks(n_events, sm_count);
-    if (rt)
-        pack_kernel<true><<<blocks, PK_WARPS * 32, 0, stream>>>(rec, off, n_events, wire_pos_f, rt, hv, errw);
-    else
-        pack_kernel<false><<<blocks, PK_WARPS * 32, 0, stream>>>(rec, off, n_events, wire_pos_f, nullptr, hv, errw);
+    // records of an aligned table are read whole; those of any other (a record
+    // is 16 bytes of 4-byte alignment) field by field (20,000 events of high
+    // occupancy: 236 and 248 us)
+    const bool al = (reinterpret_cast<uintptr_t>(rec) & 15u) == 0;
+    auto *kernel = rt ? (al ? pack_kernel<true, true> : pack_kernel<true, false>)
+                      : (al ? pack_kernel<false, true> : pack_kernel<false, false>);
+    kernel<<<blocks, PK_WARPS * 32, 0, stream>>>(rec, off, n_events, wire_pos_f, rt, hv, errw);
     return cudaGetLastError();
 }
 
