@@ -43,7 +43,7 @@ cudaError_t launch_yz_outer_labels(void *, int, int, int, or_tracks_view_t, cons
                                    const uint32_t *, long, uint8_t *, cudaStream_t, int);
 cudaError_t launch_rt_apply(const or_rt_table_t *, or_hits_view_t, int, cudaStream_t, int);
 cudaError_t launch_collect(or_tracks_view_t, const uint8_t *, int, float, float *, long long, unsigned long long *,
-                           cudaStream_t);
+                           cudaStream_t, int);
 cudaError_t launch_yz_pruned(const or_plane_t *, or_hits_view_t, or_tracks_view_t, const uint8_t *, int, uint32_t *,
                              void *, int, int, int, cudaStream_t, int, const int32_t *, const uint8_t *, long, int,
                              long long, int);
@@ -818,7 +818,7 @@ int or_collect_tracks(or_ctx_t *ctx, or_tracks_view_t tracks, const uint8_t *too
         return fail(OR_ERR_ARG, "bad collect arguments");
     if ((rc = check_tracks(tracks))) return rc;
     cudaError_t e = orgpu::launch_collect(tracks, toomany, n_events, stid, out, (long long)capacity,
-                                          reinterpret_cast<unsigned long long *>(d_count), S(stream));
+                                          reinterpret_cast<unsigned long long *>(d_count), S(stream), ctx->sm_count);
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "collect launch");
 }
 
