@@ -278,17 +278,27 @@ struct YzEvent {
     short dl[8];
 };
 
+// What the lanes exchange while a chunk of survivors is evaluated
+struct YzPhase2 {
+    float term[16 * 12];      // chi2 terms
+    signed char res[32 * 8];  // per survivor and hit: the pair's resolution or the hit's sign
+    unsigned char item[32 * 8];
+};
+
 struct YzWarp {
     YzEvent ev;  // the event's plane views, the same for every lane
     Stale st[4];  // scratch entries 4..7 as the next combination finds them, the same for every lane
     YzHit arena[YZ_ARENA_HITS];
     short2 pair[4][YZ_MAXPAIR];  // windowed indices (or -1) in sides 0, 1 of list q
-    struct {
-        int start[8];
-        float xmin[4], xmax[4];
-        unsigned fl[(8 * YZ_MAXWIN + 31) / 32];  // windowed hits that are in a pair
-        unsigned char widx[8 * YZ_MAXWIN];       // plane hit index of each windowed hit
-    } w;                                         // while the windows are built
+    union {
+        struct {
+            int start[8];
+            float xmin[4], xmax[4];
+            unsigned fl[(8 * YZ_MAXWIN + 31) / 32];  // windowed hits that are in a pair
+            unsigned char widx[8 * YZ_MAXWIN];       // plane hit index of each windowed hit
+        };                                           // while the windows are built
+        YzPhase2 d;                                  // while survivors are evaluated
+    } w;
     int np[4], nw[8], woff[8];
     float x0, tx, ex0, etx;
     int nhx;
@@ -627,72 +637,27 @@ __device__ __forceinline__ void uv_set_sign(UvSet &U, int k, int s) {
     U.sign = (U.sign & ~(3u << (2 * k))) | (((unsigned)s & 3u) << (2 * k));
 }
 
-// resolve_leftright_newhits walk over the n hits of U with the scratch entry
-// past the end given by `st` (H:714-780), then the singles (H:785-804).
-__device__ __forceinline__ void walk_newhits(int n, UvSet &U, const YzHit *base, const Stale &st, float x0, float tx,
-                                             float y0, float ty, float ex0, float etx, float ey0, float ety,
-                                             const or_plane_t &P) {
+// The pairs resolve_leftright_newhits walks over (H:714-780): hits i and i + 1
+// (or the scratch entry past the end, plane `dst`) of neighbouring planes, not
+// both with a sign; bit i set.  They depend on the planes and the starting
+// signs alone, and no hit is in two of them.
+__device__ __forceinline__ unsigned yz_walk_pairs(int n, const UvSet &U, const YzHit *base, short dst) {
+    unsigned pm = 0u;
+    if (n == 0) return pm;
+    short di = base[uv_off(U, 0)].det;
+    bool paired = false;  // hit i was the second of a pair
 #pragma unroll 1
-    for (int i = 0; i < n;) {
-        const int j = i + 1;
-        const YzHit &hi = base[uv_off(U, i)];
-        const short di = hi.det;
-        short dj = st.det, sj = 0;
-        float pj = st.pos, drj = st.drift;
-        if (j < n) {
-            const YzHit &hj = base[uv_off(U, j)];
-            dj = hj.det;
-            sj = uv_sign(U, j);
-            pj = hj.pos;
-            drj = hj.drift;
+    for (int i = 0; i < n; ++i) {
+        const short dj = i + 1 < n ? base[uv_off(U, i + 1)].det : dst;
+        if (!paired && abs(di - dj) == 1) {
+            if (!uv_sign(U, i) || i + 1 >= n || !uv_sign(U, i + 1)) pm |= 1u << i;
+            paired = true;
+        } else {
+            paired = false;
         }
-        if (abs(di - dj) != 1) {
-            i += 1;
-            continue;
-        }
-        if (uv_sign(U, i) * sj == 0) {
-            const int k = lr_pair_newhits(x0, tx, y0, ty, ex0, etx, ey0, ety, di, dj, hi.pos, hi.drift, pj, drj, P,
-                                          150.f);
-            if (k >= 0) {
-                uv_set_sign(U, i, c_lrpossibility[k][0]);
-                if (j < n) uv_set_sign(U, j, c_lrpossibility[k][1]);
-            }
-        }
-        i += 2;
+        di = dj;
     }
-#pragma unroll 1
-    for (int k = 0; k < n; ++k) {
-        if (uv_sign(U, k)) continue;
-        const YzHit &h = base[uv_off(U, k)];
-        uv_set_sign(U, k, single_sign_newhits(x0, tx, y0, ty, h.det, h.pos, P));
-    }
-}
-
-// The per-survivor work below runs once per 32 queued survivors, between long
-// stretches of the first-cut loop; it is kept out of line (one copy each) so
-// that the loop's instructions stay resident in the instruction cache.  The
-// walk takes and returns the hit set by value (registers, not a stack frame).
-__device__ __noinline__ unsigned walk_uv(int n, UvSet U, const YzHit *base, Stale st, float x0, float tx, float y0,
-                                         float ty, float ex0, float etx, float ey0, float ety, const or_plane_t &P) {
-    walk_newhits(n, U, base, st, x0, tx, y0, ty, ex0, etx, ey0, ety, P);
-    return U.sign;
-}
-
-// Index of the last station-3 hit when the walk pairs it with the first
-// station-2 hit, else -1.  The walk's pairs depend only on plane ids.
-__device__ __forceinline__ int cross_pair_index(int n3, const UvSet &U, const YzHit *base, int nuv) {
-#pragma unroll 1
-    for (int i = 0; i < n3;) {
-        const int j = i + 1;
-        if (j >= nuv) return -1;
-        if (abs(base[uv_off(U, i)].det - base[uv_off(U, j)].det) != 1) {
-            i += 1;
-            continue;
-        }
-        if (j == n3) return i;
-        i += 2;
-    }
-    return -1;
+    return pm;
 }
 
 __device__ __forceinline__ const YzHit *yz_list(const YzWarp &S, const YzHit *base, int l) { return base + S.woff[l]; }
@@ -1046,19 +1011,6 @@ __device__ __forceinline__ float yz_residual(const YzWarp &S, const UvSet &U, co
                          P.deltapz[d], h.drift, uv_sign(U, k), x0, y0, tx, ty);
 }
 
-// chi2_track over the x hits and the uv hits (H:1182-1204)
-__device__ __noinline__ float yz_chi2(const YzWarp &S, UvSet U, const YzHit *base, int nuv, int nhx,
-                                      const or_plane_t &P, float x0, float y0, float tx, float ty) {
-    float chi2 = 0.f;
-#pragma unroll 1
-    for (int m = 0; m < nhx + nuv; ++m) {
-        float res;
-        const float r = yz_residual(S, U, base, m, nhx, P, x0, y0, tx, ty, res);
-        chi2 += r * r / res / res;
-    }
-    return chi2;
-}
-
 // Sign state carried from one survivor chunk to the next (the first
 // combination of an outer iteration fixes the station-3 signs), and the best
 // key so far.
@@ -1072,8 +1024,13 @@ struct Phase2Carry {
 
 // The full evaluation of n (<= 32) queued survivors Qc[0..n), in order: sign
 // state, left/right walk, prop and hodoscope gates, chi2, best key
-// (K:1613-1799).  Out of line: it runs once per 32 survivors, and inlined it
-// would sit in the middle of the first-cut loop's instructions.  GATED: the
+// (K:1613-1799).  The pairs to resolve, the single hits and the chi2 terms of
+// all survivors are dealt to the lanes one by one: a chunk holds 8 (dimuon
+// events) or 20 (uneven ones) survivors on average, and a lane per survivor
+// left the others idle and the walks diverging (survivor kernel, 10,000
+// dimuon events 317 -> 214 us, 100,000 uneven 8.2 -> 6.2 ms).  Out of line: it
+// runs once per 32 survivors, and inlined it would sit in the middle of the
+// first-cut loop's instructions.  GATED: the
 // survivors come from the first-cut kernel (YzSurv), which has evaluated the
 // gates; `tab` is the station half's table, S.st the unit's starting entries.
 template <bool GATED>
@@ -1138,13 +1095,99 @@ __device__ __noinline__ void yz_phase2(YzWarp &S, const YzEvent &E, const YzHit 
     // station-3 pairs and singles and resolves the station-2 hits and the
     // cross pair exactly as it does after their real signs, which are put in
     // below (the first survivor's, or the cross pair's where it resolved).
+    // The pairs and then the single hits of all survivors are dealt to the
+    // lanes (item: survivor << 3 | hit): a chunk holds a few survivors more
+    // often than 32.
+    YzPhase2 &D = S.w.d;
+    auto deal = [&](unsigned m) {
+        int tot = 0;
+        for (unsigned b; (b = __ballot_sync(0xffffffffu, m != 0u)) != 0u;) {
+            if (m) D.item[tot + __popc(b & lanemask_lt())] = (unsigned char)(lane << 3 | (__ffs(m) - 1));
+            tot += __popc(b);
+            m &= m - 1;
+        }
+        __syncwarp();
+        return tot;
+    };
+    // survivor o's hits
+    auto shfl_set = [&](int o) {
+        const unsigned l0 = __shfl_sync(0xffffffffu, (unsigned)U.lo, o), l1 = __shfl_sync(0xffffffffu, (unsigned)(U.lo >> 32), o);
+        const unsigned h0 = __shfl_sync(0xffffffffu, (unsigned)U.hi, o), h1 = __shfl_sync(0xffffffffu, (unsigned)(U.hi >> 32), o);
+        UvSet V{(unsigned long long)l1 << 32 | l0, (unsigned long long)h1 << 32 | h0, 0u};
+        return V;
+    };
+    unsigned pm = 0u;
     if (valid) {
         if (!is_first) {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
                 if (k < n3) uv_set_sign(U, k, 1);
         }
-        U.sign = walk_uv(nuv, U, base, stj, x0, tx, y0, ty, ex0, etx, ey0, ety, P);
+        pm = yz_walk_pairs(nuv, U, base, stj.det);
+    }
+    {
+        const int tot = deal(pm);
+#pragma unroll 1
+        for (int t0 = 0; t0 < tot; t0 += 32) {
+            const bool in = t0 + lane < tot;
+            const int it = in ? D.item[t0 + lane] : 0, o = it >> 3, i = it & 7;
+            const UvSet V = shfl_set(o);
+            const float oy = __shfl_sync(0xffffffffu, y0, o), ot = __shfl_sync(0xffffffffu, ty, o);
+            const float oey = __shfl_sync(0xffffffffu, ey0, o), oet = __shfl_sync(0xffffffffu, ety, o);
+            const int on = __shfl_sync(0xffffffffu, nuv, o);
+            short dj = (short)__shfl_sync(0xffffffffu, (int)stj.det, o);
+            float pj = __shfl_sync(0xffffffffu, stj.pos, o), drj = __shfl_sync(0xffffffffu, stj.drift, o);
+            if (in) {
+                const YzHit &hi = base[uv_off(V, i)];
+                if (i + 1 < on) {
+                    const YzHit &hj = base[uv_off(V, i + 1)];
+                    dj = hj.det;
+                    pj = hj.pos;
+                    drj = hj.drift;
+                }
+                D.res[it] = (signed char)lr_pair_newhits(x0, tx, oy, ot, ex0, etx, oey, oet, hi.det, dj, hi.pos,
+                                                         hi.drift, pj, drj, P, 150.f);
+            }
+        }
+        __syncwarp();
+    }
+    bool xok = false;
+    short xval = 0;
+    for (unsigned m = pm; m; m &= m - 1) {
+        const int i = __ffs(m) - 1, k = D.res[lane << 3 | i];
+        if (k < 0) continue;
+        uv_set_sign(U, i, c_lrpossibility[k][0]);
+        if (i + 1 < nuv) uv_set_sign(U, i + 1, c_lrpossibility[k][1]);
+        // the cross pair: the last station-3 hit with the first station-2 hit
+        if (!is_first && i == n3 - 1 && i + 1 < nuv) {
+            xok = true;
+            xval = c_lrpossibility[k][0];
+        }
+    }
+    {
+        unsigned single = 0u;
+        if (valid)
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (k < nuv && !uv_sign(U, k)) single |= 1u << k;
+        __syncwarp();  // every lane has read its results
+        const int tot = deal(single);
+#pragma unroll 1
+        for (int t0 = 0; t0 < tot; t0 += 32) {
+            const bool in = t0 + lane < tot;
+            const int it = in ? D.item[t0 + lane] : 0, o = it >> 3, i = it & 7;
+            const UvSet V = shfl_set(o);
+            const float oy = __shfl_sync(0xffffffffu, y0, o), ot = __shfl_sync(0xffffffffu, ty, o);
+            if (in) {
+                const YzHit &h = base[uv_off(V, i)];
+                D.res[it] = (signed char)single_sign_newhits(x0, tx, oy, ot, h.det, h.pos, P);
+            }
+        }
+        __syncwarp();
+        for (; single; single &= single - 1) {
+            const int k = __ffs(single) - 1;
+            uv_set_sign(U, k, D.res[lane << 3 | k]);
+        }
     }
     short sig[4];
 #pragma unroll
@@ -1152,20 +1195,6 @@ __device__ __noinline__ void yz_phase2(YzWarp &S, const YzEvent &E, const YzHit 
         const short mine = (k < n3) ? uv_sign(U, k) : (short)0;
         const short v = (short)__shfl_sync(0xffffffffu, (int)mine, fl < 0 ? 0 : fl);
         sig[k] = carried_f ? cs.sig[k] : v;
-    }
-    bool xok = false;
-    short xval = 0;
-    if (valid && !is_first) {
-        const int xi = cross_pair_index(n3, U, base, nuv);
-        if (xi >= 0) {
-            const YzHit &ha = base[uv_off(U, xi)], &hb = base[uv_off(U, xi + 1)];
-            const int k = lr_pair_newhits_ool(x0, tx, y0, ty, ex0, etx, ey0, ety, ha.det, hb.det, ha.pos, ha.drift,
-                                              hb.pos, hb.drift, P, 150.f);
-            if (k >= 0) {
-                xok = true;
-                xval = c_lrpossibility[k][0];
-            }
-        }
     }
     const unsigned xm = __ballot_sync(0xffffffffu, xok);
     const int xs = last_lane(xm & seg & lanemask_lt());
@@ -1187,7 +1216,38 @@ __device__ __noinline__ void yz_phase2(YzWarp &S, const YzEvent &E, const YzHit 
     }
     if (valid) {
         pass = GATED ? gated : yz_gates(E, P, x0, y0, tx, ty, ex0, ey0, etx, ety);
-        if (pass) chi2 = yz_chi2(S, U, base, nuv, nhx, P, x0, y0, tx, ty);
+    }
+    // chi2_track over the x hits and the uv hits (H:1182-1204): the terms of
+    // the passing survivors dealt to the lanes, 16 survivors at a time; each
+    // survivor adds its own in order
+    {
+        const unsigned passm = __ballot_sync(0xffffffffu, pass);
+        const int rank = __popc(passm & lanemask_lt()), np = __popc(passm);
+        if (pass) D.item[rank] = (unsigned char)lane;
+        __syncwarp();
+#pragma unroll 1
+        for (int g0 = 0; g0 < np; g0 += 16) {
+            const int tot = min(16, np - g0) * 12;
+#pragma unroll 1
+            for (int t0 = 0; t0 < tot; t0 += 32) {
+                const int t = t0 + lane;
+                const int o = t < tot ? D.item[g0 + t / 12] : 0, m = t % 12;
+                UvSet V = shfl_set(o);
+                V.sign = __shfl_sync(0xffffffffu, U.sign, o);
+                const float oy = __shfl_sync(0xffffffffu, y0, o), ot = __shfl_sync(0xffffffffu, ty, o);
+                const int on = __shfl_sync(0xffffffffu, nuv, o);
+                if (t < tot && m < nhx + on) {
+                    float res;
+                    const float r = yz_residual(S, V, base, m, nhx, P, x0, oy, tx, ot, res);
+                    D.term[t] = r * r / res / res;
+                }
+            }
+            __syncwarp();
+            if (pass && rank >= g0 && rank < g0 + 16)
+#pragma unroll 1
+                for (int m = 0; m < nhx + nuv; ++m) chi2 += D.term[(rank - g0) * 12 + m];
+            __syncwarp();
+        }
     }
     // carry of the sign state to the next survivor chunk
     {
@@ -1234,22 +1294,25 @@ __device__ __noinline__ void yz_phase2(YzWarp &S, const YzEvent &E, const YzHit 
                 S.b.y0 = y0;
                 S.b.ety = ety;
                 S.b.ey0 = ey0;
-#pragma unroll 1
-                for (int n = 0; n < nuv; ++n) {
-                    const YzHit &h = base[uv_off(U, n)];
-                    S.b.det[n] = h.det;
-                    S.b.el[n] = h.el;
-                    S.b.pos[n] = h.pos;
-                    S.b.drift[n] = h.drift;
-                    S.b.sign[n] = uv_sign(U, n);
-                    S.b.tdc[n] = h.tdc;
-                }
-                // the winner's residuals, recomputed as chi2 formed them
-#pragma unroll 1
-                for (int n = 0; n < nhx + nuv; ++n) {
-                    float res;
-                    S.b.res[n] = yz_residual(S, U, base, n, nhx, P, x0, y0, tx, ty, res);
-                }
+            }
+            UvSet V = shfl_set(win);
+            V.sign = __shfl_sync(0xffffffffu, U.sign, win);
+            const float wy = __shfl_sync(0xffffffffu, y0, win), wt = __shfl_sync(0xffffffffu, ty, win);
+            const int wn = __shfl_sync(0xffffffffu, nuv, win);
+            if (lane < wn) {
+                const int n = lane;
+                const YzHit &h = base[uv_off(V, n)];
+                S.b.det[n] = h.det;
+                S.b.el[n] = h.el;
+                S.b.pos[n] = h.pos;
+                S.b.drift[n] = h.drift;
+                S.b.sign[n] = uv_sign(V, n);
+                S.b.tdc[n] = h.tdc;
+            }
+            // the winner's residuals, recomputed as chi2 formed them
+            if (lane < nhx + wn) {
+                float res;
+                S.b.res[lane] = yz_residual(S, V, base, lane, nhx, P, x0, wy, tx, wt, res);
             }
         }
     }
