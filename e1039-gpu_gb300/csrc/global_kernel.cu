@@ -1008,13 +1008,17 @@ __global__ void __launch_bounds__(W * 32, (OR_GL_WARPS_SM / W > 0 ? OR_GL_WARPS_
         for (int c = 1; c < GL_CLASSES; ++c) end[c] = end[c - 1] + sched[1 + c];
     }
     const unsigned long long nunits = end[GL_CLASSES - 1];
-    // the next slot is taken while the current one is worked on
-    unsigned long long nxt = 0;
-    if (lane == 0) nxt = atomicAdd(sched, 1ull);
+    // the next slot is taken while the current one is worked on; with no more
+    // slots than warps each warp has its own (one taken ahead would wait while
+    // other warps are idle)
+    const bool own = nunits <= (unsigned long long)gridDim.x * W;
+    unsigned long long nxt = own ? (unsigned long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x : 0ull;
+    if (!own && lane == 0) nxt = atomicAdd(sched, 1ull);
     for (;;) {
         unsigned long long u = __shfl_sync(0xffffffffu, nxt, 0);
         if (u >= nunits) break;
-        if (lane == 0) nxt = atomicAdd(sched, 1ull);
+        nxt = nunits;
+        if (!own && lane == 0) nxt = atomicAdd(sched, 1ull);
         if (list) {
             int c = 0;
 #pragma unroll

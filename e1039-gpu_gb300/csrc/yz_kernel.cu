@@ -1927,6 +1927,8 @@ struct YzInner {
     int first_two;        // first u2 pair with two accepted hits
 };
 
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 __device__ __forceinline__ bool yz_img_acc(const uint4 *hits, int off) { return hits[2 * off + 1].w != 0u; }
 
 // List the pairs of projection q with an accepted hit, in order; returns
@@ -2061,11 +2063,15 @@ __device__ __forceinline__ unsigned yz_first_event(YzFirstWarp &S, const or_hits
         }
     }
     __syncwarp();
+    float v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = lane < min(S.pp[q].n, YZ_PROP_SMEM) ? S.pp[q].pos(lane) : 0.f;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int n = min(S.pp[q].n, YZ_PROP_SMEM);
+        if (lane < n) S.prop[q][lane] = v[q];
 #pragma unroll 1
-        for (int i = lane; i < n; i += 32) S.prop[q][i] = S.pp[q].pos(i);
+        for (int i = lane + 32; i < n; i += 32) S.prop[q][i] = S.pp[q].pos(i);
     }
     return __ballot_sync(0xffffffffu, has) >> 4;
 }
@@ -2426,13 +2432,16 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_PLAN_WARPS_SM / W > 0 ? OR_YZ_P
     const unsigned nlarge = sc.list ? sc.counters[6] : 0u;
     const unsigned long long nplan = sc.list ? (unsigned long long)nlarge + sc.counters[7] : nall;
     unsigned long long *plan_ctr = reinterpret_cast<unsigned long long *>(sc.counters + 4);
-    // the next unit is taken while the current one is worked on
-    unsigned long long nxt = 0;
-    if (lane == 0) nxt = atomicAdd(plan_ctr, 1ull);
+    // the next unit is taken while the current one is worked on; with no more
+    // units than warps each warp has its own
+    const bool own = nplan <= (unsigned long long)gridDim.x * W;
+    unsigned long long nxt = own ? (unsigned long long)w * gridDim.x + blockIdx.x : 0ull;
+    if (!own && lane == 0) nxt = atomicAdd(plan_ctr, 1ull);
     for (;;) {
         const unsigned long long pt = __shfl_sync(0xffffffffu, nxt, 0);
         if (pt >= nplan) break;
-        if (lane == 0) nxt = atomicAdd(plan_ctr, 1ull);
+        nxt = nplan;
+        if (!own && lane == 0) nxt = atomicAdd(plan_ctr, 1ull);
         const unsigned long long pu =
             sc.list ? (unsigned long long)sc.list[pt < nlarge ? pt : nall - 1 - (pt - nlarge)] : pt;
         const long e = (long)(pu / per_event);
@@ -2706,28 +2715,47 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_FIRST_WARPS_SM / W > 0 ? OR_YZ_
     unsigned long long *pool_ctr = reinterpret_cast<unsigned long long *>(sc.counters + 8);
     const int nunits = min((int)sc.counters[0], sc.cap_units);
     unsigned long long n_surv = 0ull;
-    // the next unit is taken while the current one is worked on
-    int nxt = 0;
-    if (lane == 0) nxt = (int)atomicAdd(&sc.counters[2], 1u);
-    for (;;) {
-        const int u = __shfl_sync(0xffffffffu, nxt, 0);
-        if (u >= nunits) break;
-        if (lane == 0) nxt = (int)atomicAdd(&sc.counters[2], 1u);
-        const int heavy = sc.units[u].heavy;
-        const int r0 = sc.units[u].r0, r1 = sc.units[u].r1;
-        if (heavy < 0) continue;
-        const YzHeavy hv2 = sc.heavy[heavy];
+    // The next unit is taken while the current one is worked on, and read
+    // before that is done; with no more units than warps each warp has its
+    // own (a unit taken ahead would wait while other warps are idle).
+    const bool own = nunits <= (int)gridDim.x * W;
+    int nxt = own ? w * (int)gridDim.x + (int)blockIdx.x : 0;
+    if (!own && lane == 0) nxt = (int)atomicAdd(&sc.counters[2], 1u);
+    int u = __shfl_sync(0xffffffffu, nxt, 0);
+    int heavy = -1, r0 = 0, r1 = 0;
+    auto read_unit = [&](int i) {
+        if (i >= nunits) return;
+        heavy = sc.units[i].heavy;
+        r0 = sc.units[i].r0;
+        r1 = sc.units[i].r1;
+    };
+    read_unit(u);
+    while (u < nunits) {
+        const int cu = u, cheavy = heavy, c0 = r0, c1 = r1;
+        nxt = nunits;
+        if (!own && lane == 0) nxt = (int)atomicAdd(&sc.counters[2], 1u);
+        if (cheavy < 0) {
+            u = __shfl_sync(0xffffffffu, nxt, 0);
+            read_unit(u);
+            continue;
+        }
+        const YzHeavy hv2 = sc.heavy[cheavy];
         const int st3 = 3 + (hv2.slot & 1);
         const YzTab *tab = sc.tab + YZ_TAB_SETS * (st3 - 3);
         int ns = -1, count = 0;  // -1: the unit runs on the combined path (survivor kernel)
         __syncwarp();            // every lane is done with the previous unit's state
-        if (hv2.img >= 0) {
+        if (hv2.img < 0) {
+            u = __shfl_sync(0xffffffffu, nxt, 0);
+            read_unit(u);
+        } else {
             const uint4 *img = sc.img + hv2.img;
             const YzImgHead &h = *reinterpret_cast<const YzImgHead *>(img);
             const int total = h.total;
             if (lane < 4) S.np[lane] = h.np[lane];
             if (lane < 8) S.woff[lane] = h.woff[lane];
             const unsigned hasx = yz_first_event(S, hv, hv2.e, G, gplane, h.x0, h.tx, h.ex0, h.etx);
+            u = __shfl_sync(0xffffffffu, nxt, 0);
+            read_unit(u);
             __syncwarp();
             // a station without a hodoscope hit in the x window closes the
             // gates for every combination
@@ -2749,6 +2777,22 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_FIRST_WARPS_SM / W > 0 ? OR_YZ_
                 YzLast last;
                 int first_two;
                 const short2 *pq = pair;
+                {
+                    // the hits of all four lists' first pairs are on their way
+                    // to L1 before the first list is made
+                    short2 pp[4];
+                    int at = 0;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        pp[q] = lane < S.np[q] ? pair[at + lane] : make_short2(-1, -1);
+                        at += S.np[q];
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if (pp[q].x >= 0) prefetch_l1(I.hits + 2 * (S.woff[2 * q] + pp[q].x));
+                        if (pp[q].y >= 0) prefetch_l1(I.hits + 2 * (S.woff[2 * q + 1] + pp[q].y));
+                    }
+                }
 #pragma unroll 1
                 for (int q = 0; q < 4; ++q) {
                     const int n = yz_first_list(S, q, pq, I.hits, term + q * cap, info + q * cap, last, first_two);
@@ -2786,7 +2830,7 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_FIRST_WARPS_SM / W > 0 ? OR_YZ_
                 } else {
                     const unsigned long long lasto = yz_lasto(S.np[0], S.np[1], I.u, I.v, second, rel0);
                     const float *osc = PRUNE ? yz_tracklet_scores(prune, hv2) : nullptr;
-                    ns = yz_first_walk<PRUNE>(S, G, hasx, term, info, cap, na, I, lasto, r0, r1, st3 == 3, tab, Q, qcap,
+                    ns = yz_first_walk<PRUNE>(S, G, hasx, term, info, cap, na, I, lasto, c0, c1, st3 == 3, tab, Q, qcap,
                                               osc, prune.t_keep, &count);
                 }
             }
@@ -2805,7 +2849,7 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_FIRST_WARPS_SM / W > 0 ? OR_YZ_
 #pragma unroll 1
             for (int i = lane; i < ns; i += 32) dst[i] = src[i];
         }
-        if (lane == 0) sc.useg[u] = make_int2(off >= 0 ? (int)off : -1, off >= 0 ? ns : 0);
+        if (lane == 0) sc.useg[cu] = make_int2(off >= 0 ? (int)off : -1, off >= 0 ? ns : 0);
         __syncwarp();
     }
     if (lane == 0 && sc.count_work) yz_flush_counts(sc, 0ull, 0ull, n_surv);
@@ -2836,10 +2880,16 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_SECOND_WARPS_SM / W > 0 ? OR_YZ
     if (lane == 0) S.nsurv = 0ull;
     __syncwarp();
     const int nunits = min((int)sc.counters[0], sc.cap_units);
-    for (;;) {
-        int u = 0;
-        if (lane == 0) u = (int)atomicAdd(&sc.counters[3], 1u);
-        u = __shfl_sync(0xffffffffu, u, 0);
+    // with no more units than warps each warp has its own (taking one ahead,
+    // as the first kernel does, is no gain here: 10,000 dimuon events 218 ->
+    // 228 us)
+    const bool own = nunits <= (int)gridDim.x * W;
+    for (int mine = own ? w * (int)gridDim.x + (int)blockIdx.x : 0;; mine = nunits) {
+        int u = mine;
+        if (!own) {
+            if (lane == 0) u = (int)atomicAdd(&sc.counters[3], 1u);
+            u = __shfl_sync(0xffffffffu, u, 0);
+        }
         if (u >= nunits) break;
         const YzUnit un = sc.units[u];
         if (un.heavy < 0) continue;
