@@ -12,11 +12,11 @@
 #include "or_device.cuh"
 
 namespace orgpu {
-cudaError_t launch_event_reduce(or_hits_view_t, uint8_t *, int, uint32_t *, cudaStream_t, int, int);
+cudaError_t launch_event_reduce(or_hits_view_t, uint8_t *, int, uint32_t *, cudaStream_t, int, int, ChainClear);
 cudaError_t launch_xz(const or_plane_t *, or_hits_view_t, or_tracks_view_t, int32_t *, uint8_t *, int, cudaStream_t,
                       int, int);
 cudaError_t launch_yz_tuned(const or_plane_t *, or_hits_view_t, or_tracks_view_t, const uint8_t *, int, uint32_t *,
-                            void *, int, int, int, cudaStream_t, int, int, long long, int);
+                            void *, int, int, int, cudaStream_t, int, int, long long, int, bool);
 cudaError_t launch_yz(const or_plane_t *, or_hits_view_t, or_tracks_view_t, const uint8_t *, int, uint32_t *, void *,
                       int, int, int, cudaStream_t, int);
 size_t yz_scratch_bytes_ctx(int, int, int);
@@ -30,7 +30,7 @@ cudaError_t launch_histograms(or_tracks_view_t, or_dimuons_view_t, const int32_t
                               int, cudaStream_t, int);
 cudaError_t launch_back_clean(or_tracks_view_t, const uint8_t *, int, cudaStream_t, int, int);
 cudaError_t launch_global(const or_plane_t *, or_hits_view_t, or_tracks_view_t, const uint8_t *, int, uint32_t *,
-                          unsigned long long *, int, cudaStream_t, int, int);
+                          unsigned long long *, int, cudaStream_t, int, int, bool);
 size_t global_sched_bytes(int);
 cudaError_t launch_pack(const or_hit_record_t *, const int64_t *, int, const float *, const or_rt_table_t *,
                         or_hits_view_t, uint32_t *, cudaStream_t, int);
@@ -305,14 +305,19 @@ int or_selftest_bounded_wait(or_ctx_t *ctx, int polls, void *stream) {
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "wait self-test launch");
 }
 
-int or_event_reduce(or_ctx_t *ctx, or_hits_view_t hits, uint8_t *toomany, int n_events, void *stream) {
+static int event_reduce(or_ctx_t *ctx, or_hits_view_t hits, uint8_t *toomany, int n_events, void *stream,
+                        orgpu::ChainClear clear) {
     int rc = check_ctx(ctx, false);
     if (rc) return rc;
     if (n_events < 0 || !toomany) return fail(OR_ERR_ARG, "bad event count or flag array");
     if ((rc = check_hits(hits))) return rc;
     cudaError_t e = orgpu::launch_event_reduce(hits, toomany, n_events, ctx->d_errw, S(stream), ctx->sm_count,
-                                               ctx->warps[OR_K_EVENT_REDUCE]);
+                                               ctx->warps[OR_K_EVENT_REDUCE], clear);
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "event reducer launch");
+}
+
+int or_event_reduce(or_ctx_t *ctx, or_hits_view_t hits, uint8_t *toomany, int n_events, void *stream) {
+    return event_reduce(ctx, hits, toomany, n_events, stream, {});
 }
 
 int or_xz(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, int32_t *ntracklets, uint8_t *toomany,
@@ -327,8 +332,9 @@ int or_xz(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, int32_t *
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "XZ launch");
 }
 
-int or_yz(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, const uint8_t *toomany, int n_events,
-          void *stream) {
+// `cleared`: the stage's counters are zero already (ChainClear)
+static int yz_tracking(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, const uint8_t *toomany,
+                       int n_events, void *stream, bool cleared) {
     int rc = check_ctx(ctx, true);
     if (rc) return rc;
     if (n_events < 0 || !toomany) return fail(OR_ERR_ARG, "bad event count or flag array");
@@ -336,8 +342,13 @@ int or_yz(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, const uin
     cudaError_t e = orgpu::launch_yz_tuned(ctx->d_plane, hits, tracks, toomany, n_events, ctx->d_errw,
                                            ctx->yz_scratch, ctx->yz_cap_units, ctx->yz_cap_heavy,
                                            ctx->yz_garena_warps, S(stream), ctx->sm_count, ctx->warps[OR_K_YZ],
-                                           ctx->yz_pool_limit, ctx->yz_count_work);
+                                           ctx->yz_pool_limit, ctx->yz_count_work, cleared);
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "YZ launch");
+}
+
+int or_yz(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, const uint8_t *toomany, int n_events,
+          void *stream) {
+    return yz_tracking(ctx, hits, tracks, toomany, n_events, stream, false);
 }
 
 int or_yz_scored(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, const uint8_t *toomany, int n_events,
@@ -439,16 +450,21 @@ int or_back_clean(or_ctx_t *ctx, or_tracks_view_t tracks, const uint8_t *toomany
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "cleaning launch");
 }
 
-int or_global(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, const uint8_t *toomany, int n_events,
-              void *stream) {
+static int global_tracking(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, const uint8_t *toomany,
+                           int n_events, void *stream, bool cleared) {
     int rc = check_ctx(ctx, true);
     if (rc) return rc;
     if (n_events < 0 || !toomany) return fail(OR_ERR_ARG, "bad event count or flag array");
     if ((rc = check_hits(hits)) || (rc = check_tracks(tracks))) return rc;
     cudaError_t e =
         orgpu::launch_global(ctx->d_plane, hits, tracks, toomany, n_events, ctx->d_errw, ctx->d_sched,
-                             ctx->sched_slots, S(stream), ctx->sm_count, ctx->warps[OR_K_GLOBAL]);
+                             ctx->sched_slots, S(stream), ctx->sm_count, ctx->warps[OR_K_GLOBAL], cleared);
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "global tracking launch");
+}
+
+int or_global(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, const uint8_t *toomany, int n_events,
+              void *stream) {
+    return global_tracking(ctx, hits, tracks, toomany, n_events, stream, false);
 }
 
 int or_run_batch(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, int32_t *ntracklets,
@@ -457,13 +473,13 @@ int or_run_batch(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, in
     if (rc) return rc;
     if (n_events < 0 || !toomany || !ntracklets) return fail(OR_ERR_ARG, "bad event count or output arrays");
     if ((rc = check_hits(hits)) || (rc = check_tracks(tracks))) return rc;
-    cudaError_t e = cudaMemsetAsync(ntracklets, 0, sizeof(int32_t) * (size_t)n_events, S(stream));
-    if (e != cudaSuccess) return cuda_fail(e, "clear tracklet counts");
-    if ((rc = or_event_reduce(ctx, hits, toomany, n_events, stream))) return rc;
+    const orgpu::ChainClear clear{
+        ntracklets, {static_cast<uint32_t *>(ctx->yz_scratch), reinterpret_cast<uint32_t *>(ctx->d_sched)}};
+    if ((rc = event_reduce(ctx, hits, toomany, n_events, stream, clear))) return rc;
     if ((rc = or_xz(ctx, hits, tracks, ntracklets, toomany, n_events, stream))) return rc;
-    if ((rc = or_yz(ctx, hits, tracks, toomany, n_events, stream))) return rc;
+    if ((rc = yz_tracking(ctx, hits, tracks, toomany, n_events, stream, true))) return rc;
     if ((rc = or_back_clean(ctx, tracks, toomany, n_events, stream))) return rc;
-    return or_global(ctx, hits, tracks, toomany, n_events, stream);
+    return global_tracking(ctx, hits, tracks, toomany, n_events, stream, true);
 }
 
 /* ---- post-global selection ---------------------------------------------- */
@@ -884,7 +900,7 @@ extern "C" int or_gKernel_YZ_tracking(gEventHitCollections *hitcolls, gEventTrac
         reinterpret_cast<const or_plane_t *>(planes), or_hits_view_from_collection(hitcolls),
         or_tracks_view_from_collection(tklcoll), reinterpret_cast<const uint8_t *>(hastoomanyhits), OR_REF_EVTMAX,
         ctx->d_errw, ctx->yz_scratch, ctx->yz_cap_units, ctx->yz_cap_heavy, ctx->yz_garena_warps, nullptr,
-        ctx->sm_count, ctx->warps[OR_K_YZ], ctx->yz_pool_limit, 0);
+        ctx->sm_count, ctx->warps[OR_K_YZ], ctx->yz_pool_limit, 0, false);
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "or_gKernel_YZ_tracking launch");
 }
 
@@ -909,7 +925,7 @@ extern "C" int or_gKernel_Global_tracking(gEventHitCollections *hitcolls, gEvent
                                                or_tracks_view_from_collection(tklcoll),
                                                reinterpret_cast<const uint8_t *>(hastoomanyhits), OR_REF_EVTMAX,
                                                ctx->d_errw, ctx->d_sched, ctx->sched_slots, nullptr, ctx->sm_count,
-                                               ctx->warps[OR_K_GLOBAL]);
+                                               ctx->warps[OR_K_GLOBAL], false);
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "or_gKernel_Global_tracking launch");
 }
 

@@ -105,7 +105,9 @@ __global__ void __launch_bounds__(CO_THREADS)
         }
         const int all = __shfl_sync(0xffffffffu, incl, 31);
         unsigned long long b = 0ull;
-        if (lane == 0 && all) b = atomicAdd(cursor, (unsigned long long)all);
+        // a single cluster's count is the batch's
+        if (lane == 0 && n_events <= CO_EVENTS) *cursor = (unsigned long long)all;
+        else if (lane == 0 && all) b = atomicAdd(cursor, (unsigned long long)all);
         b = __shfl_sync(0xffffffffu, b, 0);
         if (lane < nb) *cluster.map_shared_rank(&base, lane) = b + (unsigned)(incl - v);
     }
@@ -153,8 +155,9 @@ __global__ void __launch_bounds__(CO_THREADS)
 cudaError_t launch_collect(or_tracks_view_t tv, const uint8_t *toomany, int n_events, float stid, float *out,
                            long long capacity, unsigned long long *cursor, cudaStream_t stream, int sm_count) {
     if (n_events <= 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), stream);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
+    if (n_events > CO_EVENTS && (e = cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), stream)) != cudaSuccess)
+        return e;
     const long groups = ((long)n_events + CO_EVENTS - 1) / CO_EVENTS;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(CO_THREADS);

@@ -319,7 +319,7 @@ static __device__ __forceinline__ int er_reduce(ErWarp &S, int p0, int p1, int h
 
 template <int W>
 __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *__restrict__ toomany, int n_events,
-                                                    uint32_t *__restrict__ errw) {
+                                                    uint32_t *__restrict__ errw, ChainClear clear) {
     extern __shared__ __align__(16) unsigned char er_smem[];
     ErWarp *sm = reinterpret_cast<ErWarp *>(er_smem);
     const int w = threadIdx.x >> 5;
@@ -328,6 +328,11 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
     if (lane == 0) mbar_init(&S.bar, 1);
     __syncwarp();
     uint32_t phase = 0;
+    if (blockIdx.x == 0 && w == 0)
+        for (int i = lane; i < 64; i += 32)
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+                if (clear.counters[b]) clear.counters[b][i] = 0u;
 
     for (long e = (long)blockIdx.x * W + w; e < n_events; e += (long)gridDim.x * W) {
         for (int p = lane; p < ER_NPLANES; p += 32) {
@@ -417,7 +422,10 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
 #pragma unroll
             for (int k = 0; k < 6; ++k) sum += __shfl_sync(0xffffffffu, m, min(31, st * 6 + k));
             const bool over = __any_sync(0xffffffffu, lane < ER_NCHAMBERS && sum > lim);
-            if (lane == 0) toomany[e] = (uint8_t)over;
+            if (lane == 0) {
+                toomany[e] = (uint8_t)over;
+                if (clear.ntracklets) clear.ntracklets[e] = 0;
+            }
         }
         __syncwarp();
     }
@@ -426,14 +434,14 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
 // Host launcher.
 template <int W>
 static cudaError_t er_launch(or_hits_view_t hv, uint8_t *toomany, int n_events, uint32_t *errw, cudaStream_t stream,
-                             int sm_count) {
+                             int sm_count, ChainClear clear) {
     const size_t smem = sizeof(ErWarp) * W;
     cudaError_t e = smem_attr_once((const void *)er_kernel<W>, (int)smem);
     if (e != cudaSuccess) return e;
     long blocks = (n_events + W - 1) / W;
     const long cap = (long)sm_count * (48 / W > 0 ? 48 / W : 1);  // up to 48 resident warps per SM
     if (blocks > cap) blocks = cap;
-    er_kernel<W><<<(unsigned)blocks, W * 32, smem, stream>>>(hv, toomany, n_events, errw);
+    er_kernel<W><<<(unsigned)blocks, W * 32, smem, stream>>>(hv, toomany, n_events, errw, clear);
     return cudaGetLastError();
 }
 
@@ -458,14 +466,14 @@ cudaError_t launch_wait_selftest(uint32_t *errw, uint32_t polls, cudaStream_t st
 
 // Host launcher; `warps` = events per CTA (1, 2, 4, 8 or 16).
 cudaError_t launch_event_reduce(or_hits_view_t hv, uint8_t *toomany, int n_events, uint32_t *errw,
-                                cudaStream_t stream, int sm_count, int warps) {
+                                cudaStream_t stream, int sm_count, int warps, ChainClear clear) {
     if (n_events <= 0) return cudaSuccess;
     switch (warps) {
-    case 1: return er_launch<1>(hv, toomany, n_events, errw, stream, sm_count);
-    case 2: return er_launch<2>(hv, toomany, n_events, errw, stream, sm_count);
-    case 8: return er_launch<8>(hv, toomany, n_events, errw, stream, sm_count);
-    case 16: return er_launch<16>(hv, toomany, n_events, errw, stream, sm_count);
-    default: return er_launch<4>(hv, toomany, n_events, errw, stream, sm_count);
+    case 1: return er_launch<1>(hv, toomany, n_events, errw, stream, sm_count, clear);
+    case 2: return er_launch<2>(hv, toomany, n_events, errw, stream, sm_count, clear);
+    case 8: return er_launch<8>(hv, toomany, n_events, errw, stream, sm_count, clear);
+    case 16: return er_launch<16>(hv, toomany, n_events, errw, stream, sm_count, clear);
+    default: return er_launch<4>(hv, toomany, n_events, errw, stream, sm_count, clear);
     }
 }
 

@@ -1056,11 +1056,12 @@ size_t global_sched_bytes(int list_cap) { return 256 + 2 * sizeof(unsigned) * (s
 template <int W>
 static cudaError_t global_launch(const or_plane_t *d_plane, or_hits_view_t hv, or_tracks_view_t tv,
                                  const uint8_t *toomany, int n_events, uint32_t *errw, unsigned long long *sched,
-                                 int list_cap, cudaStream_t stream, int sm_count) {
+                                 int list_cap, cudaStream_t stream, int sm_count, bool cleared) {
     const size_t smem = global_smem_bytes(W);
     cudaError_t err = smem_attr_once((const void *)global_kernel<W>, (int)smem);
     if (err != cudaSuccess) return err;
-    if ((err = cudaMemsetAsync(sched, 0, (1 + GL_CLASSES) * sizeof(unsigned long long), stream)) != cudaSuccess) return err;
+    if (!cleared && (err = cudaMemsetAsync(sched, 0, (1 + GL_CLASSES) * sizeof(unsigned long long), stream)) != cudaSuccess)
+        return err;
     const long nslots = (long)n_events * OR_NSLOTS;
     // the list saves an atomic per slot without a track; a batch beyond its
     // room visits every slot
@@ -1077,13 +1078,14 @@ static cudaError_t global_launch(const or_plane_t *d_plane, or_hits_view_t hv, o
     return cudaGetLastError();
 }
 
-// `warps` = slots in flight per CTA: 1, 2, 4, 8 or 16
+// `warps` = slots in flight per CTA: 1, 2, 4, 8 or 16; `cleared`: the counters
+// are zero already (ChainClear)
 cudaError_t launch_global(const or_plane_t *d_plane, or_hits_view_t hv, or_tracks_view_t tv, const uint8_t *toomany,
                           int n_events, uint32_t *errw, unsigned long long *sched, int list_cap, cudaStream_t stream,
-                          int sm_count, int warps) {
+                          int sm_count, int warps, bool cleared) {
     if (n_events <= 0) return cudaSuccess;
 #define OR_GL_LAUNCH(W) \
-    global_launch<W>(d_plane, hv, tv, toomany, n_events, errw, sched, list_cap, stream, sm_count)
+    global_launch<W>(d_plane, hv, tv, toomany, n_events, errw, sched, list_cap, stream, sm_count, cleared)
     switch (warps) {
     case 1: return OR_GL_LAUNCH(1);
     case 2: return OR_GL_LAUNCH(2);

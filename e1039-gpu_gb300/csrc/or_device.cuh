@@ -456,6 +456,14 @@ __device__ __forceinline__ void tma_load_1d(void *dst_smem, const void *src_gmem
         "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar))
         : "memory");
 }
+// What the event reducer clears for the stages of a whole-chain call, so that
+// the chain needs no memsets between its kernels (null: nothing): the
+// events' tracklet counts and two 256-byte blocks of counters.
+struct ChainClear {
+    int32_t *ntracklets;
+    uint32_t *counters[2];
+};
+
 // Bounded wait for phase `parity` of `bar`; false when the limit ran out.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, uint32_t max_iter) {
     const uint32_t a = smem_u32(bar);

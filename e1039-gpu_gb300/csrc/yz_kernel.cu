@@ -3252,7 +3252,7 @@ template <int W>
 static cudaError_t launch_yz_impl(const or_plane_t *d_plane, or_hits_view_t hv, or_tracks_view_t tv,
                                   const uint8_t *toomany, int n_events, uint32_t *errw, void *scratch, int cap_units,
                                   int cap_heavy, int garena_warps, cudaStream_t stream, int sm_count, YzPrune prune,
-                                  int qcap, long long pool_limit, int count_work) {
+                                  int qcap, long long pool_limit, int count_work, bool cleared) {
     if (n_events <= 0) return cudaSuccess;
     const size_t smem = yz_smem_bytes(W);
     cudaError_t err;
@@ -3267,7 +3267,7 @@ static cudaError_t launch_yz_impl(const or_plane_t *d_plane, or_hits_view_t hv, 
     YzScratch sc = yz_scratch_layout(scratch, cap_units, cap_heavy, garena_warps, qcap, pool_limit);
     YzTab *tab = const_cast<YzTab *>(sc.tab);
     sc.count_work = count_work;
-    if ((err = cudaMemsetAsync(sc.counters, 0, 256, stream))) return err;
+    if (!cleared && (err = cudaMemsetAsync(sc.counters, 0, 256, stream))) return err;
     // One slot per planning unit: a heavy event's tracklets spread over 32
     // warps (a single uneven event's planning pass 442 -> 59 us, 333 of them
     // 619 -> 107 us, 100,000 12.6 -> 11.8 ms).  With the combination scorer
@@ -3332,10 +3332,10 @@ static cudaError_t launch_yz_impl(const or_plane_t *d_plane, or_hits_view_t hv, 
 static cudaError_t launch_yz_w(const or_plane_t *d_plane, or_hits_view_t hv, or_tracks_view_t tv,
                                const uint8_t *toomany, int n_events, uint32_t *errw, void *scratch, int cap_units,
                                int cap_heavy, int garena_warps, cudaStream_t stream, int sm_count, YzPrune prune,
-                               int warps, int qcap, long long pool_limit, int count_work) {
+                               int warps, int qcap, long long pool_limit, int count_work, bool cleared = false) {
 #define OR_YZ_LAUNCH(W)                                                                                         \
     launch_yz_impl<W>(d_plane, hv, tv, toomany, n_events, errw, scratch, cap_units, cap_heavy, garena_warps, stream, \
-                      sm_count, prune, qcap, pool_limit, count_work)
+                      sm_count, prune, qcap, pool_limit, count_work, cleared)
     switch (warps) {
     case 1: return OR_YZ_LAUNCH(1);
     case 2: return OR_YZ_LAUNCH(2);
@@ -3357,9 +3357,9 @@ cudaError_t launch_yz(const or_plane_t *d_plane, or_hits_view_t hv, or_tracks_vi
 cudaError_t launch_yz_tuned(const or_plane_t *d_plane, or_hits_view_t hv, or_tracks_view_t tv,
                             const uint8_t *toomany, int n_events, uint32_t *errw, void *scratch, int cap_units,
                             int cap_heavy, int garena_warps, cudaStream_t stream, int sm_count, int warps,
-                            long long pool_limit, int count_work) {
+                            long long pool_limit, int count_work, bool cleared) {
     return launch_yz_w(d_plane, hv, tv, toomany, n_events, errw, scratch, cap_units, cap_heavy, garena_warps, stream,
-                       sm_count, YzPrune{}, warps, YZ_QCAP_CTX, pool_limit, count_work);
+                       sm_count, YzPrune{}, warps, YZ_QCAP_CTX, pool_limit, count_work, cleared);
 }
 
 // YZ with the scorer's keep flags: pruned tracklets are left as tracklets no
