@@ -244,11 +244,16 @@ class Trainer:
     def epoch(self, rng):
         """One pass over the rows in a random order; returns the mean batch loss."""
         torch = _torch()
-        perm = torch.from_numpy(rng.permutation(self.n).astype(np.int64)).to(self.dev)
-        total = torch.zeros((), dtype=torch.float32, device=self.dev)
-        nb = 0
-        for s in range(0, self.n - self.batch + 1, self.batch):
-            idx = perm[s:s + self.batch]
+        perm = torch.from_numpy(rng.permutation(self.n).astype(np.int64, copy=False)).to(self.dev)
+        nb = self.n // self.batch
+        if nb == 0:
+            return 0.0
+        # a row of block losses per batch, added up once (adding them up batch
+        # by batch took two launches each)
+        losses = torch.empty(nb, self.nblk, dtype=torch.float32, device=self.dev)
+        for b in range(nb):
+            idx = perm[b * self.batch:(b + 1) * self.batch]
+            self.loss = losses[b]
             _lib.check(self.lib.or_mlp_gradient(self.ctx, self.model.ptr(), self.features.data_ptr(),
                                                 self.labels.data_ptr(), idx.data_ptr(), self.batch,
                                                 float(self.pos_weight), self.grad.data_ptr(), self.loss.data_ptr(),
@@ -257,9 +262,10 @@ class Trainer:
             _lib.check(self.lib.or_mlp_adam(self.ctx, self.param.data_ptr(), self.m1.data_ptr(), self.m2.data_ptr(),
                                             self.grad.data_ptr(), self.nblk, self.step_no, float(self.lr), 0.9, 0.999,
                                             1e-8, self.model.ptr(), self.stream), "or_mlp_adam")
-            total += self.loss.sum()
-            nb += 1
-        return float(total.item()) / max(nb, 1)
+        total = np.float32(0)
+        for x in losses.sum(1).cpu().numpy():
+            total += x
+        return float(total) / nb
 
     def result(self):
         return ScorerParams(self.param.cpu().numpy(), self.sp.mean, self.sp.inv_std, self.sp.t_keep, self.sp.t_unc,
