@@ -34,7 +34,7 @@
 // and the serial chain of one slot's tracks on small batches.  Evaluating
 // each (u1, v1) combination with its hits' acceptance and the scratch
 // entries' scan, 32 of one x1 pair at a time, took 13.7 ms for 100,000 uneven
-// events and 1,223 us for 333 of them; this takes 9.2 ms and 400 us (11.8 ms
+// events and 1,223 us for 333 of them; this takes 8.4 ms and 385 us (11.8 ms
 // with the windows and pairs walked plane by plane).
 #include "window_pairs.cuh"
 

@@ -19,12 +19,13 @@
 //     the same slot.
 // Work per event is heavily skewed (a few events hold most combinations),
 // so the GPU version splits it:
-//   yz_plan_kernel   one warp per event walks its slots and tracklets in
-//                    order; builds each tracklet's hit windows once (y, error
-//                    and acceptance of every windowed hit for this tracklet);
-//                    evaluates light tracklets itself, and cuts heavy ones
-//                    into units of whole (u3,v3) iterations on a device queue,
-//                    storing each one's windows as an image;
+//   yz_plan_kernel   a warp per slot (per eight slots with the combination
+//                    scorer's rows) walks its tracklets in order; builds each
+//                    one's hit windows once (y, error and acceptance of every
+//                    windowed hit for this tracklet) and cuts it into units
+//                    of whole (u3,v3) iterations on a device queue, storing
+//                    its windows as an image; with the scorer's rows it
+//                    evaluates light tracklets itself;
 //   yz_first_kernel  persistent warps (28 per SM, 72 registers) drain the
 //                    queue with the first cut (fit of the station-3 and
 //                    station-2 y hits, 2-sigma cut) and the prop-tube and
@@ -1892,7 +1893,7 @@ __device__ unsigned long long yz_range_t(YzWarp &S, const YzEvent &E, const YzHi
 // Bound: instruction issue.  Rebuilding each combination's station-3 part and
 // attempts, scanning the scratch entries over every chunk of 32 and passing
 // every survivor on took 22.9 ms of the 100,000-event uneven batch with 19.5
-// ms in the survivor kernel; this takes 9.2 ms with 8.3 ms.
+// ms in the survivor kernel; this takes 8.9 ms with 6.2 ms.
 constexpr int YZ_KEPT_BATCH = 32;  // outer iterations listed at a time
 constexpr int YZ_LIST_SMEM = 48;   // pairs per projection listed in shared memory; a unit with more uses the
                                    // warp's overflow arena
