@@ -28,6 +28,13 @@ __device__ __forceinline__ int plane_count(const or_hits_view_t &hv, long e, int
     return (int)hv.nhits_prop[e * OR_NPROP + det - OR_NCHAM - OR_NHODO - 1];
 }
 
+__device__ __forceinline__ const float *plane_slot(const or_hits_view_t &hv, long e, int det) {
+    if (det <= OR_NCHAM) return hv.hits_cham + e * OR_EVT_CHAM_FLOATS + (long)OR_NHITSPARAM * OR_MAXHITS_CHAM * (det - 1);
+    if (det <= OR_NCHAM + OR_NHODO)
+        return hv.hits_hodo + e * OR_EVT_HODO_FLOATS + (long)OR_NHITSPARAM * OR_MAXHITS_HODO * (det - OR_NCHAM - 1);
+    return hv.hits_prop + e * OR_EVT_PROP_FLOATS + (long)OR_NHITSPARAM * OR_MAXHITS_PROP * (det - OR_NCHAM - OR_NHODO - 1);
+}
+
 // the track's hit count as the host reads it (M:1138), within the record's 18
 __device__ __forceinline__ int track_nhits(const float *T) {
     return max(0, min((int)T[OR_TRK_NHITS], OR_MAXHITS_PER_TRACK));
@@ -68,8 +75,8 @@ __global__ void __launch_bounds__(256)
 // one block: exclusive offsets of every event's rows, totals into counts[5]
 __global__ void __launch_bounds__(1024)
     out_scan_kernel(const OutCount *__restrict__ cnt, int n_events, OutOffset *off, long long *counts) {
-    __shared__ long long part[5][1024];
-    const int t = threadIdx.x;
+    __shared__ long long part[5][32];  // before each warp's events
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const long per = ((long)n_events + blockDim.x - 1) / blockDim.x;
     const long e0 = min((long)n_events, t * per), e1 = min((long)n_events, e0 + per);
     long long s[5] = {0, 0, 0, 0, 0};
@@ -77,25 +84,35 @@ __global__ void __launch_bounds__(1024)
         const OutCount c = cnt[e];
         s[0] += c.acc; s[1] += c.hits; s[2] += c.tracks; s[3] += c.thits; s[4] += c.dims;
     }
-    for (int q = 0; q < 5; ++q) part[q][t] = s[q];
-    __syncthreads();
-    // inclusive scan of the per-thread sums (Hillis-Steele in shared memory)
-    for (int o = 1; o < (int)blockDim.x; o <<= 1) {
-        long long v[5];
-        for (int q = 0; q < 5; ++q) v[q] = t >= o ? part[q][t - o] : 0;
-        __syncthreads();
-        for (int q = 0; q < 5; ++q) part[q][t] += v[q];
-        __syncthreads();
-    }
+    auto scan = [&](long long v) {  // inclusive, over the lanes
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        return v;
+    };
     long long run[5];
-    for (int q = 0; q < 5; ++q) run[q] = part[q][t] - s[q];
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+        const long long v = scan(s[q]);
+        run[q] = v - s[q];
+        if (lane == 31) part[q][w] = v;
+    }
+    __syncthreads();
+    if (w < 5) {
+        const long long v = part[w][lane], incl = scan(v);
+        part[w][lane] = incl - v;
+        if (lane == 31) counts[w] = incl;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 5; ++q) run[q] += part[q][w];
     for (long e = e0; e < e1; ++e) {
         const OutCount c = cnt[e];
         off[e] = OutOffset{run[0], run[1], run[2], run[3], run[4]};
         run[0] += c.acc; run[1] += c.hits; run[2] += c.tracks; run[3] += c.thits; run[4] += c.dims;
     }
-    if (t == blockDim.x - 1)
-        for (int q = 0; q < 5; ++q) counts[q] = part[q][t];
 }
 
 __constant__ int c_dim_out_src[OR_OUT_DIMUON_FIELDS] = {
@@ -113,11 +130,23 @@ __constant__ int c_trk_out_src[OR_OUT_TRACK_FIELDS] = {
     OR_TRK_ERR_Y0, OR_TRK_ERR_TX, OR_TRK_ERR_TY, OR_TRK_ERR_INVP, OR_TRK_CHARGE, OR_TRK_VX, OR_TRK_VX + 1,
     OR_TRK_VX + 2, OR_TRK_PX, OR_TRK_PX + 1, OR_TRK_PX + 2};
 
+// a track hit's fields in the record
+__constant__ int c_hit_out_src[OR_OUT_TRACKHIT_FIELDS] = {OR_TRK_HIT_DETID, OR_TRK_HIT_CHAN,  OR_TRK_HIT_POS,
+                                                          OR_TRK_HIT_DRIFT, OR_TRK_HIT_SIGN, OR_TRK_HIT_TDC,
+                                                          OR_TRK_HIT_RESID};
+
+// A warp per event: its hits are one index space over the 54 planes, a track's
+// fields and its hits' fields go a lane each, so do a dimuon's.  Bound: memory
+// latency.  A plane, a track or a dimuon at a time, the fields of one after
+// the other, each stored before the next was read, took 57 us for 2,000
+// dimuon events; this takes 14 us.
 __global__ void __launch_bounds__(256)
     out_write_kernel(or_hits_view_t hv, or_tracks_view_t tv, or_dimuons_view_t dv, const int32_t *__restrict__ event_ids,
                      float min_stid, int n_events, const OutCount *__restrict__ cnt,
                      const OutOffset *__restrict__ off, or_output_view_t out) {
+    __shared__ int first[256 / 32][OR_NDET];  // the event's hits before each plane; [54]: all of them
     const int lane = threadIdx.x & 31;
+    int *start = first[threadIdx.x >> 5];
     for (long e = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < n_events;
          e += ((long)gridDim.x * blockDim.x) >> 5) {
         const OutCount c = cnt[e];
@@ -135,8 +164,10 @@ __global__ void __launch_bounds__(256)
             R[OR_OUT_EV_TRACKHIT0] = o.thits;
             R[OR_OUT_EV_DIMUON0] = o.dims;
         }
-        // hits, planes 1..54 in order (M:1082-1116): plane offsets by a warp scan
-        long long row = o.hits;
+        // hits, planes 1..54 in order (M:1082-1116)
+        __syncwarp();  // every lane is done with the previous event's planes
+        int total = 0;
+#pragma unroll
         for (int d0 = 1; d0 < OR_NDET; d0 += 32) {
             const int d = d0 + lane;
             const int n = d < OR_NDET ? plane_count(hv, e, d) : 0;
@@ -146,74 +177,62 @@ __global__ void __launch_bounds__(256)
                 const int v = __shfl_up_sync(0xffffffffu, incl, s);
                 if (lane >= s) incl += v;
             }
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            for (int src = 0; src < 32 && d0 + src < OR_NDET; ++src) {
-                const int np = __shfl_sync(0xffffffffu, n, src);
-                if (np == 0) continue;
-                const long long r0 = row + __shfl_sync(0xffffffffu, incl - n, src);
-                const HitPlane h = hits_of(hv, e, d0 + src);
-                for (int l = lane; l < np; l += 32) {
-                    const long long r = r0 + l;
-                    if (r >= out.cap_hits) continue;
-                    float *R = out.hits + r * OR_OUT_HIT_FIELDS;
-                    R[0] = (float)(d0 + src);
-                    R[1] = h.chan(l);
-                    R[2] = h.pos(l);
-                    R[3] = h.tdc(l);
-                    R[4] = h.drift(l);
-                }
-            }
-            row += total;
+            if (d < OR_NDET) start[d - 1] = total + incl - n;
+            total += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) start[OR_NDET - 1] = total;
+        __syncwarp();
+#pragma unroll 2
+        for (int f = lane; f < total; f += 32) {
+            int p = 0;  // the last plane that starts at or before the hit
+#pragma unroll
+            for (int s = 32; s > 0; s >>= 1)
+                if (p + s < OR_NDET - 1 && start[p + s] <= f) p += s;
+            const int n = start[p + 1] - start[p], i = f - start[p];
+            const float *h = plane_slot(hv, e, p + 1) + i;
+            const float chan = __ldg(h), pos = __ldg(h + n), tdc = __ldg(h + 2 * n), drift = __ldg(h + 4 * n);
+            const long long r = o.hits + f;
+            if (r >= out.cap_hits) continue;
+            float *R = out.hits + r * OR_OUT_HIT_FIELDS;
+            R[0] = (float)(p + 1);
+            R[1] = chan;
+            R[2] = pos;
+            R[3] = tdc;
+            R[4] = drift;
         }
         // tracks in (slot, position) order with their hits (M:1122-1162)
         {
             const int n = min((int)tv.ntracks[e * OR_NSLOTS + lane], OR_SLOTCAP);
-            int ntr = 0, nth = 0;
-            for (int k = 0; k < n; ++k) {
-                const float *T = trk_rec(tv, e, lane, k);
-                if (T[OR_TRK_STID] < min_stid) continue;
-                ++ntr;
-                nth += track_nhits(T);
-            }
-            int itr = ntr, ith = nth;
-#pragma unroll
-            for (int s = 1; s < 32; s <<= 1) {
-                const int a = __shfl_up_sync(0xffffffffu, itr, s), b = __shfl_up_sync(0xffffffffu, ith, s);
-                if (lane >= s) {
-                    itr += a;
-                    ith += b;
-                }
-            }
-            long long tr = o.tracks + itr - ntr, th = o.thits + ith - nth;
-            for (int k = 0; k < n; ++k) {
-                const float *T = trk_rec(tv, e, lane, k);
-                if (T[OR_TRK_STID] < min_stid) continue;
-                if (tr < out.cap_tracks) {
-                    float *R = out.tracks + tr * OR_OUT_TRACK_FIELDS;
-                    for (int f = 0; f < OR_OUT_TRACK_FIELDS; ++f) R[f] = T[c_trk_out_src[f]];
-                }
-                const int nh = track_nhits(T);
-                for (int l = 0; l < nh; ++l, ++th) {
-                    if (th >= out.cap_track_hits) continue;
+            unsigned take = 0u;
+            for (int k = 0; k < n; ++k)
+                if (!(trk_rec(tv, e, lane, k)[OR_TRK_STID] < min_stid)) take |= 1u << k;
+            long long tr = o.tracks, th = o.thits;
+            for (unsigned slots = __ballot_sync(0xffffffffu, take != 0u); slots; slots &= slots - 1) {
+                const int slot = __ffs(slots) - 1;
+                for (unsigned m = __shfl_sync(0xffffffffu, take, slot); m; m &= m - 1) {
+                    const float *T = trk_rec(tv, e, slot, __ffs(m) - 1);
+                    const int nh = track_nhits(T);
+                    if (lane < OR_OUT_TRACK_FIELDS && tr < out.cap_tracks)
+                        out.tracks[tr * OR_OUT_TRACK_FIELDS + lane] = __ldg(T + c_trk_out_src[lane]);
+                    const int room = (int)max(0ll, min((long long)nh, (long long)out.cap_track_hits - th));
                     float *R = out.track_hits + th * OR_OUT_TRACKHIT_FIELDS;
-                    R[0] = T[OR_TRK_HIT_DETID + l];
-                    R[1] = T[OR_TRK_HIT_CHAN + l];
-                    R[2] = T[OR_TRK_HIT_POS + l];
-                    R[3] = T[OR_TRK_HIT_DRIFT + l];
-                    R[4] = T[OR_TRK_HIT_SIGN + l];
-                    R[5] = T[OR_TRK_HIT_TDC + l];
-                    R[6] = T[OR_TRK_HIT_RESID + l];
+#pragma unroll 4
+                    for (int q = lane; q < room * OR_OUT_TRACKHIT_FIELDS; q += 32) {
+                        const int l = q / OR_OUT_TRACKHIT_FIELDS, f = q - l * OR_OUT_TRACKHIT_FIELDS;
+                        R[q] = __ldg(T + c_hit_out_src[f] + l);
+                    }
+                    ++tr;
+                    th += nh;
                 }
-                ++tr;
             }
         }
         // dimuons (M:1166-1220)
-        for (int i = lane; i < c.dims; i += 32) {
+        for (int i = 0; i < c.dims; ++i) {
             const long long r = o.dims + i;
-            if (r >= out.cap_dimuons) continue;
+            if (r >= out.cap_dimuons) break;
             const float *D = dv.dimuons + (size_t)e * OR_EVT_DIM_FLOATS + (size_t)i * OR_NDIMUONPARAM;
             float *R = out.dimuons + r * OR_OUT_DIMUON_FIELDS;
-            for (int f = 0; f < OR_OUT_DIMUON_FIELDS; ++f) {
+            for (int f = lane; f < OR_OUT_DIMUON_FIELDS; f += 32) {
                 const int sidx = c_dim_out_src[f];
                 R[f] = sidx >= 0 ? D[sidx] : D[OR_DIM_POS_P - 1 - sidx] + D[OR_DIM_NEG_P - 1 - sidx];
             }
