@@ -17,8 +17,13 @@
 //    second branch (H:2323), so there the charge test alone decides.
 //  - The cross-slot pass runs the reference block's 32 threads in lockstep,
 //    as clean_kernel does: lane = slot, decisions of a step on the state
-//    before it, demotions after a __syncwarp.
-// One warp per event.
+//    before it, demotions after a __syncwarp.  Only pairs of global tracks do
+//    anything, so the steps are gone through by masks of each slot's.
+// One warp per event.  Bound: memory latency of the segment tests, a lane per
+// slot.  The cross-slot pass over all positions of all slots took 61 us for
+// 10,000 one-dimuon events and 199 us for 1,000 uneven ones; this takes 44 and
+// 148 us (with the tracks as one list and the planes' positions in shared
+// memory 41 and 191 us: fewer warps).
 #include "or_device.cuh"
 
 namespace orgpu {
@@ -112,19 +117,23 @@ __global__ void __launch_bounds__(W * 32)
         }
         __syncwarp();
         // --- across slots, in lockstep (H:2333-2380) --------------------------
-        const int maxn = __reduce_max_sync(0xffffffffu, (unsigned)n_own);
-        for (int u = 0; u < OR_NSLOTS; ++u) {
-            const int m = __shfl_sync(0xffffffffu, n_own, u);
-            if (m == 0) continue;
-            for (int i = 0; i < maxn; ++i) {
-                float *Ti = (i < n_own) ? trk_rec(tv, e, lane, i) : nullptr;
-                const bool act = lane != u && Ti && Ti[OR_TRK_STID] >= 6;
+        // Only pairs of global tracks do anything, and an event has few: the
+        // steps are gone through by masks of each slot's.
+        unsigned alive = 0u;
+        for (int i = 0; i < n_own; ++i)
+            if (trk_rec(tv, e, lane, i)[OR_TRK_STID] >= 6) alive |= 1u << i;
+        for (unsigned um = __ballot_sync(0xffffffffu, alive != 0u); um; um &= um - 1) {
+            const int u = __ffs(um) - 1;
+            for (unsigned im = __reduce_or_sync(0xffffffffu, lane != u ? alive : 0u); im; im &= im - 1) {
+                const int i = __ffs(im) - 1;
+                const bool act = lane != u && ((alive >> i) & 1u);
                 if (!__any_sync(0xffffffffu, act)) continue;
-                for (int j = 0; j < m; ++j) {
+                float *Ti = trk_rec(tv, e, lane, i);
+                for (unsigned jm = __shfl_sync(0xffffffffu, alive, u); jm; jm &= jm - 1) {
+                    const int j = __ffs(jm) - 1;
                     float *Tj = trk_rec(tv, e, u, j);
-                    const bool alive_j = Tj[OR_TRK_STID] >= 6;
                     int d = 0;
-                    if (act && alive_j) {
+                    if (act) {
                         const bool same_q = Ti[OR_TRK_CHARGE] * Tj[OR_TRK_CHARGE] > 0;
                         if (chi2dof(Ti) < chi2dof(Tj)) {
                             if ((Ti[OR_TRK_INVP] - Tj[OR_TRK_INVP]) / Ti[OR_TRK_INVP] < SEL_MERGE_THRES && same_q) d = 1;
@@ -132,9 +141,15 @@ __global__ void __launch_bounds__(W * 32)
                             if ((Ti[OR_TRK_INVP] - Tj[OR_TRK_INVP]) / Tj[OR_TRK_INVP] < SEL_MERGE_THRES && same_q) d = 2;
                         }
                     }
-                    __syncwarp();
-                    if (d == 1) Tj[OR_TRK_STID] = 5.f;
-                    else if (d == 2) Ti[OR_TRK_STID] = 5.f;
+                    const bool gone = __any_sync(0xffffffffu, d == 1);
+                    if (lane == u && gone) {
+                        Tj[OR_TRK_STID] = 5.f;
+                        alive &= ~(1u << j);
+                    }
+                    if (d == 2) {
+                        Ti[OR_TRK_STID] = 5.f;
+                        alive &= ~(1u << i);
+                    }
                     __syncwarp();
                 }
             }
