@@ -528,34 +528,40 @@ __device__ __forceinline__ FF ff_dedx(float p, FF d1) {
     return ff_add(ff_mul(a, p), d0);
 }
 
-// (float)(ptot + p(ptot) * len) as the reference rounds it
-__device__ __forceinline__ float dim_energy(float ptot, float len, double d1, FF d1f) {
+// the double statements themselves, as calls (see slow_sqrt)
+__device__ __noinline__ float slow_energy(float ptot, float len, double d1) {
     using namespace phys;
-    const FF v = ff_add(ff_mul(ff_dedx(ptot, d1f), len), FF{ptot, 0.f});
-    // up to these bounds the loss stays well below ptot, and the polynomial's
-    // terms below 2^6
-    if (ptot < 1000.f && len < 16.f && ff_sure(v)) return v.h;
     return (float)(ptot + (DEDX_UNIT_0 + d1 * ptot + DEDX_UNIT_2 * ptot * ptot + DEDX_UNIT_3 * ptot * ptot * ptot +
                            DEDX_UNIT_4 * ptot * ptot * ptot * ptot) *
                               len);
 }
+__device__ __noinline__ float slow_step(float t) { return (float)(t * phys::STEP_FMAG); }
+__device__ __noinline__ float slow_kick(float tx, double kick, float len) { return (float)(tx + kick / len); }
+
+// (float)(ptot + p(ptot) * len) as the reference rounds it
+__device__ __forceinline__ float dim_energy(float ptot, float len, FF d1f, bool &sure) {
+    const FF v = ff_add(ff_mul(ff_dedx(ptot, d1f), len), FF{ptot, 0.f});
+    // up to these bounds the loss stays well below ptot, and the polynomial's
+    // terms below 2^6
+    sure = (ptot < 1000.f) & (len < 16.f) & ff_sure(v);
+    return v.h;
+}
 
 // (float)(t * STEP_FMAG)
-__device__ __forceinline__ float dim_step(float t) {
-    using namespace phys;
-    const FF v = ff_mul(ff_const(STEP_FMAG), t);
-    if (ff_sure(v)) return v.h;
-    return (float)(t * STEP_FMAG);
+__device__ __forceinline__ float dim_step(float t, bool &sure) {
+    const FF v = ff_mul(ff_const(phys::STEP_FMAG), t);
+    sure = ff_sure(v);
+    return v.h;
 }
 
 // (float)(tx + kick / len)
-__device__ __forceinline__ float dim_kick(float tx, double kick, FF kf, float len) {
+__device__ __forceinline__ float dim_kick(float tx, FF kf, float len, bool &sure) {
     const float q = kf.h / len;
     const FF s = ff_sum(tx, q);
     const FF v = ff_fast(s.h, s.l + (__fmaf_rn(-q, len, kf.h) + kf.l) / len);
     // (a sum that all but cancels keeps the quotient's error)
-    if (fabsf(v.h) > 0x1p-8f * fabsf(q) && ff_sure(v)) return v.h;
-    return (float)(tx + kick / len);
+    sure = (fabsf(v.h) > 0x1p-8f * fabsf(q)) & ff_sure(v);
+    return v.h;
 }
 
 // What a track's steps have in common.
@@ -568,22 +574,34 @@ struct DimTrack {
 // one FMag step (H:1290-1333)
 __device__ __forceinline__ void dim_fmag_step(SwimPt &s, const DimTrack &k) {
     using namespace phys;
+    // what depends on the same values side by side, then one branch for the
+    // lanes that need the double statements
     const float t2 = (float)STEP_FMAG;
-    const float tx_i = s.mx / s.mz;
-    const float tx_f = dim_kick(tx_i, k.kick, k.kickf, sqrtf(s.mx * s.mx + s.mz * s.mz));
-    const float t10 = dim_step(tx_i);
-    const float b0 = s.x - t10, b1 = s.y - k.t1, b2 = s.z - t2;
+    bool ok1, ok2;
+    const float tx_i = s.mx / s.mz, pxz = sqrtf(s.mx * s.mx + s.mz * s.mz);
     const float ptot_i = sqrtf(s.mx * s.mx + s.my * s.my + s.mz * s.mz);
-    float ptot_b = ptot_i;
-    if (b2 > HOLE_LENGTH_F || b0 * b0 + b1 * b1 > HOLE_RADIUS_F)
-        ptot_b = dim_energy(ptot_i, sqrtf(t10 * t10 + k.t1 * k.t1 + t2 * t2), k.d1, k.d1f);
-    const float t20 = dim_step(tx_f);
+    float tx_f = dim_kick(tx_i, k.kickf, pxz, ok1), t10 = dim_step(tx_i, ok2);
+    if (!(ok1 & ok2)) {
+        if (!ok1) tx_f = slow_kick(tx_i, k.kick, pxz);
+        if (!ok2) t10 = slow_step(tx_i);
+    }
+    const float b0 = s.x - t10, b1 = s.y - k.t1, b2 = s.z - t2;
+    const float len1 = sqrtf(t10 * t10 + k.t1 * k.t1 + t2 * t2);
+    float t20 = dim_step(tx_f, ok1), ptot_b = dim_energy(ptot_i, len1, k.d1f, ok2);
+    const bool in1 = b2 > HOLE_LENGTH_F || b0 * b0 + b1 * b1 > HOLE_RADIUS_F;
+    if (!(ok1 & (ok2 | !in1))) {
+        if (!ok1) t20 = slow_step(tx_f);
+        if (!ok2) ptot_b = slow_energy(ptot_i, len1, k.d1);
+    }
+    if (!in1) ptot_b = ptot_i;
     s.x = b0 - t20;
     s.y = b1 - k.t1;
     s.z = b2 - t2;
-    float ptot_f = ptot_b;
-    if (s.z > HOLE_LENGTH_F || s.x * s.x + s.y * s.y > HOLE_RADIUS_F)
-        ptot_f = dim_energy(ptot_f, sqrtf(t20 * t20 + k.t1 * k.t1 + t2 * t2), DEDX_UNIT_1, ff_const(DEDX_UNIT_1));
+    const float len2 = sqrtf(t20 * t20 + k.t1 * k.t1 + t2 * t2);
+    float ptot_f = dim_energy(ptot_b, len2, ff_const(DEDX_UNIT_1), ok1);
+    const bool in2 = s.z > HOLE_LENGTH_F || s.x * s.x + s.y * s.y > HOLE_RADIUS_F;
+    if (!ok1 & in2) ptot_f = slow_energy(ptot_b, len2, DEDX_UNIT_1);
+    if (!in2) ptot_f = ptot_b;
     const float pz_f = ptot_f / sqrtf(1.f + tx_f * tx_f + k.ty * k.ty);
     s.mx = pz_f * tx_f;
     s.my = pz_f * k.ty;
@@ -786,7 +804,7 @@ static_assert(OR_DIM_GROUP <= 32 && DIM_LIST >= OR_TRKMAX, "lane = event; one ev
 // j; opposite charges), sixteen pairs over the events at a time being swum
 // by the whole warp.  A thread per event swimming its pairs one after the
 // other, both tracks in turn, in blocks of 128 took 947 us for 10,000 events
-// and for 2,000; this takes 136 and 126 us.
+// and for 2,000; this takes 117 and 106 us.
 __global__ void __launch_bounds__(32)
     dimuon_kernel(const or_plane_t *__restrict__ gplane, or_tracks_view_t tv, or_dimuons_view_t dv,
                   const uint8_t *__restrict__ toomany, int n_events, int group) {
