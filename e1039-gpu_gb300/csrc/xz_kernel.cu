@@ -126,7 +126,9 @@ __device__ __forceinline__ void xz_append(XzEvent &E, bool take, int key, uchar2
     __syncwarp();
 }
 
-// Steps 1 and 2 up to the prefix sums.  False: a bin has too many entries.
+// Steps 1 and 2 up to the prefix sums.  False: a plane states more hits than
+// the reference's scratch holds (before any hit is read: a view's stride is
+// the stated count), or a bin has too many entries.
 template <int WPE>
 __device__ __forceinline__ bool xz_lists(XzEvent &E, const or_hits_view_t &hv, long e, const or_plane_t &P) {
     const int lane = lane_id(), tid = xz_thread<WPE>(), w = WPE == 1 ? 0 : threadIdx.x >> 5;
@@ -149,8 +151,10 @@ __device__ __forceinline__ bool xz_lists(XzEvent &E, const or_hits_view_t &hv, l
     xz_sync<WPE>();
     // prefix sums over the planes (lanes 0-5) and the gates' planes (8-17)
     if (w == 0) {
-        const int nraw = lane < 6 ? E.hc[lane].n : 0, n = min(nraw, XZ_MAXPLANEHITS);
-        const int g = lane >= 8 && lane < 18 ? E.gn[lane - 8] : 0;
+        const int nraw = lane < 6 ? E.hc[lane].n : 0, n = max(0, min(nraw, XZ_MAXPLANEHITS));
+        // a gate plane that states more hits than its slot holds is not staged
+        const int graw = lane >= 8 && lane < 18 ? E.gn[lane - 8] : 0;
+        const int g = graw > (lane < 12 ? OR_MAXHITS_PROP : OR_MAXHITS_HODO) ? XZ_GATE + 1 : max(0, graw);
         int a = n, b = g;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -180,6 +184,7 @@ __device__ __forceinline__ bool xz_lists(XzEvent &E, const or_hits_view_t &hv, l
         if (lane == 0) E.staged = fit ? staged : 0;
     }
     xz_sync<WPE>();
+    if (E.over) return false;
     const int total = E.start[6];
 #pragma unroll 1
     for (int f = tid; f < E.staged; f += NT) {
@@ -241,7 +246,7 @@ __device__ __forceinline__ bool xz_lists(XzEvent &E, const or_hits_view_t &hv, l
     }
     xz_sync<WPE>();
     if (tid < 10 && E.goff[tid] + E.gn[tid] <= E.staged) E.gpos[tid] = E.gate + E.goff[tid];
-    bool over = E.over;
+    bool over = false;
 #pragma unroll 1
     for (int q = 0; q < 3; ++q) {
         const int n = lane < 28 ? E.np[q][lane] : 0;
@@ -525,8 +530,8 @@ __device__ __forceinline__ void xz_counts(const or_tracks_view_t &tv, long e, in
     }
 }
 
-// An event not reconstructed: no tracklets (K:195-200), or a bin with too
-// many entries.
+// An event not reconstructed: no tracklets (K:195-200), or a plane or a bin
+// with too many entries.
 __device__ __forceinline__ void xz_reject(const or_tracks_view_t &tv, long e, bool over,
                                           int32_t *__restrict__ ntracklets, uint8_t *__restrict__ toomany) {
     tv.ntracks[e * OR_NSLOTS + lane_id()] = 0;
