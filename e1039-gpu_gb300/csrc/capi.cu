@@ -12,7 +12,8 @@
 #include "or_device.cuh"
 
 namespace orgpu {
-cudaError_t launch_event_reduce(or_hits_view_t, uint8_t *, int, uint32_t *, cudaStream_t, int, int, ChainClear);
+cudaError_t launch_event_reduce(or_hits_view_t, uint8_t *, int, uint32_t *, cudaStream_t, int, int, ChainClear,
+                                long long);
 cudaError_t launch_xz(const or_plane_t *, or_hits_view_t, or_tracks_view_t, int32_t *, uint8_t *, int, cudaStream_t,
                       int, int);
 cudaError_t launch_yz_tuned(const or_plane_t *, or_hits_view_t, or_tracks_view_t, const uint8_t *, int, uint32_t *,
@@ -79,6 +80,7 @@ struct or_ctx {
     void *yz_scratch;
     int yz_cap_units, yz_cap_heavy, yz_garena_warps;
     long long yz_pool_limit;  // survivor-pool entries the split YZ path may use (-1: all)
+    long long wait_limit = -1;  // polls of an event-reducer wait (or_set_wait_limit; -1: the default)
     int yz_count_work = 0;    // YZ calls add up their work counters (or_set_yz_work_counting)
     int warps[OR_K_COUNT];  // events (work units) per CTA of each tunable kernel
     // per-event row counts and offsets of or_output_rows, grown on demand
@@ -240,6 +242,12 @@ int or_set_yz_pool_limit(or_ctx_t *ctx, int64_t entries) {
     return OR_OK;
 }
 
+int or_set_wait_limit(or_ctx_t *ctx, int64_t polls) {
+    if (!ctx) return fail(OR_ERR_ARG, "null context");
+    ctx->wait_limit = polls < 0 ? -1 : (long long)polls;
+    return OR_OK;
+}
+
 int or_set_launch(or_ctx_t *ctx, int kernel, int events_per_cta) {
     if (!ctx) return fail(OR_ERR_ARG, "null context");
     if (kernel < 0 || kernel >= OR_K_COUNT) return fail(OR_ERR_ARG, "unknown kernel id");
@@ -312,7 +320,7 @@ static int event_reduce(or_ctx_t *ctx, or_hits_view_t hits, uint8_t *toomany, in
     if (n_events < 0 || !toomany) return fail(OR_ERR_ARG, "bad event count or flag array");
     if ((rc = check_hits(hits))) return rc;
     cudaError_t e = orgpu::launch_event_reduce(hits, toomany, n_events, ctx->d_errw, S(stream), ctx->sm_count,
-                                               ctx->warps[OR_K_EVENT_REDUCE], clear);
+                                               ctx->warps[OR_K_EVENT_REDUCE], clear, ctx->wait_limit);
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "event reducer launch");
 }
 

@@ -51,7 +51,7 @@ constexpr int ER_MAX_STAGED_HITS = ER_BUF_FLOATS / 5 + 8;
 constexpr int ER_FIRST_WORDS = (ER_MAX_STAGED_HITS + 31) / 32;
 constexpr int ER_NPLANES = 48, ER_NCHAMBERS = 24;
 static_assert(ER_BUF_FLOATS >= 5 * OR_MAXHITS_CHAM + 3, "a full plane fits the buffer");
-constexpr uint32_t ER_WAIT_LIMIT = 1u << 26;        // bounded mbarrier wait
+constexpr uint32_t ER_WAIT_LIMIT = 1u << 26;        // bounded mbarrier wait, unless or_set_wait_limit says otherwise
 constexpr uint32_t ER_DRAIN_LIMIT = 1u << 28;       // ... and the wait for copies in flight after it gave up
 
 // the 48 planes the reducer touches: the 24 chambers of the E1039 set
@@ -319,7 +319,8 @@ static __device__ __forceinline__ int er_reduce(ErWarp &S, int p0, int p1, int h
 
 template <int W>
 __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *__restrict__ toomany, int n_events,
-                                                    uint32_t *__restrict__ errw, ChainClear clear) {
+                                                    uint32_t *__restrict__ errw, ChainClear clear,
+                                                    uint32_t wait_limit) {
     extern __shared__ __align__(16) unsigned char er_smem[];
     ErWarp *sm = reinterpret_cast<ErWarp *>(er_smem);
     const int w = threadIdx.x >> 5;
@@ -333,6 +334,10 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
 #pragma unroll
             for (int b = 0; b < 2; ++b)
                 if (clear.counters[b]) clear.counters[b][i] = 0u;
+    // before the events: a warp whose wait gives up leaves none uncleared
+    if (clear.ntracklets)
+        for (long i = ((long)blockIdx.x * W + w) * 32 + lane; i < n_events; i += (long)gridDim.x * W * 32)
+            clear.ntracklets[i] = 0;
 
     for (long e = (long)blockIdx.x * W + w; e < n_events; e += (long)gridDim.x * W) {
         for (int p = lane; p < ER_NPLANES; p += 32) {
@@ -386,7 +391,7 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
                     if (sz == 0) continue;
                     tma_load_1d(S.buf + S.soff[p], S.slot[p], (uint32_t)sz * 4u, &S.bar);
                 }
-                if (!__all_sync(0xffffffffu, mbar_wait_bounded(&S.bar, phase, ER_WAIT_LIMIT))) {
+                if (!__all_sync(0xffffffffu, mbar_wait_bounded(&S.bar, phase, wait_limit))) {
                     // the wait gave up: raise the error word, then wait (again
                     // bounded) for this batch's copies still in flight, so that
                     // the warp leaves no bulk copy writing into shared memory
@@ -422,10 +427,7 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
 #pragma unroll
             for (int k = 0; k < 6; ++k) sum += __shfl_sync(0xffffffffu, m, min(31, st * 6 + k));
             const bool over = __any_sync(0xffffffffu, lane < ER_NCHAMBERS && sum > lim);
-            if (lane == 0) {
-                toomany[e] = (uint8_t)over;
-                if (clear.ntracklets) clear.ntracklets[e] = 0;
-            }
+            if (lane == 0) toomany[e] = (uint8_t)over;
         }
         __syncwarp();
     }
@@ -434,14 +436,14 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
 // Host launcher.
 template <int W>
 static cudaError_t er_launch(or_hits_view_t hv, uint8_t *toomany, int n_events, uint32_t *errw, cudaStream_t stream,
-                             int sm_count, ChainClear clear) {
+                             int sm_count, ChainClear clear, uint32_t wait_limit) {
     const size_t smem = sizeof(ErWarp) * W;
     cudaError_t e = smem_attr_once((const void *)er_kernel<W>, (int)smem);
     if (e != cudaSuccess) return e;
     long blocks = (n_events + W - 1) / W;
     const long cap = (long)sm_count * (48 / W > 0 ? 48 / W : 1);  // up to 48 resident warps per SM
     if (blocks > cap) blocks = cap;
-    er_kernel<W><<<(unsigned)blocks, W * 32, smem, stream>>>(hv, toomany, n_events, errw, clear);
+    er_kernel<W><<<(unsigned)blocks, W * 32, smem, stream>>>(hv, toomany, n_events, errw, clear, wait_limit);
     return cudaGetLastError();
 }
 
@@ -464,16 +466,18 @@ cudaError_t launch_wait_selftest(uint32_t *errw, uint32_t polls, cudaStream_t st
     return cudaGetLastError();
 }
 
-// Host launcher; `warps` = events per CTA (1, 2, 4, 8 or 16).
+// Host launcher; `warps` = events per CTA (1, 2, 4, 8 or 16), `polls` = the
+// wait's limit (< 0: ER_WAIT_LIMIT).
 cudaError_t launch_event_reduce(or_hits_view_t hv, uint8_t *toomany, int n_events, uint32_t *errw,
-                                cudaStream_t stream, int sm_count, int warps, ChainClear clear) {
+                                cudaStream_t stream, int sm_count, int warps, ChainClear clear, long long polls) {
     if (n_events <= 0) return cudaSuccess;
+    const uint32_t limit = polls < 0 || polls > ER_WAIT_LIMIT ? ER_WAIT_LIMIT : (uint32_t)polls;
     switch (warps) {
-    case 1: return er_launch<1>(hv, toomany, n_events, errw, stream, sm_count, clear);
-    case 2: return er_launch<2>(hv, toomany, n_events, errw, stream, sm_count, clear);
-    case 8: return er_launch<8>(hv, toomany, n_events, errw, stream, sm_count, clear);
-    case 16: return er_launch<16>(hv, toomany, n_events, errw, stream, sm_count, clear);
-    default: return er_launch<4>(hv, toomany, n_events, errw, stream, sm_count, clear);
+    case 1: return er_launch<1>(hv, toomany, n_events, errw, stream, sm_count, clear, limit);
+    case 2: return er_launch<2>(hv, toomany, n_events, errw, stream, sm_count, clear, limit);
+    case 8: return er_launch<8>(hv, toomany, n_events, errw, stream, sm_count, clear, limit);
+    case 16: return er_launch<16>(hv, toomany, n_events, errw, stream, sm_count, clear, limit);
+    default: return er_launch<4>(hv, toomany, n_events, errw, stream, sm_count, clear, limit);
     }
 }
 

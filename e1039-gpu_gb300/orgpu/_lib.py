@@ -23,7 +23,7 @@ EXPORTS = ("or_version", "or_last_error", "or_status_string", "or_geometry_load"
            "or_mlp_adam", "or_prop_matching", "or_global_clean", "or_run_selection", "or_set_launch",
            "or_get_launch", "or_vertexing", "or_dimuons", "or_fill_histograms", "or_hist_table_init",
            "or_run_physics", "or_output_rows", "or_rt_load", "or_rt_set_plane", "or_rt_table_bytes",
-           "or_pack_hits_rt", "or_rt_apply", "or_set_yz_pool_limit", "or_selftest_bounded_wait",
+           "or_pack_hits_rt", "or_rt_apply", "or_set_yz_pool_limit", "or_set_wait_limit", "or_selftest_bounded_wait",
            "or_yz_work_counts", "or_set_yz_work_counting", "or_gkernel_eR", "or_gKernel_XZ_tracking", "or_gKernel_YZ_tracking",
            "or_gKernel_BackTrackCleaning", "or_gKernel_Global_tracking", "or_dropin_sync", "or_yz_scored",
            "or_outer_labels", "or_run_batch_scored")
@@ -138,6 +138,7 @@ def load(path):
     lb.or_pack_hits_rt.argtypes = [vp, vp, vp, i32, vp, vp, L.OrHitsView, vp]
     lb.or_rt_apply.argtypes = [vp, vp, L.OrHitsView, i32, vp]
     lb.or_set_yz_pool_limit.argtypes = [vp, i64]
+    lb.or_set_wait_limit.argtypes = [vp, i64]
     for name in EXPORTS:
         getattr(lb, name)
     return lb

@@ -105,6 +105,11 @@ int or_get_launch(or_ctx_t *ctx, int kernel);
  * `entries` survivors (< 0: the whole pool, 192 Mi).  A tuning and test
  * knob: results do not depend on it. */
 int or_set_yz_pool_limit(or_ctx_t *ctx, int64_t entries);
+/* Polls the event reducer's wait for an event's bulk copies takes before it
+ * gives up (< 0 and above 2^26: 2^26).  A test knob: with 0 every wait gives
+ * up at once; the copies are still waited for before the warp returns, and
+ * or_stream_sync reports OR_ERR_TIMEOUT. */
+int or_set_wait_limit(or_ctx_t *ctx, int64_t polls);
 /* Copy a host or_plane_t to the device (online_reconstruction.cu:754). */
 int or_set_geometry(or_ctx_t *ctx, const or_plane_t *plane);
 /* Wait for `stream` and report the device-side error words raised since the
