@@ -237,9 +237,19 @@ class Trainer:
         self.pos_weight = pos_weight
         self.nblk = self.lib.or_mlp_grad_blocks(batch)
         self.grad = torch.zeros(self.nblk * NP, dtype=torch.float32, device=dev)
-        self.loss = torch.zeros(self.nblk, dtype=torch.float32, device=dev)
-        self.step_no = 0
         self.dev = dev
+        self._losses = None
+        self._block_losses(self.n // batch)
+        self.step_no = 0
+
+    def _block_losses(self, nb):
+        """The block losses of an epoch, a row per batch.  They stay the
+        trainer's, as the calls write them on its stream; `loss` is the last
+        row, so it has the last batch's after every epoch."""
+        if self._losses is None or len(self._losses) != max(nb, 1):
+            self._losses = _torch().zeros(max(nb, 1), self.nblk, dtype=_torch().float32, device=self.dev)
+            self.loss = self._losses[-1]
+        return self._losses
 
     def epoch(self, rng):
         """One pass over the rows in a random order; returns the mean batch loss."""
@@ -248,15 +258,13 @@ class Trainer:
         nb = self.n // self.batch
         if nb == 0:
             return 0.0
-        # a row of block losses per batch, added up once (adding them up batch
-        # by batch took two launches each)
-        losses = torch.empty(nb, self.nblk, dtype=torch.float32, device=self.dev)
+        # added up once (batch by batch took two launches each)
+        losses = self._block_losses(nb)
         for b in range(nb):
             idx = perm[b * self.batch:(b + 1) * self.batch]
-            self.loss = losses[b]
             _lib.check(self.lib.or_mlp_gradient(self.ctx, self.model.ptr(), self.features.data_ptr(),
                                                 self.labels.data_ptr(), idx.data_ptr(), self.batch,
-                                                float(self.pos_weight), self.grad.data_ptr(), self.loss.data_ptr(),
+                                                float(self.pos_weight), self.grad.data_ptr(), losses[b].data_ptr(),
                                                 self.stream), "or_mlp_gradient")
             self.step_no += 1
             _lib.check(self.lib.or_mlp_adam(self.ctx, self.param.data_ptr(), self.m1.data_ptr(), self.m2.data_ptr(),
