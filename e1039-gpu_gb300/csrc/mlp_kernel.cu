@@ -84,7 +84,7 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 
 constexpr int MS_ROWS = 128;       // tracklets per tile = MMA M
 constexpr int MS_TMEM_COLS = 64;   // D1, then D2: D1 is read before the second layer's MMAs
-constexpr int MS_CTAS = 7;         // per SM: 33 KB of shared memory and 64 TMEM columns each
+constexpr int MS_CTAS = 7;         // per SM: 32 KB of shared memory and 64 TMEM columns each
 
 struct __align__(1024) MlpSmem {
     uint8_t a1[MS_ROWS * MLP_IN * 2];  // x tile, K = 16
@@ -96,6 +96,8 @@ struct __align__(1024) MlpSmem {
     uint32_t tmem_base;
     uint64_t bar;
 };
+static_assert(MS_CTAS * (sizeof(MlpSmem) + 1024) <= 228 * 1024, "an SM holds them, with the 1 KB each that CUDA takes");
+static_assert(MS_CTAS * MS_TMEM_COLS <= 512, "and their tensor memory");
 
 // A tile's time is its two MMA round trips and the epilogues between them, so
 // the CTAs of an SM overlap their tiles: seven of them at 72 registers (the
@@ -103,8 +105,10 @@ struct __align__(1024) MlpSmem {
 // take the same 64), each loading its next rows while its first layer runs.
 // Weights come in 16 bytes at a time, which is also the core matrix's row.
 // Bound: issue of the epilogues.  With four CTAs, 2-byte weight loads and
-// all 64 columns in registers 1,000,003 rows took 61.1 us; this takes
-// 47.4 us (floor: 10 us for 68 bytes a row).
+// all 64 columns in registers 1,000,003 and 4,000,000 rows took 66 and 197 us;
+// with six CTAs (a seventh did not fit beside 1 KB of unused shared memory
+// each, and its share of the tiles ran after the others) 56 and 187 us; this
+// takes 50 and 154 us (floor: 10 us for 68 bytes a row, and 40).
 __device__ __forceinline__ void mlp_load_row(const float *__restrict__ feat, long row, long n_rows, const float *mean,
                                              float4 x[MLP_IN / 4]) {
     const float4 *src = reinterpret_cast<const float4 *>(row < n_rows ? feat + row * MLP_IN : mean);
@@ -533,7 +537,7 @@ __global__ void mlp_adam_kernel(float *__restrict__ param, float *__restrict__ m
     }
 }
 
-size_t mlp_score_smem() { return sizeof(MlpSmem) + 1024; }
+size_t mlp_score_smem() { return sizeof(MlpSmem); }
 size_t mlp_train_smem() { return sizeof(TrainSmem); }
 
 cudaError_t launch_mlp_score(const or_mlp_t *model, const float *feat, long n_rows, const int32_t *n_rows_dev,
