@@ -103,7 +103,8 @@ static_assert(MS_CTAS * MS_TMEM_COLS <= 512, "and their tensor memory");
 // the CTAs of an SM overlap their tiles: seven of them at 72 registers (the
 // epilogues hold 16 accumulator columns at a time, both layers' accumulators
 // take the same 64), each loading its next rows while its first layer runs.
-// Weights come in 16 bytes at a time, which is also the core matrix's row.
+// Weights come in four bytes at a time, whatever the model's address (100,000
+// rows 17 us; in 16 bytes, where the address allows it, the same; in two 29).
 // Bound: issue of the epilogues.  With four CTAs, 2-byte weight loads and
 // all 64 columns in registers 1,000,003 and 4,000,000 rows took 66 and 197 us;
 // with six CTAs (a seventh did not fit beside 1 KB of unused shared memory
@@ -126,22 +127,19 @@ __global__ void __launch_bounds__(MS_ROWS, MS_CTAS)
     extern __shared__ __align__(1024) uint8_t ms_raw[];
     MlpSmem &S = *reinterpret_cast<MlpSmem *>(ms_raw);
     const int t = threadIdx.x, w = t >> 5;
-    // weights into the B operand layouts (8 elements of a row are 16 bytes
-    // there too), small vectors as floats
-    if ((reinterpret_cast<uintptr_t>(model) & 15u) == 0) {
-        static_assert(offsetof(or_mlp_t, w1) % 16 == 0 && offsetof(or_mlp_t, w2) % 16 == 0, "16-byte weight loads");
-        const uint4 *w1 = reinterpret_cast<const uint4 *>(model->w1), *w2 = reinterpret_cast<const uint4 *>(model->w2);
+    // weights into the B operand layouts, two at a time (their address in the
+    // model is that of its floats), small vectors as floats
+    {
+        static_assert(alignof(or_mlp_t) >= 4 && offsetof(or_mlp_t, w1) % 4 == 0 && offsetof(or_mlp_t, w2) % 4 == 0,
+                      "4-byte weight loads");
+        const uint32_t *w1 = reinterpret_cast<const uint32_t *>(model->w1);
+        const uint32_t *w2 = reinterpret_cast<const uint32_t *>(model->w2);
 #pragma unroll
-        for (int i = t; i < MLP_H * MLP_IN / 8; i += MS_ROWS)
-            *reinterpret_cast<uint4 *>(S.b1 + cm_offset(i * 8 / MLP_IN, i * 8 % MLP_IN, MLP_IN)) = w1[i];
+        for (int i = t; i < MLP_H * MLP_IN / 2; i += MS_ROWS)
+            *reinterpret_cast<uint32_t *>(S.b1 + cm_offset(i * 2 / MLP_IN, i * 2 % MLP_IN, MLP_IN)) = w1[i];
 #pragma unroll
-        for (int i = t; i < MLP_H * MLP_H / 8; i += MS_ROWS)
-            *reinterpret_cast<uint4 *>(S.b2 + cm_offset(i * 8 / MLP_H, i * 8 % MLP_H, MLP_H)) = w2[i];
-    } else {
-        for (int i = t; i < MLP_H * MLP_IN; i += MS_ROWS)
-            *reinterpret_cast<uint16_t *>(S.b1 + cm_offset(i / MLP_IN, i % MLP_IN, MLP_IN)) = model->w1[i];
-        for (int i = t; i < MLP_H * MLP_H; i += MS_ROWS)
-            *reinterpret_cast<uint16_t *>(S.b2 + cm_offset(i / MLP_H, i % MLP_H, MLP_H)) = model->w2[i];
+        for (int i = t; i < MLP_H * MLP_H / 2; i += MS_ROWS)
+            *reinterpret_cast<uint32_t *>(S.b2 + cm_offset(i * 2 / MLP_H, i * 2 % MLP_H, MLP_H)) = w2[i];
     }
     if (t < MLP_IN) {
         S.mean[t] = model->mean[t];
