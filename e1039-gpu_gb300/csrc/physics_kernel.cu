@@ -1009,7 +1009,13 @@ __global__ void __launch_bounds__(W * 32)
         nbins[i] = min((int)H->nbins[i], OR_HIST_NBINS_MAX);
         hw[i] = H->pts_hw[i];
     }
-    __syncthreads();
+    // the tables' order is looked at by blocks that may have something to
+    // count: some event of theirs has tracks or dimuons (3,000 rejected events
+    // 21 -> 8 us)
+    bool some = false;
+    for (long e = (long)blockIdx.x * W + w; e < n_events && !some; e += (long)gridDim.x * W)
+        if (!toomany[e]) some = __any_sync(0xffffffffu, tv.ntracks[e * OR_NSLOTS + lane] != 0 || dv.ndimuons[e] != 0);
+    if (!__syncthreads_or(some)) return;
     for (int i = w; i < NT; i += W) {
         const float *xp = H->xpts + (size_t)i * OR_HIST_NBINS_MAX;
         bool ok = true;
