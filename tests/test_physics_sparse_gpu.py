@@ -88,3 +88,86 @@ def test_histograms(setup, what, tracks):
     got = h.download().values_array()
     np.testing.assert_array_equal(got, want.values_array())
     assert (got.sum() > 0) == (tracks and what != "none")
+
+
+# events whose tracks go beyond what a warp lists at a time: tracks per event
+# from a multiple of the largest group on, in a batch large enough for it
+# (some 9,100 events on 152 SMs)
+BATCH = 9200
+DENSE = {0: [3], 160: [100] * 16, 320: [512, 0, 512, 1, 0, 300, 40, 0, 0, 224, 223, 225, 256, 2, 0, 512], 9199: [40]}
+
+
+def _dense(s, stid, opposite):
+    """The events of DENSE from vertexed tracks of the batch, their charges
+    negative in `opposite` of each event's and among them records below
+    `stid`."""
+    from orgpu import layout as L
+    pool = np.array([r for e in range(s["n"]) if not s["snap"].toomany_xz[e]
+                     for _, _, r in s["vertexed"].records(e) if r[L.TRK_STID] == 7], np.float32)
+    assert len(pool) > 50
+    rng = np.random.default_rng(61)
+    at = [p + i for p, c in DENSE.items() for i in range(len(c))]
+    counts = [m for c in DENSE.values() for m in c]
+    t = L.HostTracks(len(at))
+    T = t.tracks.reshape(len(at), L.NSLOTS, L.SLOTCAP, L.NTRKPARAM)
+    for e, m in enumerate(counts):
+        r = pool[rng.integers(0, len(pool), m)]
+        r[:, L.TRK_CHARGE] = 1.0
+        r[rng.permutation(m)[:opposite], L.TRK_CHARGE] = -1.0
+        r[:, L.TRK_STID] = np.where(rng.random(m) < 0.05, 3.0, stid)
+        # slot after slot, or spread over the slots
+        slot, k = (np.arange(m) // L.SLOTCAP, np.arange(m) % L.SLOTCAP) if e % 2 else (np.arange(m) % L.NSLOTS, np.arange(m) // L.NSLOTS)
+        T[e, slot, k] = r
+        t.ntracks[e * L.NSLOTS:(e + 1) * L.NSLOTS] = np.bincount(slot, minlength=L.NSLOTS)
+    return np.array(at), t
+
+
+def _dense_batch(at, t):
+    import torch
+    from orgpu import layout as L, pipeline
+    b = pipeline.DeviceBatch(BATCH)
+    idx = torch.from_numpy(at).cuda()
+    b.ntracks.view(BATCH, L.NSLOTS)[idx] = torch.from_numpy(t.ntracks.view(np.int16)).view(-1, L.NSLOTS).cuda()
+    b.tracks.view(BATCH, -1)[idx] = torch.from_numpy(t.tracks).view(len(at), -1).cuda()
+    return b, idx
+
+
+def test_vertexing_of_dense_events(setup):
+    from oracle import pyoracle as O
+    from orgpu import layout as L
+    s = setup
+    at, t = _dense(s, 6.0, 4)
+    b, idx = _dense_batch(at, t)
+    s["rc"].vertexing(b)
+    s["rc"].sync()
+    got = L.HostTracks(len(at))
+    got.ntracks[:] = t.ntracks
+    got.tracks[:] = b.tracks.view(BATCH, -1)[idx].cpu().numpy().reshape(-1)
+    st = O.OracleState(len(at))
+    O.vertexing(s["plane"], t, st)
+    assert track_mismatches(got, t) == []
+    assert (t.tracks.reshape(-1, L.NTRKPARAM)[:, L.TRK_STID] == 7).sum() > 2000
+
+
+def test_dimuons_of_dense_events(setup):
+    import golden_io as G
+    from oracle import pyoracle as O
+    from orgpu import layout as L, pipeline
+    s = setup
+    at, t = _dense(s, 7.0, 4)
+    b, idx = _dense_batch(at, t)
+    d = pipeline.DeviceDimuons(BATCH)
+    d.ndimuons.fill_(5)
+    s["rc"].dimuons(b, d)
+    s["rc"].sync()
+    st = O.OracleState(len(at))
+    want, got = L.HostDimuons(len(at)), L.HostDimuons(len(at))
+    O.dimuons(s["plane"], t, want, st)
+    counts = d.ndimuons.cpu().numpy().view(np.uint16)
+    assert not np.delete(counts, at).any()
+    got.ndimuons[:] = counts[at]
+    got.dimuons[:] = d.dimuons.view(BATCH, -1)[idx].cpu().numpy().reshape(-1)
+    no = np.zeros(len(at), np.uint8)
+    r = G.compare_dimuons(G.compact_dimuons(got, no), G.compact_dimuons(want, no), 0.0, phi_ulps=4)
+    assert r["count_mismatch"] == [] and r["value_mismatch"] == [], r
+    assert want.ndimuons.sum() > 20
