@@ -48,14 +48,11 @@ constexpr short DET_SENTINEL = -100;  // never adjacent to a plane id
 constexpr int DET_X2 = 16, DET_XP2 = 15;           // st2 x/x'  (detsuperid[2][0]*2)
 constexpr int DET_U2 = 18, DET_UP2 = 17;           // st2 u/u'
 constexpr int DET_V2 = 14, DET_VP2 = 13;           // st2 v/v'
-__host__ __device__ constexpr int det_x3(int st3) { return st3 == 3 ? 22 : 28; }   // detsuperid[3|4][0]*2
 __host__ __device__ constexpr int det_u3(int st3) { return st3 == 3 ? 24 : 30; }
 __host__ __device__ constexpr int det_v3(int st3) { return st3 == 3 ? 20 : 26; }
 constexpr int DET_P1X1 = 50, DET_P1X2 = 49, DET_P2X1 = 52, DET_P2X2 = 51;  // detsuperid[5|6][0]
 constexpr int DET_P1Y1 = 48, DET_P1Y2 = 47, DET_P2Y1 = 54, DET_P2Y2 = 53;  // detsuperid[5|6][1]
 
-__device__ __constant__ short c_eff_detid_chambers[24] = {1,  2,  3,  4,  5,  6,  13, 14, 15, 16, 17, 18,
-                                                          19, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 30};
 __device__ __constant__ short c_hodoplanesx[4][2] = {{31, 32}, {37, 38}, {39, 40}, {45, 46}};
 __device__ __constant__ float c_hodofudgefac[4] = {0.25f, 0.2f, 0.15f, 0.0f};
 __device__ __constant__ float c_hodoXcellwidth[4] = {7.32f, 13.0f, 14.5875f, 19.6475f};

@@ -157,12 +157,6 @@ __device__ __forceinline__ FF dbl_ff(double x, bool &ok) {
     const int u = (__float_as_int(h) & 0xFF800000) - (23 << 23);
     return FF{h, __int_as_float(u | (int)((lo >> 6) & 0x7FFFFF)) - __int_as_float(u)};
 }
-// a float as a double (normal numbers)
-__device__ __forceinline__ double flt_dbl(float x) {
-    const int u = __float_as_int(x), e = (u >> 23) & 0xFF;
-    if (e == 0 || e == 255) return (double)x;
-    return __hiloint2double((u & 0x80000000) | ((u & 0x7FFFFFFF) >> 3) + 0x38000000, u << 29);
-}
 // x plus k units of its last place
 __device__ __forceinline__ double dbl_ulps(double x, int k) {
     return __longlong_as_double(__double_as_longlong(x) + k);
@@ -569,7 +563,7 @@ __device__ __forceinline__ float dim_kick(float tx, FF kf, float len, bool &sure
 
 // What a track's steps have in common.
 struct DimTrack {
-    float charge, ty, t1;  // t1 = (float)(ty * STEP_FMAG)
+    float ty, t1;          // t1 = (float)(ty * STEP_FMAG)
     double kick, d1;       // d1 = the linear energy-loss coefficient of the first update, DEDX_UNIT_2 for the
     FF kickf, d1f;         // reference's second track (H:1354)
 };
@@ -633,7 +627,6 @@ struct SwimResult {
 __device__ __noinline__ void pair_swim(SwimPt s, float charge, float ty, double d1, SwimResult &o) {
     using namespace phys;
     DimTrack k;
-    k.charge = charge;
     k.ty = ty;
     k.t1 = (float)(ty * STEP_FMAG);
     k.kick = 2.f * charge * PTKICK_UNIT * STEP_FMAG;
