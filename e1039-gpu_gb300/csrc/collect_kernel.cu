@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(CO_THREADS)
     }
     most = __reduce_max_sync(0xffffffffu, most);
 #pragma unroll 1
-    for (int k0 = 0; k0 < most; k0 += 4) {  // 32 reads in flight per lane
+    for (int k0 = 0; k0 < most; k0 += 4) {  // 4 P reads in flight per lane
         float v[P][4];
 #pragma unroll
         for (int i = 0; i < P; ++i)

@@ -20,7 +20,7 @@
 // accepted depends on the x1 pair and the hit alone, so the last combination
 // that reaches the y fit is the last accepted v1 pair with the last accepted
 // u1 pair, and the last writer of each scratch entry follows from the two
-// lists in the same way (gl_scan).  So
+// lists in the same way (the end of gl_track's loop).  So
 //   - the x fits of up to 32 x1 pairs are made at once, one per lane, up to
 //     the first one inside the momentum window (only that one changes y0 and
 //     ty);

@@ -21,8 +21,8 @@
 // (`#pragma unroll 1`): those kernels are limited by instruction-cache
 // misses, and one copy of a loop body costs less there than unrolled copies
 // save in issue slots (measured per loop group on the 100,000-event uneven
-// batch: YZ 191 -> 122 ms, global 33 -> 16 ms, outputs bit-identical).
-// The XZ kernel is the exception: there the unrolled loops are faster.
+// batch, on earlier forms of the kernels: YZ 191 -> 122 ms, global 33 -> 16
+// ms, outputs bit-identical).
 
 
 namespace orgpu {

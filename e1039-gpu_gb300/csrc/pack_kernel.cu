@@ -11,8 +11,8 @@
 // (or_stream_sync reports it as an argument error); its slots are then
 // undefined but every write stays inside them.  Records whose det is outside
 // 1..54 (they sort first or last) are skipped.  One warp per event: the planes'
-// runs are where the det changes from one record to the next, then the field
-// writes, 128 records in flight in both passes.
+// runs are where the det changes from one record to the next (512 records'
+// planes in flight), then the field writes (128 records in flight).
 //
 // Bound: the pieces of 100 to 600 bytes, off sector boundaries, that an
 // event's planes are written in (3.5 of 6.9 TB/s; staging the records in

@@ -213,7 +213,8 @@ __device__ __forceinline__ double dbl_settle(double g, float x, bool &ok) {
 }
 
 // sqrt(s): two floats' worth of it, then one FMA gives what is left, exactly
-// enough to round.  y is 1 / sqrt(s) to a float.
+// enough to round (the remainder of an approximate root, as that of a quotient
+// above: Markstein 2000).  y is 1 / sqrt(s) to a float.
 __device__ __forceinline__ double vtx_sqrt(double s, float &y, bool &sure) {
     bool ok = true;
     const FF a = dbl_ff(s, ok);
@@ -228,7 +229,8 @@ __device__ __forceinline__ double vtx_sqrt(double s, float &y, bool &sure) {
     return exact ? g : r;
 }
 
-// m / p, y being 1 / p to a float, the same way
+// m / p, y being 1 / p to a float, the same way (Markstein's remainder of the
+// quotient)
 __device__ __forceinline__ double vtx_div(double m, double p, float y, bool &sure) {
     bool ok = y > 0.f;
     const FF a = dbl_ff(m, ok), b = dbl_ff(p, ok);

@@ -161,7 +161,7 @@ struct YzHeavy {
     // outer-iteration scoring: the tracklet's first score row (-1: no rows,
     // nothing pruned), its row count (the live outer iterations), the inner
     // combinations per outer iteration, and the outer index of its best
-    // combination (written by yz_apply_kernel; -1: none)
+    // combination (written with that combination by yz_finish; -1: none)
     int orow0, nrows, c2, best_g;
     // its window image in the image pool (16-byte words), -1: none
     int img;
@@ -2856,9 +2856,10 @@ __global__ void __launch_bounds__(W * 32, (OR_YZ_FIRST_WARPS_SM / W > 0 ? OR_YZ_
     if (lane == 0 && sc.count_work) yz_flush_counts(sc, 0ull, 0ull, n_surv);
 }
 
-// Split path, second kernel: per unit, the windows again and then its
-// survivors replayed in order with the sign carry (or the whole unit on the
-// combined path when its survivors did not fit); writes the unit's best.
+// Split path, second kernel: per unit, the tracklet's windows from their image
+// and then its survivors replayed in order with the sign carry (or the whole
+// unit on the combined path when its survivors or its image did not fit);
+// writes the unit's best.
 #ifndef OR_YZ_SECOND_WARPS_SM
 #define OR_YZ_SECOND_WARPS_SM 28
 #endif
@@ -3276,8 +3277,8 @@ static cudaError_t launch_yz_impl(const or_plane_t *d_plane, or_hits_view_t hv, 
     // and so which ones have score rows, depends on the unit's budget.
     const int chunk = prune.ofeat ? YZ_PLAN_CHUNK_SCORED : YZ_PLAN_CHUNK;
     const long nplan = (long)n_events * (OR_NSLOTS / chunk);
-    // the list stands in the best records' area, which no kernel before the
-    // survivor kernel uses
+    // the list stands in the best records' area: it is read by the planning
+    // pass alone, and nothing writes a best record before that is done
     const bool listed = nplan <= (long)(sizeof(YzBest) / 4) * cap_units;
     sc.list = listed ? reinterpret_cast<unsigned *>(sc.best) : nullptr;
     const unsigned list_blocks = listed ? (unsigned)(((long)n_events * 32 + YZ_LIST_THREADS - 1) / YZ_LIST_THREADS) : 0u;
