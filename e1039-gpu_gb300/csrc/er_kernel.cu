@@ -336,7 +336,8 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
                 if (clear.counters[b]) clear.counters[b][i] = 0u;
     // before the events: a warp whose wait gives up leaves none uncleared
     if (clear.ntracklets)
-        for (long i = ((long)blockIdx.x * W + w) * 32 + lane; i < n_events; i += (long)gridDim.x * W * 32)
+#pragma unroll 1
+        for (unsigned i = (blockIdx.x * W + w) * 32 + lane; i < (unsigned)n_events; i += gridDim.x * W * 32)
             clear.ntracklets[i] = 0;
 
     for (long e = (long)blockIdx.x * W + w; e < n_events; e += (long)gridDim.x * W) {
