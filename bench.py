@@ -525,8 +525,8 @@ def yz_roofline(counts, yz_ms, n, clk, dev, prof, nx=4):
 
 
 # kernels one step launches: pack, event reducer, XZ, YZ fit table / plan /
-# first cut / survivors / apply, cleaning, global tracking
-LAUNCHES_PER_STEP = 10
+# first cut / survivors / apply, cleaning, global tracking's list and itself
+LAUNCHES_PER_STEP = 11
 
 
 def rt_leg(args, rc, b, plane, rec, d_rec, d_off, d_wp, dev):

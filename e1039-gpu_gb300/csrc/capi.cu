@@ -152,12 +152,12 @@ const char *or_status_string(int s) {
 #define OR_YZ_FIRST_WARPS_SM 28
 #endif
 
-// Room for every heavy tracklet of a 100,000-event batch of the uneven
-// workload (about 0.7 M heavy tracklets, 0.75 M units), and in proportion
-// for a context sized to a smaller largest batch (42 units and 21 heavy
-// tracklets per event, at least 64 Ki and 32 Ki); a batch beyond it
-// evaluates the excess in the planning pass, correct but without the queue's
-// balance.  The survivor pool and the window images scale with the units.
+// Room for every tracklet that a 100,000-event batch of the uneven workload
+// queues (1.34 M of them in as many units; light ones are queued too, except
+// with the combination scorer's rows), and in proportion for a context sized
+// to a smaller largest batch (42 units and 21 tracklets per event, at least 64
+// Ki and 32 Ki); a batch beyond it evaluates the excess in the planning pass,
+// correct but without the queue's balance.  The survivor pool and the window images scale with the units.
 static void yz_caps(int max_events, int &units, int &heavy) {
     if (max_events <= 0 || max_events >= 100000) {
         units = 1 << 22;

@@ -59,8 +59,12 @@ namespace orgpu {
 
 constexpr int YZ_MAXWIN = 100;          // windowed hits per plane (the reference's hitidx arrays)
 constexpr int YZ_MAXPAIR = 100;         // pairs per projection (the reference's hitpairs arrays)
-// Build-time tunables (-D...), with the values measured best on the
-// 100,000-event uneven batch; results do not depend on any of them:
+// Build-time tunables (-D...); results do not depend on any of them.  On the
+// present kernels and the 100,000-event uneven batch: first cut 8.9 / 9.2 /
+// 9.9 ms at 28 / 24 / 20 warps per SM, survivors 6.2 / 6.6 / 7.4, planning 5.3
+// / 5.1 / 5.8; units of 1,024 / 4,096 / 8,192 / 16,384 combinations 28.6 / 21.4
+// / 20.4 / 20.4 ms (the three together).  The others were chosen on earlier
+// forms of the kernels.
 //   OR_YZ_ARENA          windowed hit records per warp in shared memory
 //   OR_YZ_WARPS_SM       warps per SM of the combined work kernel
 //   OR_YZ_SPLIT          first-cut / survivor kernels (1) or the combined one (0)
