@@ -703,9 +703,9 @@ static cudaError_t xz_launch(const or_plane_t *d_plane, or_hits_view_t hv, or_tr
     long blocks = (n_events + W - 1) / W;
     // An event per warp, as blocks come free, evens out events of different
     // size; on large batches loading the planes for every block costs more
-    // than that (uneven events, resident blocks that go round -> a block per
-    // W events: 10,000 820 -> 702 us, 20,000 1,248 -> 1,231, 40,000 1,906 ->
-    // 2,238).
+    // than that (W = 4, uneven events, resident blocks that go round -> a block
+    // per W events: 10,000 820 -> 702 us, 20,000 1,248 -> 1,231, 40,000 1,906
+    // -> 2,238).
     const long cap = (long)sm_count * (32 / W > 0 ? 32 / W : 1);
     if (blocks > cap && n_events > 128 * sm_count) blocks = cap;
     xz_kernel<W><<<(unsigned)blocks, W * 32, smem, stream>>>(d_plane, hv, tv, ntracklets, toomany, n_events);
