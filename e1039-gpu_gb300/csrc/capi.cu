@@ -15,7 +15,7 @@ namespace orgpu {
 cudaError_t launch_event_reduce(or_hits_view_t, uint8_t *, int, uint32_t *, cudaStream_t, int, int, ChainClear,
                                 long long);
 cudaError_t launch_xz(const or_plane_t *, or_hits_view_t, or_tracks_view_t, int32_t *, uint8_t *, int, cudaStream_t,
-                      int, int);
+                      int, int, bool);
 cudaError_t launch_yz_tuned(const or_plane_t *, or_hits_view_t, or_tracks_view_t, const uint8_t *, int, uint32_t *,
                             void *, int, int, int, cudaStream_t, int, int, long long, int, bool);
 cudaError_t launch_yz(const or_plane_t *, or_hits_view_t, or_tracks_view_t, const uint8_t *, int, uint32_t *, void *,
@@ -328,16 +328,22 @@ int or_event_reduce(or_ctx_t *ctx, or_hits_view_t hits, uint8_t *toomany, int n_
     return event_reduce(ctx, hits, toomany, n_events, stream, {});
 }
 
-int or_xz(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, int32_t *ntracklets, uint8_t *toomany,
-          int n_events, void *stream) {
+// `chain`: the tracklet counts of events flagged before are cleared too
+static int xz_tracking(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, int32_t *ntracklets,
+                       uint8_t *toomany, int n_events, void *stream, bool chain) {
     int rc = check_ctx(ctx, true);
     if (rc) return rc;
     if (n_events < 0 || !toomany || !ntracklets) return fail(OR_ERR_ARG, "bad event count or output arrays");
     if ((rc = check_hits(hits)) || (rc = check_tracks(tracks))) return rc;
     cudaError_t e =
         orgpu::launch_xz(ctx->d_plane, hits, tracks, ntracklets, toomany, n_events, S(stream), ctx->sm_count,
-                         ctx->warps[OR_K_XZ]);
+                         ctx->warps[OR_K_XZ], chain);
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "XZ launch");
+}
+
+int or_xz(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, int32_t *ntracklets, uint8_t *toomany,
+          int n_events, void *stream) {
+    return xz_tracking(ctx, hits, tracks, ntracklets, toomany, n_events, stream, false);
 }
 
 // `cleared`: the stage's counters are zero already (ChainClear)
@@ -482,9 +488,9 @@ int or_run_batch(or_ctx_t *ctx, or_hits_view_t hits, or_tracks_view_t tracks, in
     if (n_events < 0 || !toomany || !ntracklets) return fail(OR_ERR_ARG, "bad event count or output arrays");
     if ((rc = check_hits(hits)) || (rc = check_tracks(tracks))) return rc;
     const orgpu::ChainClear clear{
-        ntracklets, {static_cast<uint32_t *>(ctx->yz_scratch), reinterpret_cast<uint32_t *>(ctx->d_sched)}};
+        {static_cast<uint32_t *>(ctx->yz_scratch), reinterpret_cast<uint32_t *>(ctx->d_sched)}};
     if ((rc = event_reduce(ctx, hits, toomany, n_events, stream, clear))) return rc;
-    if ((rc = or_xz(ctx, hits, tracks, ntracklets, toomany, n_events, stream))) return rc;
+    if ((rc = xz_tracking(ctx, hits, tracks, ntracklets, toomany, n_events, stream, true))) return rc;
     if ((rc = yz_tracking(ctx, hits, tracks, toomany, n_events, stream, true))) return rc;
     if ((rc = or_back_clean(ctx, tracks, toomany, n_events, stream))) return rc;
     return global_tracking(ctx, hits, tracks, toomany, n_events, stream, true);
@@ -893,7 +899,7 @@ extern "C" int or_gKernel_XZ_tracking(gEventHitCollections *hitcolls, gEventTrac
                                            or_hits_view_from_collection(hitcolls),
                                            or_tracks_view_from_collection(tklcoll), nTracklets,
                                            reinterpret_cast<uint8_t *>(hastoomanyhits), OR_REF_EVTMAX, nullptr,
-                                           ctx->sm_count, ctx->warps[OR_K_XZ]);
+                                           ctx->sm_count, ctx->warps[OR_K_XZ], false);
     return e == cudaSuccess ? OR_OK : cuda_fail(e, "or_gKernel_XZ_tracking launch");
 }
 

@@ -334,11 +334,6 @@ __global__ void __launch_bounds__(W * 32) er_kernel(or_hits_view_t hv, uint8_t *
 #pragma unroll
             for (int b = 0; b < 2; ++b)
                 if (clear.counters[b]) clear.counters[b][i] = 0u;
-    // before the events: a warp whose wait gives up leaves none uncleared
-    if (clear.ntracklets)
-#pragma unroll 1
-        for (unsigned i = (blockIdx.x * W + w) * 32 + lane; i < (unsigned)n_events; i += gridDim.x * W * 32)
-            clear.ntracklets[i] = 0;
 
     for (long e = (long)blockIdx.x * W + w; e < n_events; e += (long)gridDim.x * W) {
         for (int p = lane; p < ER_NPLANES; p += 32) {

@@ -454,10 +454,9 @@ __device__ __forceinline__ void tma_load_1d(void *dst_smem, const void *src_gmem
         : "memory");
 }
 // What the event reducer clears for the stages of a whole-chain call, so that
-// the chain needs no memsets between its kernels (null: nothing): the
-// events' tracklet counts and two 256-byte blocks of counters.
+// the chain needs no memsets between its kernels (null: nothing): two 256-byte
+// blocks of counters.
 struct ChainClear {
-    int32_t *ntracklets;
     uint32_t *counters[2];
 };
 

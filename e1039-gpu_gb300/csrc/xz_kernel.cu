@@ -151,10 +151,10 @@ __device__ __forceinline__ bool xz_lists(XzEvent &E, const or_hits_view_t &hv, l
     xz_sync<WPE>();
     // prefix sums over the planes (lanes 0-5) and the gates' planes (8-17)
     if (w == 0) {
-        const int nraw = lane < 6 ? E.hc[lane].n : 0, n = max(0, min(nraw, XZ_MAXPLANEHITS));
+        const int n = lane < 6 ? max(0, E.hc[lane].n) : 0;
         // a gate plane that states more hits than its slot holds is not staged
-        const int graw = lane >= 8 && lane < 18 ? E.gn[lane - 8] : 0;
-        const int g = graw > (lane < 12 ? OR_MAXHITS_PROP : OR_MAXHITS_HODO) ? XZ_GATE + 1 : max(0, graw);
+        const unsigned graw = lane >= 8 && lane < 18 ? (unsigned)E.gn[lane - 8] : 0u;
+        const int g = graw > (lane < 12 ? OR_MAXHITS_PROP : OR_MAXHITS_HODO) ? XZ_GATE + 1 : (int)graw;
         int a = n, b = g;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -174,7 +174,7 @@ __device__ __forceinline__ bool xz_lists(XzEvent &E, const or_hits_view_t &hv, l
         if (lane < 7) E.start[lane] = a - n;
         if (lane < 6 && (lane & 1)) E.cpair[(lane >> 1) + 1] = c;
         if (lane == 6) E.cpair[0] = 0;
-        const bool many = __any_sync(0xffffffffu, nraw > XZ_MAXPLANEHITS);
+        const bool many = __any_sync(0xffffffffu, n > XZ_MAXPLANEHITS);
         if (lane == 0) E.over = many;
         // the gates' hits go to shared memory as far as whole planes fit
         if (lane >= 8 && lane < 18) E.goff[lane - 8] = b <= XZ_GATE ? b - g : XZ_GATE;
@@ -531,13 +531,15 @@ __device__ __forceinline__ void xz_counts(const or_tracks_view_t &tv, long e, in
 }
 
 // An event not reconstructed: no tracklets (K:195-200), or a plane or a bin
-// with too many entries.
-__device__ __forceinline__ void xz_reject(const or_tracks_view_t &tv, long e, bool over,
+// with too many entries.  On its own the stage leaves a flagged event's
+// tracklet count as it stands, as the reference's kernel does; a whole-chain
+// call (`chain`) wants it cleared.
+__device__ __forceinline__ void xz_reject(const or_tracks_view_t &tv, long e, bool over, bool chain,
                                           int32_t *__restrict__ ntracklets, uint8_t *__restrict__ toomany) {
     tv.ntracks[e * OR_NSLOTS + lane_id()] = 0;
-    if (over && lane_id() == 0) {
-        toomany[e] = 1;
-        ntracklets[e] = 0;
+    if (lane_id() == 0) {
+        if (over) toomany[e] = 1;
+        if (over || chain) ntracklets[e] = 0;
     }
 }
 
@@ -557,7 +559,7 @@ struct XzSlot {
 template <int W>
 __global__ void __launch_bounds__(W * 32, (OR_XZ_WARPS_SM / W > 0 ? OR_XZ_WARPS_SM / W : 1))
     xz_kernel(const or_plane_t *__restrict__ gplane, or_hits_view_t hv, or_tracks_view_t tv,
-              int32_t *__restrict__ ntracklets, uint8_t *__restrict__ toomany, int n_events) {
+              int32_t *__restrict__ ntracklets, uint8_t *__restrict__ toomany, int n_events, bool chain) {
     extern __shared__ __align__(16) unsigned char xz_smem[];
     or_plane_t &P = *reinterpret_cast<or_plane_t *>(xz_smem);
     XzSlot *slots = reinterpret_cast<XzSlot *>(xz_smem + ((sizeof(or_plane_t) + 15) & ~size_t(15)));
@@ -568,11 +570,11 @@ __global__ void __launch_bounds__(W * 32, (OR_XZ_WARPS_SM / W > 0 ? OR_XZ_WARPS_
     XzWarp &S = slots[w].warp;
     for (long e = (long)blockIdx.x * W + w; e < n_events; e += (long)gridDim.x * W) {
         if (toomany[e]) {  // K:195-200
-            xz_reject(tv, e, false, ntracklets, toomany);
+            xz_reject(tv, e, false, chain, ntracklets, toomany);
             continue;
         }
         if (!xz_lists<1>(E, hv, e, P)) {
-            xz_reject(tv, e, true, ntracklets, toomany);
+            xz_reject(tv, e, true, chain, ntracklets, toomany);
             continue;
         }
         int kpar0 = 0, kpar1 = 0;
@@ -597,7 +599,7 @@ struct XzTeam {
 // warp or none.
 __global__ void __launch_bounds__(XZ_TEAM * 32)
     xz_team_kernel(const or_plane_t *__restrict__ gplane, or_hits_view_t hv, or_tracks_view_t tv,
-                   int32_t *__restrict__ ntracklets, uint8_t *__restrict__ toomany, int n_events) {
+                   int32_t *__restrict__ ntracklets, uint8_t *__restrict__ toomany, int n_events, bool chain) {
     extern __shared__ __align__(16) unsigned char xz_smem[];
     or_plane_t &P = *reinterpret_cast<or_plane_t *>(xz_smem);
     XzTeam &M = *reinterpret_cast<XzTeam *>(xz_smem + ((sizeof(or_plane_t) + 15) & ~size_t(15)));
@@ -610,11 +612,11 @@ __global__ void __launch_bounds__(XZ_TEAM * 32)
         const bool rejected = toomany[e];
         __syncthreads();  // every warp has read the flag before one of them sets it
         if (rejected) {
-            if (w == 0) xz_reject(tv, e, false, ntracklets, toomany);
+            if (w == 0) xz_reject(tv, e, false, chain, ntracklets, toomany);
             continue;
         }
         if (!xz_lists<XZ_TEAM>(E, hv, e, P)) {
-            if (w == 0) xz_reject(tv, e, true, ntracklets, toomany);
+            if (w == 0) xz_reject(tv, e, true, chain, ntracklets, toomany);
             continue;
         }
         // the warp's run of candidates: whole chunks, shared out evenly
@@ -696,7 +698,7 @@ size_t xz_smem_bytes(int warps) {
 
 template <int W>
 static cudaError_t xz_launch(const or_plane_t *d_plane, or_hits_view_t hv, or_tracks_view_t tv, int32_t *ntracklets,
-                             uint8_t *toomany, int n_events, cudaStream_t stream, int sm_count) {
+                             uint8_t *toomany, int n_events, cudaStream_t stream, int sm_count, bool chain) {
     const size_t smem = xz_smem_bytes(W);
     cudaError_t err = smem_attr_once((const void *)xz_kernel<W>, (int)smem);
     if (err != cudaSuccess) return err;
@@ -708,13 +710,15 @@ static cudaError_t xz_launch(const or_plane_t *d_plane, or_hits_view_t hv, or_tr
     // -> 2,238).
     const long cap = (long)sm_count * (32 / W > 0 ? 32 / W : 1);
     if (blocks > cap && n_events > 128 * sm_count) blocks = cap;
-    xz_kernel<W><<<(unsigned)blocks, W * 32, smem, stream>>>(d_plane, hv, tv, ntracklets, toomany, n_events);
+    xz_kernel<W><<<(unsigned)blocks, W * 32, smem, stream>>>(d_plane, hv, tv, ntracklets, toomany, n_events,
+                                                               chain);
     return cudaGetLastError();
 }
 
-// `warps` = events per CTA: 1, 2, 4 or 8 (the per-warp scratch is too large for 16)
+// `warps` = events per CTA: 1, 2, 4 or 8 (the per-warp scratch is too large for
+// 16); `chain`: every event's tracklet count is written (xz_reject)
 cudaError_t launch_xz(const or_plane_t *d_plane, or_hits_view_t hv, or_tracks_view_t tv, int32_t *ntracklets,
-                      uint8_t *toomany, int n_events, cudaStream_t stream, int sm_count, int warps) {
+                      uint8_t *toomany, int n_events, cudaStream_t stream, int sm_count, int warps, bool chain) {
     if (n_events <= 0) return cudaSuccess;
     // A CTA per event on small batches, where a warp per event leaves a heavy
     // event's chain to itself: 333 uneven events 238 -> 83 us, 1,000 of them
@@ -726,14 +730,14 @@ cudaError_t launch_xz(const or_plane_t *d_plane, or_hits_view_t hv, or_tracks_vi
         cudaError_t err = smem_attr_once((const void *)xz_team_kernel, (int)smem);
         if (err != cudaSuccess) return err;
         xz_team_kernel<<<(unsigned)n_events, XZ_TEAM * 32, smem, stream>>>(d_plane, hv, tv, ntracklets, toomany,
-                                                                           n_events);
+                                                                           n_events, chain);
         return cudaGetLastError();
     }
     switch (warps) {
-    case 1: return xz_launch<1>(d_plane, hv, tv, ntracklets, toomany, n_events, stream, sm_count);
-    case 2: return xz_launch<2>(d_plane, hv, tv, ntracklets, toomany, n_events, stream, sm_count);
-    case 8: return xz_launch<8>(d_plane, hv, tv, ntracklets, toomany, n_events, stream, sm_count);
-    default: return xz_launch<4>(d_plane, hv, tv, ntracklets, toomany, n_events, stream, sm_count);
+    case 1: return xz_launch<1>(d_plane, hv, tv, ntracklets, toomany, n_events, stream, sm_count, chain);
+    case 2: return xz_launch<2>(d_plane, hv, tv, ntracklets, toomany, n_events, stream, sm_count, chain);
+    case 8: return xz_launch<8>(d_plane, hv, tv, ntracklets, toomany, n_events, stream, sm_count, chain);
+    default: return xz_launch<4>(d_plane, hv, tv, ntracklets, toomany, n_events, stream, sm_count, chain);
     }
 }
 
